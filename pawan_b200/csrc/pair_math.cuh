@@ -88,6 +88,19 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+// 1/sqrt(x) in FP64: the hardware approximation (rsqrt.approx.ftz.f64, good to
+// about 2^-20) refined by one third-order step of Halley's iteration for
+// f(y) = 1/y^2 - x: with e = 1 - x y^2, y + y e (1/2 + 3/8 e), whose error is
+// e^3 / 3 or so.  Five FP64 operations; arguments that are not positive normal
+// numbers (zero, subnormal, infinite, NaN) take the library function.
+__device__ __forceinline__ double fast_rsqrt(double x) {
+  if ((unsigned)__double2hiint(x) - 0x00100000u >= 0x7fe00000u) return rsqrt(x);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
 template <typename T> struct PairTerms {
   T q;   // 4 pi q
   T F;   // 4 pi F

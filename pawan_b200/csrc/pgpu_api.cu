@@ -1041,19 +1041,37 @@ int pgpu_probe(pgpu_ctx *c, int32_t system, int64_t npts, const double *pts, dou
   if (system < 0 || system >= (int32_t)c->sys.size()) return fail(c, PGPU_EINVAL, "invalid system id %d", system);
   if (npts < 0 || (npts > 0 && (!pts || !vel))) return fail(c, PGPU_EINVAL, "bad probe arrays");
   if (npts == 0) return PGPU_OK;
-  double *d = nullptr;
-  CK(cudaMallocAsync((void **)&d, 6 * npts * sizeof(double), c->st));
-  CK(cudaMemcpyAsync(d, pts, 3 * npts * sizeof(double), cudaMemcpyHostToDevice, c->st));
-  CK(cudaMemsetAsync(d + 3 * npts, 0, 3 * npts * sizeof(double), c->st));
   const int64_t lo = c->sys[system].off, hi = lo + sys_n(c, system);
+  // Particle chunks: about eight CTAs per SM in all, of at least one particle
+  // per thread, and at most 512 chunks, so that the reduction stays a small
+  // part (400 points: 24 chunks of 50 point tiles).
+  const int64_t tiles = ceil_div(npts, kProbePoints);
+  int64_t chunks = std::min<int64_t>(std::max<int64_t>(1, 8LL * c->sms / tiles), 512);
+  chunks = std::max<int64_t>(1, std::min(chunks, ceil_div(hi - lo, kProbeBlock)));
+  const int64_t per = ceil_div(std::max<int64_t>(hi - lo, 1), chunks);
+  // points, velocities and per-chunk sums: in the context's transfer staging
+  // (free between calls, ordered on its stream) where they fit, as for a few
+  // hundred points of any wake, else in an allocation of this call
+  const int64_t need = (6 + 3 * chunks) * npts;
+  const bool own = need > 8 * c->cap;
+  double *d = c->stage;
+  if (own) CK(cudaMallocAsync((void **)&d, need * sizeof(double), c->st));
+  double *d_vel = d + 3 * npts, *d_part = d + 6 * npts;
+  CK(cudaMemcpyAsync(d, pts, 3 * npts * sizeof(double), cudaMemcpyHostToDevice, c->st));
   if (hi > lo) {
-    auto fn = c->cfg.kernel == PGPU_KERNEL_HIGHORDER ? probe_kernel<128, kHighOrder> : probe_kernel<128, kGaussian>;
-    fn<<<(unsigned)ceil_div(npts, 128), 128, 0, c->st>>>(c->x0, c->sig, c->cap, lo, hi, d, npts, d + 3 * npts);
+    auto fn = c->cfg.kernel == PGPU_KERNEL_HIGHORDER ? probe_kernel<kHighOrder> : probe_kernel<kGaussian>;
+    fn<<<dim3((unsigned)tiles, (unsigned)chunks), kProbeBlock, 0, c->st>>>(c->x0, c->sig, c->cap, lo, hi, per, d, npts,
+                                                                           d_part);
     CK(cudaGetLastError());
-    c->launches++;
+    const int rg = (int)std::min<int64_t>(ceil_div(3 * npts, 128), 16LL * c->sms);
+    probe_reduce_kernel<<<rg, 128, 0, c->st>>>(d_part, (int)chunks, 3 * npts, d_vel);
+    CK(cudaGetLastError());
+    c->launches += 2;
+  } else {
+    CK(cudaMemsetAsync(d_vel, 0, 3 * npts * sizeof(double), c->st));
   }
-  CK(cudaMemcpyAsync(vel, d + 3 * npts, 3 * npts * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaFreeAsync(d, c->st));
+  CK(cudaMemcpyAsync(vel, d_vel, 3 * npts * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  if (own) CK(cudaFreeAsync(d, c->st));
   CK(cudaStreamSynchronize(c->st));
   return PGPU_OK;
 }
