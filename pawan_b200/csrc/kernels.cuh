@@ -49,6 +49,10 @@ struct PlanEntry {
   int64_t chunk;       // sources per chunk (multiple of the source tile)
   int64_t toff;        // targets: particles [off + toff, off + toff + tn) of the system
   int64_t tn;
+  // Slices kernel (pair_slices.cuh): items are rows, chunk is the rows per
+  // target tile, mult the step of their order; the sentinel's chunk is the
+  // rows per CTA.
+  int64_t mult;
 };
 
 template <typename T> struct PairArgs {
@@ -495,6 +499,7 @@ __device__ __forceinline__ void pair_body_generic(const PairArgs<T> &a) {
 }  // namespace pgpu
 
 #include "pair_f32.cuh"
+#include "pair_slices.cuh"
 
 namespace pgpu {
 
@@ -590,58 +595,81 @@ static __global__ void __launch_bounds__(256) box_kernel(const float4 *P, const 
   }
 }
 
+// One RK stage: the chunk partials summed into the rates, the stage update of
+// the FP64 state, and the next stage's source records.  Bound by latency below
+// about 1e5 particles and by HBM above: a CTA takes 32 particles with one warp
+// per component, so a small system still spreads over the SMs, and the loads
+// of four chunks are in flight together.  The components meet in shared memory for the records.
+constexpr int kStageParticles = 32;
+constexpr int kStageBlock = 6 * kStageParticles;
+
 template <typename T>
-__global__ void stage_kernel(StageArgs a) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.cap; i += (int64_t)gridDim.x * blockDim.x) {
-    const int s = find_sys(a.sys_off, a.nsys, i);
-    const int64_t li = i - a.sys_off[s];
-    if (li >= a.sys_n[s] || li < a.sys_t[2 * s] || li >= a.sys_t[2 * s + 1]) continue;
-    double k[6];
-#pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      double v = 0.0;
-      for (int c = 0; c < a.nch; ++c) v += a.partial[((int64_t)c * 6 + m) * a.cap + i];
-      k[m] = v;
-      a.rates[m * a.cap + i] = v;
+__global__ void __launch_bounds__(kStageBlock) stage_kernel(StageArgs a) {
+  __shared__ double sy[6][kStageParticles];
+  const int m = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t nb = (a.cap + kStageParticles - 1) / kStageParticles;
+  for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
+    const int64_t i = b * kStageParticles + lane;
+    bool live = i < a.cap;
+    if (live) {
+      const int s = find_sys(a.sys_off, a.nsys, i);
+      const int64_t li = i - a.sys_off[s];
+      live = li < a.sys_n[s] && li >= a.sys_t[2 * s] && li < a.sys_t[2 * s + 1];
+    }
+    if (live) {
+      const int64_t e = m * a.cap + i;
+      const double *p = a.partial + e;
+      const int64_t step = 6 * a.cap;
+      double k = 0.0;
+      int c = 0;
+      for (; c + 4 <= a.nch; c += 4) {
+        const double p0 = p[c * step], p1 = p[(c + 1) * step], p2 = p[(c + 2) * step], p3 = p[(c + 3) * step];
+        k += p0;
+        k += p1;
+        k += p2;
+        k += p3;
+      }
+      for (; c < a.nch; ++c) k += p[c * step];
+      a.rates[e] = k;
+      if (a.scheme >= 0) {
+        const double dt = a.dt, x = a.x0[e];
+        double yy;
+        bool final_stage = false;
+        if (a.scheme == 2) {  // classical RK4
+          if (a.stage == 0) { a.acc[e] = k; yy = x + 0.5 * dt * k; }
+          else if (a.stage == 1) { a.acc[e] += 2.0 * k; yy = x + 0.5 * dt * k; }
+          else if (a.stage == 2) { a.acc[e] += 2.0 * k; yy = x + dt * k; }
+          else { yy = x + (dt / 6.0) * (a.acc[e] + k); final_stage = true; }
+        } else if (a.scheme == 1) {  // Kutta RK3
+          if (a.stage == 0) { a.acc[e] = k; yy = x + 0.5 * dt * k; }
+          else if (a.stage == 1) { const double acc = a.acc[e]; yy = x + dt * (2.0 * k - acc); a.acc[e] = acc + 4.0 * k; }
+          else { yy = x + (dt / 6.0) * (a.acc[e] + k); final_stage = true; }
+        } else {  // explicit Euler
+          yy = x + dt * k;
+          final_stage = true;
+        }
+        if (final_stage) {
+          if (m < 3) yy += a.vinf[m] * dt;
+          a.x0[e] = yy;
+        }
+        if (!isfinite(yy)) *a.flag = 1;
+        sy[m][lane] = yy;
+      }
     }
     if (a.scheme < 0) continue;
-    double y[6];
-    const double dt = a.dt;
-    bool final_stage = false;
-#pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      const double x = a.x0[m * a.cap + i];
-      double acc = a.acc[m * a.cap + i];
-      double yy;
-      if (a.scheme == 2) {  // classical RK4
-        if (a.stage == 0) { acc = k[m]; yy = x + 0.5 * dt * k[m]; }
-        else if (a.stage == 1) { acc += 2.0 * k[m]; yy = x + 0.5 * dt * k[m]; }
-        else if (a.stage == 2) { acc += 2.0 * k[m]; yy = x + dt * k[m]; }
-        else { yy = x + (dt / 6.0) * (acc + k[m]); final_stage = true; }
-      } else if (a.scheme == 1) {  // Kutta RK3
-        if (a.stage == 0) { acc = k[m]; yy = x + 0.5 * dt * k[m]; }
-        else if (a.stage == 1) { yy = x + dt * (2.0 * k[m] - acc); acc += 4.0 * k[m]; }
-        else { yy = x + (dt / 6.0) * (acc + k[m]); final_stage = true; }
-      } else {  // explicit Euler
-        yy = x + dt * k[m];
-        final_stage = true;
+    __syncthreads();
+    if (live) {
+      if (m == 0) {
+        const double sg = a.sig[i];
+        static_cast<v4_t<T> *>(a.P)[i] =
+            make_v4<T>((T)sy[0][lane], (T)sy[1][lane], (T)sy[2][lane], (T)(0.5 * sg * sg));
+      } else if (m == 1) {
+        static_cast<v4_t<T> *>(a.Q)[i] = make_v4<T>((T)sy[3][lane], (T)sy[4][lane], (T)sy[5][lane], (T)a.vol[i]);
+      } else if (m == 2 && a.L) {
+        a.L[i] = split_low(sy[0][lane], sy[1][lane], sy[2][lane]);
       }
-      if (final_stage && m < 3) yy += a.vinf[m] * dt;
-      a.acc[m * a.cap + i] = acc;
-      y[m] = yy;
     }
-    if (final_stage) {
-#pragma unroll
-      for (int m = 0; m < 6; ++m) a.x0[m * a.cap + i] = y[m];
-    }
-    bool bad = false;
-#pragma unroll
-    for (int m = 0; m < 6; ++m) bad |= !isfinite(y[m]);
-    if (bad) *a.flag = 1;
-    const double sg = a.sig[i];
-    static_cast<v4_t<T> *>(a.P)[i] = make_v4<T>((T)y[0], (T)y[1], (T)y[2], (T)(0.5 * sg * sg));
-    static_cast<v4_t<T> *>(a.Q)[i] = make_v4<T>((T)y[3], (T)y[4], (T)y[5], (T)a.vol[i]);
-    if (a.L) a.L[i] = split_low(y[0], y[1], y[2]);
+    __syncthreads();
   }
 }
 

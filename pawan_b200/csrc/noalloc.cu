@@ -84,6 +84,7 @@ __global__ void noalloc_pack_kernel(const double *pos, const double *alpha, cons
     plan[0].chunk = (per + kNoAllocBlock - 1) / kNoAllocBlock * kNoAllocBlock;
     plan[0].toff = 0;
     plan[0].tn = n;
+    plan[0].mult = 0;
     plan[1].off = 0;
     plan[1].n = 0;
     plan[1].item_start = tiles * nch;
@@ -91,6 +92,7 @@ __global__ void noalloc_pack_kernel(const double *pos, const double *alpha, cons
     plan[1].chunk = 0;
     plan[1].toff = 0;
     plan[1].tn = 0;
+    plan[1].mult = 0;
   }
 }
 

@@ -43,6 +43,147 @@ constexpr int pair_f32_min_blocks() {
 // of each other on B200; 2 is best with the autotuner's usual 128x2 shape).
 constexpr int kF32Unroll = 2;
 
+// One source pair (lane .x the even source, .y the odd one) in the far limit
+// on one target: positions and n_s relative to the tile's reference point,
+// X' x (-3 alpha_t) in B3 and -3 alpha_t in AT3.  25 packed operations.
+__device__ __forceinline__ void far_pair2(float2 px, float2 py, float2 pz, float2 ax, float2 ay, float2 az, float2 nx,
+                                          float2 ny, float2 nz, const float2 *X, const float2 *AT3, const float2 *B3,
+                                          float2 *sv, float2 *sd, float2 *sp) {
+  const float2 M1 = make_float2(-1.f, -1.f);
+  // d = x_t - x_s (exact-rounded, as a subtraction)
+  const float2 dx = __ffma2_rn(px, M1, X[0]);
+  const float2 dy = __ffma2_rn(py, M1, X[1]);
+  const float2 dz = __ffma2_rn(pz, M1, X[2]);
+  float2 r2 = __fmul2_rn(dx, dx);
+  r2 = __ffma2_rn(dy, dy, r2);
+  r2 = __ffma2_rn(dz, dz, r2);
+  // far limit: q' = r^3, F' = -3 r^5 (the -3 is in AT3 and B3), no diffusion
+  const float2 ir = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
+  const float2 A = __fmul2_rn(ir, ir);
+  const float2 qq = __fmul2_rn(A, ir);
+  const float2 qA = __fmul2_rn(qq, A);
+  // sum q alpha_s and sum q n_s (the velocity is formed at the fold)
+  sp[0] = __ffma2_rn(qq, ax, sp[0]);
+  sp[1] = __ffma2_rn(qq, ay, sp[1]);
+  sp[2] = __ffma2_rn(qq, az, sp[2]);
+  sv[0] = __ffma2_rn(qq, nx, sv[0]);
+  sv[1] = __ffma2_rn(qq, ny, sv[1]);
+  sv[2] = __ffma2_rn(qq, nz, sv[2]);
+  // F (alpha_t . w) d, alpha_t . w = alpha_s . (X' x alpha_t) + n_s . alpha_t
+  float2 dot = __fmul2_rn(ax, B3[0]);
+  dot = __ffma2_rn(ay, B3[1], dot);
+  dot = __ffma2_rn(az, B3[2], dot);
+  dot = __ffma2_rn(nx, AT3[0], dot);
+  dot = __ffma2_rn(ny, AT3[1], dot);
+  dot = __ffma2_rn(nz, AT3[2], dot);
+  const float2 fd = __fmul2_rn(qA, dot);
+  sd[0] = __ffma2_rn(fd, dx, sd[0]);
+  sd[1] = __ffma2_rn(fd, dy, sd[1]);
+  sd[2] = __ffma2_rn(fd, dz, sd[2]);
+}
+
+// B3 = X' x (-3 alpha_t), duplicated into both lanes.
+__device__ __forceinline__ void far_b3(float xr0, float xr1, float xr2, const float2 *AT3, float2 *B3) {
+  const float c0 = AT3[0].x, c1 = AT3[1].x, c2 = AT3[2].x;
+  B3[0] = dup2(xr1 * c2 - xr2 * c1);
+  B3[1] = dup2(xr2 * c0 - xr0 * c2);
+  B3[2] = dup2(xr0 * c1 - xr1 * c0);
+}
+
+// One source pair in the closed form on one target (pair_terms_mid2: the mid
+// formula, which beyond u = 50 equals the far limit to within e^{-u/2});
+// lanes at u < 1, the self pair among them, take the series.  Per pair:
+// q (alpha_t x alpha_s) for the stretching (nearly parallel neighbours along a
+// filament) and the diffusion v_t a_s - v_s a_t.  uni: the sigma factors where
+// one sigma serves every pair (72 FP32 operations per pair, 63 with them), or
+// null.  All lanes of the warp together (it votes).
+template <bool SPLIT>
+__device__ __forceinline__ void mid_pair2(float2 px, float2 py, float2 pz, float2 ph, float2 ax, float2 ay, float2 az,
+                                          float2 av, float2 lx, float2 ly, float2 lz, const float2 *X, const float *xl,
+                                          const float *at, float hst, float h50, float vt, const MidSigma2 *uni,
+                                          float2 *sv, float2 *sd, float2 *sp, float2 *sdv, unsigned &nfull) {
+  const float2 M1 = make_float2(-1.f, -1.f);
+  float2 dx = __ffma2_rn(px, M1, X[0]);
+  float2 dy = __ffma2_rn(py, M1, X[1]);
+  float2 dz = __ffma2_rn(pz, M1, X[2]);
+  if constexpr (SPLIT) {
+    // the FP32 difference of nearby positions is exact; adding the
+    // difference of the residuals restores the FP64 difference
+    dx = __fadd2_rn(dx, __ffma2_rn(lx, M1, dup2(xl[0])));
+    dy = __fadd2_rn(dy, __ffma2_rn(ly, M1, dup2(xl[1])));
+    dz = __fadd2_rn(dz, __ffma2_rn(lz, M1, dup2(xl[2])));
+  }
+  float2 r2 = __fmul2_rn(dx, dx);
+  r2 = __ffma2_rn(dy, dy, r2);
+  r2 = __ffma2_rn(dz, dz, r2);
+  const float2 s2 = uni ? uni->s2 : __fadd2_rn(dup2(hst), ph);
+  PairTerms2 t = pair_terms_mid2(r2, uni ? *uni : mid_sigma2(s2));
+  const bool nx = r2.x < s2.x, ny = r2.y < s2.y;  // u < 1
+  if (__any_sync(0xffffffffu, nx || ny)) {
+    if (nx) { const PairTerms<float> e = pair_terms_near(r2.x, s2.x); t.q.x = e.q; t.F.x = e.F; t.zd.x = e.zd; }
+    if (ny) { const PairTerms<float> e = pair_terms_near(r2.y, s2.y); t.q.y = e.q; t.F.y = e.F; t.zd.y = e.zd; }
+  }
+  // pairs inside the far regime's bound count as full-formula pairs
+  nfull += (fmaf(-kFarU, ph.x, r2.x) < h50) + (fmaf(-kFarU, ph.y, r2.y) < h50);
+  // w = alpha_s x d (scalar: the negated operand is free)
+  const float2 wx = make_float2(ay.x * dz.x - az.x * dy.x, ay.y * dz.y - az.y * dy.y);
+  const float2 wy = make_float2(az.x * dx.x - ax.x * dz.x, az.y * dx.y - ax.y * dz.y);
+  const float2 wz = make_float2(ax.x * dy.x - ay.x * dx.x, ax.y * dy.y - ay.y * dx.y);
+  sv[0] = __ffma2_rn(t.q, wx, sv[0]);
+  sv[1] = __ffma2_rn(t.q, wy, sv[1]);
+  sv[2] = __ffma2_rn(t.q, wz, sv[2]);
+  float2 dot = __fmul2_rn(dup2(at[0]), wx);
+  dot = __ffma2_rn(dup2(at[1]), wy, dot);
+  dot = __ffma2_rn(dup2(at[2]), wz, dot);
+  const float2 fd = __fmul2_rn(t.F, dot);
+  sd[0] = __ffma2_rn(fd, dx, sd[0]);
+  sd[1] = __ffma2_rn(fd, dy, sd[1]);
+  sd[2] = __ffma2_rn(fd, dz, sd[2]);
+  const float2 cx = __ffma2_rn(dup2(at[1]), az, __fmul2_rn(dup2(-at[2]), ay));
+  const float2 cy = __ffma2_rn(dup2(at[2]), ax, __fmul2_rn(dup2(-at[0]), az));
+  const float2 cz = __ffma2_rn(dup2(at[0]), ay, __fmul2_rn(dup2(-at[1]), ax));
+  sp[0] = __ffma2_rn(t.q, cx, sp[0]);
+  sp[1] = __ffma2_rn(t.q, cy, sp[1]);
+  sp[2] = __ffma2_rn(t.q, cz, sp[2]);
+  const float2 VT = dup2(vt);
+  sdv[0] = __ffma2_rn(t.zd, __ffma2_rn(av, dup2(-at[0]), __fmul2_rn(VT, ax)), sdv[0]);
+  sdv[1] = __ffma2_rn(t.zd, __ffma2_rn(av, dup2(-at[1]), __fmul2_rn(VT, ay)), sdv[1]);
+  sdv[2] = __ffma2_rn(t.zd, __ffma2_rn(av, dup2(-at[2]), __fmul2_rn(VT, az)), sdv[2]);
+}
+
+// Folds one compensation group of a target into its (hi, lo) sums.  Far
+// groups summed q alpha_s and q n_s (xr = x_t - ref), the others
+// q (alpha_t x alpha_s) and q w.
+__device__ __forceinline__ void fold_group_f32(bool far, float xr0, float xr1, float xr2, const float *at, float nu2,
+                                               const float2 *sv, const float2 *sd, const float2 *sp, const float *sdv,
+                                               float *vh, float *vl, float *dh, float *dl) {
+  float svs[3], sds[3], sps[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    svs[m] = sv[m].x + sv[m].y;
+    sds[m] = sd[m].x + sd[m].y;
+    sps[m] = sp[m].x + sp[m].y;
+  }
+  // da = sum q (alpha_t x alpha_s) + sum F (d.c) d + 2 nu sum z (v_t a_s - v_s a_t)
+  float c0 = sps[0], c1 = sps[1], c2 = sps[2];
+  if (far) {
+    // velocity = (sum q alpha_s) x X' + sum q n_s
+    const float n0 = svs[0], n1 = svs[1], n2 = svs[2];
+    svs[0] = sps[1] * xr2 - sps[2] * xr1 + n0;
+    svs[1] = sps[2] * xr0 - sps[0] * xr2 + n1;
+    svs[2] = sps[0] * xr1 - sps[1] * xr0 + n2;
+    c0 = at[1] * sps[2] - at[2] * sps[1];
+    c1 = at[2] * sps[0] - at[0] * sps[2];
+    c2 = at[0] * sps[1] - at[1] * sps[0];
+  }
+  two_sum_acc(vh[0], vl[0], svs[0]);
+  two_sum_acc(vh[1], vl[1], svs[1]);
+  two_sum_acc(vh[2], vl[2], svs[2]);
+  two_sum_acc(dh[0], dl[0], c0 + sds[0] + nu2 * sdv[0]);
+  two_sum_acc(dh[1], dl[1], c1 + sds[1] + nu2 * sdv[1]);
+  two_sum_acc(dh[2], dl[2], c2 + sds[2] + nu2 * sdv[2]);
+}
+
 template <int BLOCK, int TPT, int CG, bool SPLIT>
 __device__ __forceinline__ void pair_body_f32(const PairArgs<float> &a) {
   constexpr int TILE = BLOCK;
@@ -58,7 +199,6 @@ __device__ __forceinline__ void pair_body_f32(const PairArgs<float> &a) {
   __shared__ int s_item;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
-  const float2 M1 = make_float2(-1.f, -1.f);
   const int64_t total = a.plan[a.nsys].item_start;
   int64_t item;
   while (next_item(a.counters, total, item, &s_item)) {
@@ -215,11 +355,7 @@ __device__ __forceinline__ void pair_body_f32(const PairArgs<float> &a) {
           float2 B3[TPT][3];
 #pragma unroll
           for (int k = 0; k < TPT; ++k) {
-            const float xr0 = X[k][0].x - rx, xr1 = X[k][1].x - ry, xr2 = X[k][2].x - rz;
-            const float c0 = AT3[k][0].x, c1 = AT3[k][1].x, c2 = AT3[k][2].x;
-            B3[k][0] = dup2(xr1 * c2 - xr2 * c1);
-            B3[k][1] = dup2(xr2 * c0 - xr0 * c2);
-            B3[k][2] = dup2(xr0 * c1 - xr1 * c0);
+            far_b3(X[k][0].x - rx, X[k][1].x - ry, X[k][2].x - rz, AT3[k], B3[k]);
           }
 #pragma unroll kF32Unroll
           for (int r = g; r < g + CG / 2; ++r) {
@@ -231,36 +367,7 @@ __device__ __forceinline__ void pair_body_f32(const PairArgs<float> &a) {
             const float2 nx = make_float2(na.x, na.y), ny = make_float2(na.z, na.w), nz = make_float2(nb.x, nb.y);
 #pragma unroll
             for (int k = 0; k < TPT; ++k) {
-              // d = x_t - x_s (exact-rounded, as a subtraction)
-              const float2 dx = __ffma2_rn(px, M1, X[k][0]);
-              const float2 dy = __ffma2_rn(py, M1, X[k][1]);
-              const float2 dz = __ffma2_rn(pz, M1, X[k][2]);
-              float2 r2 = __fmul2_rn(dx, dx);
-              r2 = __ffma2_rn(dy, dy, r2);
-              r2 = __ffma2_rn(dz, dz, r2);
-              // far limit: q' = r^3, F' = -3 r^5 (the -3 is in AT3 and B3), no diffusion
-              const float2 ir = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
-              const float2 A = __fmul2_rn(ir, ir);
-              const float2 qq = __fmul2_rn(A, ir);
-              const float2 qA = __fmul2_rn(qq, A);
-              // sum q alpha_s and sum q n_s (the velocity is formed at the fold)
-              sp[k][0] = __ffma2_rn(qq, ax, sp[k][0]);
-              sp[k][1] = __ffma2_rn(qq, ay, sp[k][1]);
-              sp[k][2] = __ffma2_rn(qq, az, sp[k][2]);
-              sv[k][0] = __ffma2_rn(qq, nx, sv[k][0]);
-              sv[k][1] = __ffma2_rn(qq, ny, sv[k][1]);
-              sv[k][2] = __ffma2_rn(qq, nz, sv[k][2]);
-              // F (alpha_t . w) d, alpha_t . w = alpha_s . (X' x alpha_t) + n_s . alpha_t
-              float2 dot = __fmul2_rn(ax, B3[k][0]);
-              dot = __ffma2_rn(ay, B3[k][1], dot);
-              dot = __ffma2_rn(az, B3[k][2], dot);
-              dot = __ffma2_rn(nx, AT3[k][0], dot);
-              dot = __ffma2_rn(ny, AT3[k][1], dot);
-              dot = __ffma2_rn(nz, AT3[k][2], dot);
-              const float2 fd = __fmul2_rn(qA, dot);
-              sd[k][0] = __ffma2_rn(fd, dx, sd[k][0]);
-              sd[k][1] = __ffma2_rn(fd, dy, sd[k][1]);
-              sd[k][2] = __ffma2_rn(fd, dz, sd[k][2]);
+              far_pair2(px, py, pz, ax, ay, az, nx, ny, nz, X[k], AT3[k], B3[k], sv[k], sd[k], sp[k]);
             }
           }
         } else if constexpr (TPT >= 2) {
@@ -294,52 +401,8 @@ __device__ __forceinline__ void pair_body_f32(const PairArgs<float> &a) {
             }
 #pragma unroll
             for (int k = 0; k < TPT; ++k) {
-              float2 dx = __ffma2_rn(px, M1, X[k][0]);
-              float2 dy = __ffma2_rn(py, M1, X[k][1]);
-              float2 dz = __ffma2_rn(pz, M1, X[k][2]);
-              if constexpr (SPLIT) {
-                // the FP32 difference of nearby positions is exact; adding the
-                // difference of the residuals restores the FP64 difference
-                dx = __fadd2_rn(dx, __ffma2_rn(lx, M1, dup2(xl[k][0])));
-                dy = __fadd2_rn(dy, __ffma2_rn(ly, M1, dup2(xl[k][1])));
-                dz = __fadd2_rn(dz, __ffma2_rn(lz, M1, dup2(xl[k][2])));
-              }
-              float2 r2 = __fmul2_rn(dx, dx);
-              r2 = __ffma2_rn(dy, dy, r2);
-              r2 = __ffma2_rn(dz, dz, r2);
-              const float2 s2 = __fadd2_rn(dup2(hst[k]), ph);
-              PairTerms2 t = pair_terms_mid2(r2, s2);
-              const bool nx = r2.x < s2.x, ny = r2.y < s2.y;  // u < 1
-              if (__any_sync(0xffffffffu, nx || ny)) {
-                if (nx) { const PairTerms<float> e = pair_terms_near(r2.x, s2.x); t.q.x = e.q; t.F.x = e.F; t.zd.x = e.zd; }
-                if (ny) { const PairTerms<float> e = pair_terms_near(r2.y, s2.y); t.q.y = e.q; t.F.y = e.F; t.zd.y = e.zd; }
-              }
-              // pairs inside the far regime's bound count as full-formula pairs
-              nfull += (fmaf(-kFarU, ph.x, r2.x) < h50[k]) + (fmaf(-kFarU, ph.y, r2.y) < h50[k]);
-              // w = alpha_s x d (scalar: the negated operand is free)
-              const float2 wx = make_float2(ay.x * dz.x - az.x * dy.x, ay.y * dz.y - az.y * dy.y);
-              const float2 wy = make_float2(az.x * dx.x - ax.x * dz.x, az.y * dx.y - ax.y * dz.y);
-              const float2 wz = make_float2(ax.x * dy.x - ay.x * dx.x, ax.y * dy.y - ay.y * dx.y);
-              sv[k][0] = __ffma2_rn(t.q, wx, sv[k][0]);
-              sv[k][1] = __ffma2_rn(t.q, wy, sv[k][1]);
-              sv[k][2] = __ffma2_rn(t.q, wz, sv[k][2]);
-              float2 dot = __fmul2_rn(dup2(at[k][0]), wx);
-              dot = __ffma2_rn(dup2(at[k][1]), wy, dot);
-              dot = __ffma2_rn(dup2(at[k][2]), wz, dot);
-              const float2 fd = __fmul2_rn(t.F, dot);
-              sd[k][0] = __ffma2_rn(fd, dx, sd[k][0]);
-              sd[k][1] = __ffma2_rn(fd, dy, sd[k][1]);
-              sd[k][2] = __ffma2_rn(fd, dz, sd[k][2]);
-              const float2 cx = __ffma2_rn(dup2(at[k][1]), az, __fmul2_rn(dup2(-at[k][2]), ay));
-              const float2 cy = __ffma2_rn(dup2(at[k][2]), ax, __fmul2_rn(dup2(-at[k][0]), az));
-              const float2 cz = __ffma2_rn(dup2(at[k][0]), ay, __fmul2_rn(dup2(-at[k][1]), ax));
-              sp[k][0] = __ffma2_rn(t.q, cx, sp[k][0]);
-              sp[k][1] = __ffma2_rn(t.q, cy, sp[k][1]);
-              sp[k][2] = __ffma2_rn(t.q, cz, sp[k][2]);
-              const float2 VT = dup2(vt[k]);
-              sdv2[k][0] = __ffma2_rn(t.zd, __ffma2_rn(av, dup2(-at[k][0]), __fmul2_rn(VT, ax)), sdv2[k][0]);
-              sdv2[k][1] = __ffma2_rn(t.zd, __ffma2_rn(av, dup2(-at[k][1]), __fmul2_rn(VT, ay)), sdv2[k][1]);
-              sdv2[k][2] = __ffma2_rn(t.zd, __ffma2_rn(av, dup2(-at[k][2]), __fmul2_rn(VT, az)), sdv2[k][2]);
+              mid_pair2<SPLIT>(px, py, pz, ph, ax, ay, az, av, lx, ly, lz, X[k], xl[SPLIT ? k : 0], at[k], hst[k], h50[k],
+                               vt[k], nullptr, sv[k], sd[k], sp[k], sdv2[k], nfull);
             }
           }
 #pragma unroll
@@ -409,38 +472,8 @@ __device__ __forceinline__ void pair_body_f32(const PairArgs<float> &a) {
         }
 #pragma unroll
         for (int k = 0; k < TPT; ++k) {
-          float svs[3], sds[3], sps[3];
-#pragma unroll
-          for (int m = 0; m < 3; ++m) {
-            svs[m] = sv[k][m].x + sv[k][m].y;
-            sds[m] = sd[k][m].x + sd[k][m].y;
-            sps[m] = sp[k][m].x + sp[k][m].y;
-          }
-          if (far_tile) {
-            // velocity = (sum q alpha_s) x X' + sum q n_s
-            const float xr0 = X[k][0].x - rx, xr1 = X[k][1].x - ry, xr2 = X[k][2].x - rz;
-            const float n0 = svs[0], n1 = svs[1], n2 = svs[2];
-            svs[0] = sps[1] * xr2 - sps[2] * xr1 + n0;
-            svs[1] = sps[2] * xr0 - sps[0] * xr2 + n1;
-            svs[2] = sps[0] * xr1 - sps[1] * xr0 + n2;
-          }
-          // da = sum q (alpha_t x alpha_s) + sum F (d.c) d + 2 nu sum z (v_t a_s - v_s a_t);
-          // far tiles summed q alpha_s, near tiles q (alpha_t x alpha_s) itself
-          float c0 = sps[0], c1 = sps[1], c2 = sps[2];
-          if (far_tile) {
-            c0 = at[k][1] * sps[2] - at[k][2] * sps[1];
-            c1 = at[k][2] * sps[0] - at[k][0] * sps[2];
-            c2 = at[k][0] * sps[1] - at[k][1] * sps[0];
-          }
-          const float ex = c0 + sds[0] + a.nu2 * sdv[k][0];
-          const float ey = c1 + sds[1] + a.nu2 * sdv[k][1];
-          const float ez = c2 + sds[2] + a.nu2 * sdv[k][2];
-          two_sum_acc(vh[k][0], vl[k][0], svs[0]);
-          two_sum_acc(vh[k][1], vl[k][1], svs[1]);
-          two_sum_acc(vh[k][2], vl[k][2], svs[2]);
-          two_sum_acc(dh[k][0], dl[k][0], ex);
-          two_sum_acc(dh[k][1], dl[k][1], ey);
-          two_sum_acc(dh[k][2], dl[k][2], ez);
+          fold_group_f32(far_tile, X[k][0].x - rx, X[k][1].x - ry, X[k][2].x - rz, at[k], a.nu2, sv[k], sd[k], sp[k],
+                         sdv[k], vh[k], vl[k], dh[k], dl[k]);
         }
       }
       __syncthreads();

@@ -330,27 +330,41 @@ struct PairTerms2 {
 };
 __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
-__device__ __forceinline__ PairTerms2 pair_terms_mid2(float2 r2, float2 s2) {
+// The factors of the mid branch that depend on sigma alone.
+struct MidSigma2 {
+  float2 s2, is2, ea, zk, zs, azs, nk1;
+};
+__device__ __forceinline__ MidSigma2 mid_sigma2(float2 s2) {
+  MidSigma2 o;
+  o.s2 = s2;
   const float2 is = make_float2(fast_rsqrt(s2.x), fast_rsqrt(s2.y));
-  const float2 is2 = __fmul2_rn(is, is);
-  const float2 ea = __fmul2_rn(__fmul2_rn(r2, is2), dup2((float)kNegHalfLog2e));
+  o.is2 = __fmul2_rn(is, is);
+  o.ea = __fmul2_rn(o.is2, dup2((float)kNegHalfLog2e));
+  o.zk = __fmul2_rn(__fmul2_rn(dup2((float)kK1), is), o.is2);       // (k1 s) s^2
+  o.zs = __fmul2_rn(__fmul2_rn(dup2(1.41421356237309515f), s2), is);  // sqrt2 sigma
+  o.azs = __fmul2_rn(dup2(kErfcxA), o.zs);
+  o.nk1 = __fmul2_rn(dup2(-(float)kK1), is);
+  return o;
+}
+
+__device__ __forceinline__ PairTerms2 pair_terms_mid2(float2 r2, const MidSigma2 &g) {
+  const float2 ea = __fmul2_rn(r2, g.ea);
   const float2 E = make_float2(fast_exp2(ea.x), fast_exp2(ea.y));
-  const float2 z = __fmul2_rn(__fmul2_rn(__fmul2_rn(dup2((float)kK1), is), is2), E);  // (k1 s) s^2 E
+  const float2 z = __fmul2_rn(g.zk, E);
   const float2 ir = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
   const float2 A = __fmul2_rn(ir, ir);
-  const float2 zs = __fmul2_rn(__fmul2_rn(dup2(1.41421356237309515f), s2), is);  // sqrt2 sigma
-  const float2 t = __ffma2_rn(__fmul2_rn(dup2(kErfcxA), zs), ir, dup2(kErfcxB));
+  const float2 t = __ffma2_rn(g.azs, ir, dup2(kErfcxB));
   float2 np = dup2(-PGPU_E10);
   np = __ffma2_rn(np, t, dup2(-PGPU_E9)); np = __ffma2_rn(np, t, dup2(-PGPU_E8));
   np = __ffma2_rn(np, t, dup2(-PGPU_E7)); np = __ffma2_rn(np, t, dup2(-PGPU_E6));
   np = __ffma2_rn(np, t, dup2(-PGPU_E5)); np = __ffma2_rn(np, t, dup2(-PGPU_E4));
   np = __ffma2_rn(np, t, dup2(-PGPU_E3)); np = __ffma2_rn(np, t, dup2(-PGPU_E2));
   np = __ffma2_rn(np, t, dup2(-PGPU_E1)); np = __ffma2_rn(np, t, dup2(-PGPU_E0));
-  const float2 nB = __ffma2_rn(__fmul2_rn(zs, A), np, __fmul2_rn(dup2(-(float)kK1), is));
+  const float2 nB = __ffma2_rn(__fmul2_rn(g.zs, A), np, g.nk1);
   PairTerms2 o;
   o.q = __ffma2_rn(__fmul2_rn(E, A), nB, __fmul2_rn(A, ir));
   o.F = __fmul2_rn(__ffma2_rn(dup2(-3.0f), o.q, z), A);
-  o.zd = __fmul2_rn(z, is2);
+  o.zd = __fmul2_rn(z, g.is2);
   return o;
 }
 

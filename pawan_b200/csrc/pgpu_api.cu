@@ -24,6 +24,7 @@
 #include <cstdint>
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <string>
 #include <thread>
 #include <tuple>
@@ -67,6 +68,15 @@ template <typename T> PairFn<T> pair_fn(int s, int ker, bool split) {
     if (split) return pair_fn_k<T, kGaussian, true>(s);
   }
   return pair_fn_k<T, kGaussian>(s);
+}
+
+// Variants of the slices kernel (pair_slices.cuh): 32-source slices of one
+// source per lane, with or without split positions, and 64-source ones.
+constexpr int kSliceLen[] = {32, 64};
+constexpr int kNumSlices = 2;
+PairFn<float> slices_fn(int v, bool split) {
+  if (split) return pair_slices_kernel<1, true>;
+  return v == 0 ? pair_slices_kernel<1, false> : pair_slices_kernel<2, false>;
 }
 
 struct WakeRec {
@@ -117,6 +127,11 @@ struct pgpu_ctx {
   std::vector<int> sys_shape;
   std::vector<int> groups;
   int grid[kNumShapes] = {0};
+  // no shape was asked for or tuned: small FP32C Gaussian systems may take
+  // the slices kernel (choose_slices); slices is its variant, -1 for none
+  bool auto_shape = true;
+  int slices = -1;
+  int grid_slices[kNumSlices] = {0};
   int nch = 1;
   bool plan_dirty = true;
   bool timing = true;
@@ -321,6 +336,15 @@ int freeze(pgpu_ctx *c) {
   CK(cudaMemsetAsync(c->d_nfull, 0, sizeof(unsigned long long), c->st));
   CK(cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->st));
   for (int s = 0; s < kNumShapes; ++s) c->grid[s] = fp64(c) ? occupancy<double>(c, s) : occupancy<float>(c, s);
+  if (uses_boxes(c)) {
+    for (int v = 0; v < kNumSlices; ++v) {
+      int nb = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, slices_fn(v, uses_split(c)), 32 * kSliceWarps, 0) != cudaSuccess ||
+          nb < 1)
+        nb = 1;
+      c->grid_slices[v] = nb * c->sms;
+    }
+  }
   c->frozen = true;
   c->plan_dirty = true;
   return PGPU_OK;
@@ -371,6 +395,7 @@ std::vector<PlanEntry> build_plan(const pgpu_ctx *c, const std::vector<int> &sys
     e.chunk = ceil_div(ceil_div(n, nch), TILE) * TILE;
     e.toff = t.first;
     e.tn = t.second;
+    e.mult = 0;
     item += e.tiles * nch;
     plan.push_back(e);
   }
@@ -412,10 +437,80 @@ std::vector<int> group_systems(const pgpu_ctx *c, int g) {
 // Graph key part that fixes the launch sequence of one evaluation: the single
 // shape, or the set of group shapes.
 int launch_layout(const pgpu_ctx *c) {
+  if (c->slices >= 0) return 2000 + c->slices;
   if (c->groups.empty()) return c->shape;
   int mask = 0;
   for (int g : c->groups) mask |= 1 << g;
   return 1000 + mask;
+}
+
+// Work list of the slices kernel over every system, in the context's order:
+// rows per system, an equal run of rows per CTA, and in *nch the partials a
+// tile's rows can be split over.
+std::vector<PlanEntry> build_slices_plan(const pgpu_ctx *c, int variant, int *nch) {
+  const int64_t TT = 32, RS = (int64_t)kSliceLen[variant] * kSliceWarps;  // targets and sources per row
+  std::vector<PlanEntry> plan;
+  int64_t rows = 0, rps_max = 1;
+  for (int s = 0; s < (int)c->sys.size(); ++s) {
+    const int64_t n = sys_n(c, s);
+    const auto t = owned(c, s);
+    if (n <= 0 || t.second <= 0) continue;
+    PlanEntry e;
+    e.off = c->sys[s].off;
+    e.n = n;
+    e.item_start = rows;
+    e.tiles = ceil_div(t.second, TT);
+    e.chunk = ceil_div(n, RS);
+    e.toff = t.first;
+    e.tn = t.second;
+    // a step near the golden section of the rows, coprime to their number,
+    // scatters any run of rows over the system
+    e.mult = std::max<int64_t>(1, (int64_t)(0.618 * (double)e.chunk));
+    while (std::gcd(e.mult, e.chunk) != 1) ++e.mult;
+    e.mult %= e.chunk;
+    rows += e.tiles * e.chunk;
+    rps_max = std::max(rps_max, e.chunk);
+    plan.push_back(e);
+  }
+  PlanEntry sentinel{};
+  sentinel.item_start = rows;
+  // at most kMaxChunks partials per tile: a tile's rows start anywhere in a CTA's run
+  sentinel.chunk = std::max<int64_t>(
+      1, std::max(ceil_div(rows, c->grid_slices[variant]), ceil_div(rps_max, kMaxChunks - 1)));
+  *nch = 1;
+  for (const PlanEntry &e : plan)
+    *nch = std::max(*nch, (int)std::min(e.chunk, ceil_div(e.chunk, sentinel.chunk) + 1));
+  plan.push_back(sentinel);
+  return plan;
+}
+
+// Variant of the slices kernel for the context's next evaluations, -1 for the
+// CTA-wide tiles of pair_kernel.  Times per evaluation, CTA-wide 128 x 2 tiles
+// / 32-source / 64-source slices, in us:
+//   Gaussian rings (sigma = 0.02)  5000: 127 / 55 / 61;  8000: 184 / 110 / 106;
+//     20,000: 658 / 575 / 541;  40,000: 2103 / 2228 / 2065;  60,000: 4388 / 4982 / 4593
+//   station rings (sigma = 0.1)  1000: 53 / 17 / 19;  5000: 167 / 62 / 66;
+//     20,000: 850 / 687 / 658;  40,000: 2856 / 2701 / 2541
+//   rotor wakes, split positions  4800: 168 / 58 / 72;  24,000: 1308 / 931 / 949;
+//     200,000: 76,306 / 58,493 / 58,840
+// The CTA-wide tiles need about 24 items per CTA to fill the device and gain
+// two targets per staged source; the slices' finer boxes find more far pairs.
+// So dense filaments (split positions) take 32-source slices at any size, and
+// the others slices while all systems together have fewer than 48,000 targets
+// (16 rings of 2000-32,000, 160,000 in all: 5.8 ms in tiles, 6.3 ms in slices),
+// 64-source ones above 45 million pairs.  A shape or chunk count that was asked
+// for, and a tuned shape, keep the tiles.
+int choose_slices(const pgpu_ctx *c) {
+  if (!c->auto_shape || c->cfg.chunks > 0 || !uses_boxes(c) || c->sur) return -1;
+  if (uses_split(c)) return 0;
+  double pairs = 0.0, targets = 0.0;
+  for (int s = 0; s < (int)c->sys.size(); ++s) {
+    const double tn = (double)owned(c, s).second;
+    pairs += tn * (double)sys_n(c, s);
+    targets += tn;
+  }
+  if (targets > 48000.0) return -1;
+  return pairs < 4.5e7 ? 0 : 1;
 }
 
 int upload_plan(pgpu_ctx *c) {
@@ -434,7 +529,11 @@ int upload_plan(pgpu_ctx *c) {
     }
   }
   std::vector<PlanEntry> plan;
-  if (c->groups.empty()) {
+  c->slices = c->groups.empty() ? choose_slices(c) : -1;
+  if (c->slices >= 0) {
+    plan = build_slices_plan(c, c->slices, &c->nch);
+    plan.resize(ns + 1, plan.back());
+  } else if (c->groups.empty()) {
     // the surrogate writes one chunk of rates per evaluation
     c->nch = c->sur ? 1 : choose_nch(c, c->shape);
     plan = build_plan(c, all_systems(c), c->shape, c->nch);
@@ -492,7 +591,7 @@ int launch_boxes(pgpu_ctx *c) {
 
 // Kernel launches of one rate evaluation by the direct sum.
 int64_t eval_launches(const pgpu_ctx *c) {
-  return (int64_t)std::max<size_t>(1, c->groups.size()) + (uses_boxes(c) ? 1 : 0);
+  return (int64_t)std::max<size_t>(1, c->groups.size()) + (uses_boxes(c) && c->slices < 0 ? 1 : 0);
 }
 
 template <typename T> int launch_pair(pgpu_ctx *c, int slot) {
@@ -507,7 +606,7 @@ template <typename T> int launch_pair(pgpu_ctx *c, int slot) {
   a.nu2 = (T)(2.0 * c->cfg.nu);
   a.counters = c->d_counters;
   a.nfull = c->d_nfull;
-  if (uses_boxes(c)) {
+  if (uses_boxes(c) && c->slices < 0) {
     // source boxes of the current records, ahead of (and outside the timing of) the pair launch
     int r = launch_boxes(c);
     if (r) return r;
@@ -518,7 +617,13 @@ template <typename T> int launch_pair(pgpu_ctx *c, int slot) {
   // the graph when it is marked external.
   const unsigned flags = c->capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
   if (c->timing && slot >= 0) CK(cudaEventRecordWithFlags(c->ev[slot][0], c->st, flags));
-  if (c->groups.empty()) {
+  if (c->slices >= 0) {
+    if constexpr (sizeof(T) == 4) {
+      slices_fn(c->slices, uses_split(c))<<<c->grid_slices[c->slices], 32 * kSliceWarps, 0, c->st>>>(a);
+      CK(cudaGetLastError());
+      c->launches++;
+    }
+  } else if (c->groups.empty()) {
     pair_fn<T>(c->shape, c->cfg.kernel, uses_split(c))<<<c->grid[c->shape], kShapes[c->shape].block, 0, c->st>>>(a);
     CK(cudaGetLastError());
     c->launches++;
@@ -546,10 +651,9 @@ int launch_stage(pgpu_ctx *c, int scheme, int stage, double dt) {
   s.nch = c->nch; s.cap = c->cap; s.scheme = scheme; s.stage = stage; s.dt = dt;
   for (int m = 0; m < 3; ++m) s.vinf[m] = c->cfg.vinf[m];
   s.flag = c->d_flag;
-  const int block = 256;
-  const int grid = (int)std::min<int64_t>(ceil_div(c->cap, block), 16LL * c->sms);
-  if (fp64(c)) stage_kernel<double><<<grid, block, 0, c->st>>>(s);
-  else stage_kernel<float><<<grid, block, 0, c->st>>>(s);
+  const int grid = (int)std::min<int64_t>(ceil_div(c->cap, kStageParticles), 10LL * c->sms);
+  if (fp64(c)) stage_kernel<double><<<grid, kStageBlock, 0, c->st>>>(s);
+  else stage_kernel<float><<<grid, kStageBlock, 0, c->st>>>(s);
   CK(cudaGetLastError());
   c->launches++;
   return PGPU_OK;
@@ -655,6 +759,7 @@ int pgpu_create(pgpu_ctx **out, const pgpu_config *cfg) {
       return create_fail(c, PGPU_EINVAL, "no compiled pair-kernel shape with block %d and %d targets per thread",
                          c->cfg.block, c->cfg.tpt);
     c->shape = found;
+    c->auto_shape = false;
   } else if (c->cfg.kernel == PGPU_KERNEL_GAUSSIAN) {
     // untuned defaults: the fastest Gaussian shapes on the 1M ring, FP32C
     // 128 x 2 (1075 ms per evaluation against 1163 ms for 256 x 1) and FP64
@@ -1299,6 +1404,7 @@ int pgpu_autotune(pgpu_ctx *c, int reps, int *block, int *tpt, double *ms_per_la
   if (!c->frozen) return fail(c, PGPU_EINVAL, "no particles were uploaded");
   if (reps < 1) reps = 1;
   c->sys_shape.clear();  // one shape for every system from here on
+  c->auto_shape = false;
   const int saved = c->shape;
   double best = 1e300;
   int best_s = saved;
@@ -1501,6 +1607,7 @@ int pgpu_autotune_classes(pgpu_ctx *c, int reps, const char *cache_path, pgpu_tu
   }
   // one launch per class shape only if the single shape loses more than 2%
   // on some class
+  c->auto_shape = false;
   bool split = false;
   for (size_t i = 0; i < K; ++i)
     if (tms[i][single] > 1.02 * tms[i][best[i]]) split = true;

@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
             r2 = __ffma2_rn(dy, dy, r2);
             r2 = __ffma2_rn(dz, dz, r2);
             const float2 s2 = __fadd2_rn(HS2, make_float2(pb.z, pb.w));
-            PairTerms2 t = pair_terms_mid2(r2, s2);
+            PairTerms2 t = pair_terms_mid2(r2, mid_sigma2(s2));
             const bool lx = r2.x < s2.x, ly = r2.y < s2.y;  // u < 1
             if (__any_sync(0xffffffffu, lx || ly)) {
               if (lx) { const PairTerms<float> e = pair_terms_near(r2.x, s2.x); t.q.x = e.q; t.F.x = e.F; t.zd.x = e.zd; }

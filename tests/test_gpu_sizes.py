@@ -38,3 +38,54 @@ def test_probe_tiles_and_chunks(gpu, n, npts, kernel):
     rows[0] = 0
     ref = np.array([O.restate_getvi(rest if k == 0 else w, pts[k], kernel) for k in rows])
     assert np.abs(v[rows] - ref).max() <= 1e-11 * np.abs(v).max()
+
+
+def check_rates(c, k, w, rows, tol=1e-5):
+    v, a = c.rates(k)
+    rv, ra = O.restate_rates(w, NU, targets=rows)
+    scale_v, scale_a = np.abs(v).max(), np.abs(a).max()
+    assert np.abs(v[rows] - rv).max() <= tol * scale_v
+    assert np.abs(a[rows] - ra).max() <= tol * scale_a
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("n", [25, 31, 33, 255, 257, 1000, 6700, 6720, 20011, 48000, 48001])
+def test_rates_row_list(gpu, n, split):
+    """The row list of small systems: below one row, ragged tiles and slices, and both sides of every rule."""
+    w = ring(n)
+    w.sigma[: n // 3] = 0.08  # slices of one radius and of two
+    c, ids = context([w], capi.FP32C, split_positions=split)
+    c.solve()
+    rows = np.unique(np.linspace(0, n - 1, 40).astype(np.int64))
+    check_rates(c, ids[0], w, rows)
+
+
+def test_rates_row_list_batch(gpu):
+    """Systems of very uneven sizes in one row list, RK3 steps of the batch as of each system alone."""
+    wakes = [ring(n, seed=n) for n in (400, 25, 5003, 64, 12000)]
+    c, ids = context(wakes, capi.FP32C)
+    c.solve()
+    for k, w in zip(ids, wakes):
+        check_rates(c, k, w, np.unique(np.linspace(0, w.n - 1, 20).astype(np.int64)))
+    c.step("rk3", 0.01, 2)
+    c.sync()
+    for k, w in zip(ids, wakes):
+        one, one_id = context([w], capi.FP32C)
+        one.step("rk3", 0.01, 2)
+        one.sync()
+        for x, y in zip(c.state(k), one.state(one_id[0])):
+            assert np.abs(x - y).max() <= 1e-6 * np.abs(y).max()
+
+
+@pytest.mark.parametrize("first,count", [(0, 1), (37, 33), (0, 20000), (19990, 10)])
+def test_rates_row_list_target_range(gpu, first, count):
+    """Few owned targets of many sources: a tile's rows are split over at most 16 partials."""
+    w = ring(20000)
+    c, ids = context([w], capi.FP32C)
+    c.set_target_range(0, first, count)
+    c.solve()
+    v, a = c.rates(ids[0])
+    rows = np.unique(np.linspace(first, first + count - 1, 20).astype(np.int64))
+    rv, ra = O.restate_rates(w, NU, targets=rows)
+    assert np.abs(v[rows] - rv).max() <= 1e-5 * np.abs(rv).max()
+    assert np.abs(a[rows] - ra).max() <= 1e-5 * np.abs(ra).max()
