@@ -296,7 +296,9 @@ int pgpu_pair_counts(pgpu_ctx *ctx, int64_t *pairs, int64_t *full_pairs);
 int64_t pgpu_launch_count(pgpu_ctx *ctx);
 
 /* Times every compiled pair-kernel shape on the current particles (`reps`
- * launches each) and selects the fastest for subsequent solves and steps.
+ * launches each) and selects the fastest for subsequent solves and steps; a
+ * context that was not asked for a shape keeps the library's own choice where
+ * that is faster than every shape (block and tpt then give the fastest shape).
  * block/tpt receive the choice; ms_per_launch (may be NULL) receives the
  * time of each candidate in the order of pgpu_kernel_shapes. */
 int pgpu_autotune(pgpu_ctx *ctx, int reps, int *block, int *tpt, double *ms_per_launch);

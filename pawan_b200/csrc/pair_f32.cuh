@@ -82,6 +82,108 @@ __device__ __forceinline__ void far_pair2(float2 px, float2 py, float2 pz, float
   sd[2] = __ffma2_rn(fd, dz, sd[2]);
 }
 
+// Two pairs at once of the high-order kernel (pair_terms_ho): with R =
+// rho^2 + sigma^2, q' = (R + 1.5 sigma^2) R^-2.5, F'/-3 = (R + 2.5 sigma^2)
+// R^-3.5 and zd'/52.5 = sigma^4 R^-4.5.  zx, zy: lanes at rho = 0, whose terms
+// are all zero.
+struct HoTerms2 {
+  float2 q, F3, zd;
+};
+__device__ __forceinline__ HoTerms2 ho_terms2(float2 R, float2 s2, bool zx, bool zy) {
+  float2 iR = make_float2(fast_rsqrt(R.x), fast_rsqrt(R.y));
+  const float2 h = __fmul2_rn(__fmul2_rn(R, dup2(-0.5f)), iR);
+  iR = __fmul2_rn(iR, __ffma2_rn(h, iR, dup2(1.5f)));  // one Newton step, as rsqrt_nr
+  iR.x = zx ? 0.f : iR.x;
+  iR.y = zy ? 0.f : iR.y;
+  const float2 iR2 = __fmul2_rn(iR, iR);
+  const float2 iR5 = __fmul2_rn(__fmul2_rn(iR2, iR2), iR);
+  const float2 iR7 = __fmul2_rn(iR5, iR2);
+  HoTerms2 o;
+  o.q = __fmul2_rn(__ffma2_rn(s2, dup2(1.5f), R), iR5);
+  o.F3 = __fmul2_rn(__ffma2_rn(s2, dup2(2.5f), R), iR7);
+  o.zd = __fmul2_rn(__fmul2_rn(s2, s2), __fmul2_rn(iR7, iR2));
+  return o;
+}
+
+// One source pair on one target, high-order kernel, in slices far from the
+// target (the far limit's box test; the high-order kernel has no far limit, but
+// there the products formed from the reference point lose nothing, as in
+// far_pair2): 42 packed operations.  AT = alpha_t, B = X' x alpha_t; sums: sp
+// q alpha_s, sv q n, sd (F/-3) dot d, sz zd alpha_s, sw zd v_s.
+__device__ __forceinline__ void ho_far_pair2(float2 px, float2 py, float2 pz, float2 ph, float2 ax, float2 ay,
+                                             float2 az, float2 av, float2 nx, float2 ny, float2 nz, const float2 *X,
+                                             float hst, const float2 *AT, const float2 *B, float2 *sv, float2 *sd,
+                                             float2 *sp, float2 *sz, float2 &sw) {
+  const float2 M1 = make_float2(-1.f, -1.f);
+  const float2 dx = __ffma2_rn(px, M1, X[0]);
+  const float2 dy = __ffma2_rn(py, M1, X[1]);
+  const float2 dz = __ffma2_rn(pz, M1, X[2]);
+  const float2 s2 = __fadd2_rn(dup2(hst), ph);
+  float2 R = __ffma2_rn(dx, dx, s2);
+  R = __ffma2_rn(dy, dy, R);
+  R = __ffma2_rn(dz, dz, R);
+  const HoTerms2 t = ho_terms2(R, s2, false, false);
+  sp[0] = __ffma2_rn(t.q, ax, sp[0]);
+  sp[1] = __ffma2_rn(t.q, ay, sp[1]);
+  sp[2] = __ffma2_rn(t.q, az, sp[2]);
+  sv[0] = __ffma2_rn(t.q, nx, sv[0]);
+  sv[1] = __ffma2_rn(t.q, ny, sv[1]);
+  sv[2] = __ffma2_rn(t.q, nz, sv[2]);
+  float2 dot = __fmul2_rn(ax, B[0]);
+  dot = __ffma2_rn(ay, B[1], dot);
+  dot = __ffma2_rn(az, B[2], dot);
+  dot = __ffma2_rn(nx, AT[0], dot);
+  dot = __ffma2_rn(ny, AT[1], dot);
+  dot = __ffma2_rn(nz, AT[2], dot);
+  const float2 fd = __fmul2_rn(t.F3, dot);
+  sd[0] = __ffma2_rn(fd, dx, sd[0]);
+  sd[1] = __ffma2_rn(fd, dy, sd[1]);
+  sd[2] = __ffma2_rn(fd, dz, sd[2]);
+  sz[0] = __ffma2_rn(t.zd, ax, sz[0]);
+  sz[1] = __ffma2_rn(t.zd, ay, sz[1]);
+  sz[2] = __ffma2_rn(t.zd, az, sz[2]);
+  sw = __ffma2_rn(t.zd, av, sw);
+}
+
+// The same in the other slices: cross products and the diffusion's difference
+// per pair, from the pair's own distance (58 operations).
+__device__ __forceinline__ void ho_near_pair2(float2 px, float2 py, float2 pz, float2 ph, float2 ax, float2 ay,
+                                              float2 az, float2 av, const float2 *X, const float *at, float hst,
+                                              float vt, const float2 *AT, float2 *sv, float2 *sd, float2 *sp,
+                                              float2 *sz) {
+  const float2 M1 = make_float2(-1.f, -1.f);
+  const float2 dx = __ffma2_rn(px, M1, X[0]);
+  const float2 dy = __ffma2_rn(py, M1, X[1]);
+  const float2 dz = __ffma2_rn(pz, M1, X[2]);
+  float2 r2 = __fmul2_rn(dx, dx);
+  r2 = __ffma2_rn(dy, dy, r2);
+  r2 = __ffma2_rn(dz, dz, r2);
+  const float2 s2 = __fadd2_rn(dup2(hst), ph);
+  const HoTerms2 t = ho_terms2(__fadd2_rn(r2, s2), s2, !(r2.x > 0.f), !(r2.y > 0.f));
+  const float2 wx = make_float2(ay.x * dz.x - az.x * dy.x, ay.y * dz.y - az.y * dy.y);
+  const float2 wy = make_float2(az.x * dx.x - ax.x * dz.x, az.y * dx.y - ax.y * dz.y);
+  const float2 wz = make_float2(ax.x * dy.x - ay.x * dx.x, ax.y * dy.y - ay.y * dx.y);
+  sv[0] = __ffma2_rn(t.q, wx, sv[0]);
+  sv[1] = __ffma2_rn(t.q, wy, sv[1]);
+  sv[2] = __ffma2_rn(t.q, wz, sv[2]);
+  float2 dot = __fmul2_rn(AT[0], wx);
+  dot = __ffma2_rn(AT[1], wy, dot);
+  dot = __ffma2_rn(AT[2], wz, dot);
+  const float2 fd = __fmul2_rn(t.F3, dot);
+  sd[0] = __ffma2_rn(fd, dx, sd[0]);
+  sd[1] = __ffma2_rn(fd, dy, sd[1]);
+  sd[2] = __ffma2_rn(fd, dz, sd[2]);
+  const float2 cx = make_float2(at[1] * az.x - at[2] * ay.x, at[1] * az.y - at[2] * ay.y);
+  const float2 cy = make_float2(at[2] * ax.x - at[0] * az.x, at[2] * ax.y - at[0] * az.y);
+  const float2 cz = make_float2(at[0] * ay.x - at[1] * ax.x, at[0] * ay.y - at[1] * ax.y);
+  sp[0] = __ffma2_rn(t.q, cx, sp[0]);
+  sp[1] = __ffma2_rn(t.q, cy, sp[1]);
+  sp[2] = __ffma2_rn(t.q, cz, sp[2]);
+  sz[0] = __ffma2_rn(t.zd, make_float2(vt * ax.x - av.x * at[0], vt * ax.y - av.y * at[0]), sz[0]);
+  sz[1] = __ffma2_rn(t.zd, make_float2(vt * ay.x - av.x * at[1], vt * ay.y - av.y * at[1]), sz[1]);
+  sz[2] = __ffma2_rn(t.zd, make_float2(vt * az.x - av.x * at[2], vt * az.y - av.y * at[2]), sz[2]);
+}
+
 // B3 = X' x (-3 alpha_t), duplicated into both lanes.
 __device__ __forceinline__ void far_b3(float xr0, float xr1, float xr2, const float2 *AT3, float2 *B3) {
   const float c0 = AT3[0].x, c1 = AT3[1].x, c2 = AT3[2].x;

@@ -14,6 +14,11 @@
 // The arithmetic is that of pair_f32.cuh: packed far limit for slices whose box
 // is far from the targets' box, closed form for the others, one compensation
 // group per slice.  The order of every sum is fixed by the sizes.
+//
+// High-order kernel (KER): every pair takes its full terms, two sources per
+// packed instruction, 42 FP32 operations in slices far from the targets and 58
+// in the others, against 68 scalar instructions in the generic body; no pair
+// is cheap enough for wider tiles to pay, so it takes these slices at any size.
 #pragma once
 
 namespace pgpu {
@@ -40,12 +45,58 @@ __device__ __forceinline__ void reduce_box(WarpBox &b) {
   b.hs = warp_max(b.hs);
 }
 
+// The rows of one target tile that a CTA takes: from `row` up to its own end
+// row1 or the tile's last row.
+struct RowRun {
+  PlanEntry pe;
+  int64_t first;  // the tile's first row
+  int64_t t0, tend, s1;  // first target of the tile, ends of the targets and of the sources
+  // Row r holds the slices of group (r mult) mod rows-per-tile: any run of rows
+  // samples the whole system evenly, so the slices around the tile, which
+  // take the closed form, spread over the CTAs.
+  int64_t g;
+  int nrows;
+  int c;  // this CTA's partial of the tile
+  bool last;  // holds the tile's last row
+};
+__device__ __forceinline__ RowRun row_run(const PlanEntry *plan, int nsys, int64_t rpc, int64_t row, int64_t row1) {
+  RowRun r;
+  r.pe = plan[find_plan(plan, nsys, row)];
+  const int64_t rps = r.pe.chunk;  // rows per target tile
+  const int64_t tile = (row - r.pe.item_start) / rps;
+  r.first = r.pe.item_start + tile * rps;
+  r.t0 = r.pe.off + r.pe.toff + tile * 32;
+  r.tend = r.pe.off + r.pe.toff + r.pe.tn;
+  r.s1 = r.pe.off + r.pe.n;
+  r.g = ((row - r.first) * r.pe.mult) % rps;
+  r.nrows = (int)(min(r.first + rps, row1) - row);
+  r.c = (int)(row / rpc - r.first / rpc);
+  r.last = row + r.nrows == r.first + rps;
+  return r;
+}
+// The CTA's sums of a tile, red[warp][component][target], in warp order into
+// its partial; the CTA of the tile's last row also clears the partials that
+// no CTA has.
+__device__ __forceinline__ void row_run_sums(const RowRun &r, const double *red, double *partial, int64_t cap, int nch) {
+  const int clear = r.last ? nch : r.c + 1;
+  for (int e = threadIdx.x; e < 6 * 32; e += 32 * kSliceWarps) {
+    double v = 0.0;
+#pragma unroll
+    for (int k = 0; k < kSliceWarps; ++k) v += red[k * 6 * 32 + e];
+    const int64_t i = r.t0 + e % 32;
+    if (i >= r.tend) continue;
+    double *o = partial + (e / 32) * cap + i;
+    o[r.c * 6 * cap] = v * kInv4Pi;
+    for (int k = r.c + 1; k < clear; ++k) o[k * 6 * cap] = 0.0;
+  }
+}
+
 template <int SL, bool SPLIT> struct SliceStage {
   float4 P[32 * SL], Q[32 * SL], N[32 * SL];  // pair-interleaved as in pair_f32.cuh
   float4 L[SPLIT ? 32 * SL : 1];
 };
 
-template <int SL, bool SPLIT>
+template <int SL, bool SPLIT, int KER = kGaussian>
 __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairArgs<float> a) {
   constexpr int W = kSliceWarps, S = 32 * SL, TT = 32;
   using Stage = SliceStage<SL, SPLIT>;
@@ -58,19 +109,9 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
   const int64_t rpc = a.plan[a.nsys].chunk;
   const int64_t row1 = min((blockIdx.x + 1) * rpc, a.plan[a.nsys].item_start);
   for (int64_t row = blockIdx.x * rpc; row < row1;) {
-    const PlanEntry pe = a.plan[find_plan(a.plan, a.nsys, row)];
-    const int64_t rps = pe.chunk;  // rows per target tile
-    const int64_t tile = (row - pe.item_start) / rps;
-    const int64_t first = pe.item_start + tile * rps;  // the tile's first row
-    const int nrows = (int)(min(first + rps, row1) - row);
-    const int c = (int)(row / rpc - first / rpc);  // this CTA's partial of the tile
-    const int64_t t0 = pe.off + pe.toff + tile * TT;
-    const int64_t tend = pe.off + pe.toff + pe.tn;  // end of the targets
-    const int64_t s1 = pe.off + pe.n;
-    // Row r holds the slices of group (r mult) mod rps: any run of rows
-    // samples the whole system evenly, so the slices around the tile, which
-    // take the closed form, spread over the CTAs.
-    int64_t g = ((row - first) * pe.mult) % rps;
+    const RowRun run = row_run(a.plan, a.nsys, rpc, row, row1);
+    const int64_t s1 = run.s1;
+    int64_t g = run.g;
 
     // this lane's share of a slice, fetched ahead of the slice in work
     float4 gp[SL], gq[SL], gl[SPLIT ? SL : 1];
@@ -83,16 +124,21 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
         if constexpr (SPLIT) gl[j] = i < s1 ? a.L[i] : pad_Q<float>();
       }
     };
-    int64_t sb = pe.off + (g * W + w) * S;
+    int64_t sb = run.pe.off + (g * W + w) * S;
     if (sb < s1) fetch(sb);
 
-    const int64_t ti = min(t0 + lane, tend - 1);
+    const int64_t ti = min(run.t0 + lane, run.tend - 1);
     const float4 pt = a.P[ti], qt = a.Q[ti];
     float4 lt = pad_Q<float>();
     if constexpr (SPLIT) lt = a.L[ti];
     const float at[3] = {qt.x, qt.y, qt.z}, xl[3] = {lt.x, lt.y, lt.z};
     const float2 X[3] = {dup2(pt.x), dup2(pt.y), dup2(pt.z)};
-    const float2 AT3[3] = {dup2(-3.f * qt.x), dup2(-3.f * qt.y), dup2(-3.f * qt.z)};
+    // Gaussian: -3 alpha_t, the far limit's constant folded in.  High-order: the
+    // -3 of F waits for the fold, since the rounding of -3 alpha_t would turn
+    // alpha_t for every source alike (norm-wise error of dalpha on the
+    // 5000-particle ring: 2.3e-6 with it, 1.1e-6 without).
+    constexpr float kAt = KER == kHighOrder ? 1.f : -3.f;
+    const float2 AT[3] = {dup2(kAt * qt.x), dup2(kAt * qt.y), dup2(kAt * qt.z)};
     float vh[3] = {0.f, 0.f, 0.f}, vl[3] = {0.f, 0.f, 0.f}, dh[3] = {0.f, 0.f, 0.f}, dl[3] = {0.f, 0.f, 0.f};
     unsigned nfull = 0;
     WarpBox tb;
@@ -101,13 +147,13 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
     reduce_box(tb);
     const float thmin = warp_min(pt.w);
 
-    for (int r = 0; r < nrows; ++r) {
+    for (int r = 0; r < run.nrows; ++r) {
       const int64_t cur = sb;
-      g += pe.mult;
-      if (g >= rps) g -= rps;
-      sb = pe.off + (g * W + w) * S;
+      g += run.pe.mult;
+      if (g >= run.pe.chunk) g -= run.pe.chunk;
+      sb = run.pe.off + (g * W + w) * S;
       if (cur >= s1) {  // past the last source: this warp has no slice in the row
-        if (r + 1 < nrows && sb < s1) fetch(sb);
+        if (r + 1 < run.nrows && sb < s1) fetch(sb);
         continue;
       }
       __syncwarp();
@@ -140,23 +186,55 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
       reduce_box(sbox);
       const bool far = all_far(tb, sbox);
       __syncwarp();
-      if (r + 1 < nrows && sb < s1) fetch(sb);
+      if (r + 1 < run.nrows && sb < s1) fetch(sb);
       const int npr = (int)(min((int64_t)S, s1 - cur) + 1) >> 1;  // an odd tail pairs with a padding source
 
       float2 sv[3], sd[3], sp[3];
       float sdv[3] = {0.f, 0.f, 0.f};
 #pragma unroll
       for (int m = 0; m < 3; ++m) sv[m] = sd[m] = sp[m] = dup2(0.f);
-      if (far) {
+      if constexpr (KER == kHighOrder) {
+        float2 zs[3] = {dup2(0.f), dup2(0.f), dup2(0.f)};
+        if (far) {
+          float2 B[3], sw = dup2(0.f);
+          far_b3(pt.x - rx, pt.y - ry, pt.z - rz, AT, B);
+#pragma unroll 2
+          for (int r = 0; r < npr; ++r) {
+            const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1],
+                         na = st.N[2 * r], nb = st.N[2 * r + 1];
+            ho_far_pair2(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y),
+                         make_float2(pb.z, pb.w), make_float2(qa.x, qa.y), make_float2(qa.z, qa.w),
+                         make_float2(qb.x, qb.y), make_float2(qb.z, qb.w), make_float2(na.x, na.y),
+                         make_float2(na.z, na.w), make_float2(nb.x, nb.y), X, pt.w, AT, B, sv, sd, sp, zs, sw);
+          }
+#pragma unroll
+          for (int m = 0; m < 3; ++m) sdv[m] = qt.w * (zs[m].x + zs[m].y) - (sw.x + sw.y) * at[m];
+        } else {
+#pragma unroll 2
+          for (int r = 0; r < npr; ++r) {
+            const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1];
+            ho_near_pair2(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y),
+                          make_float2(pb.z, pb.w), make_float2(qa.x, qa.y), make_float2(qa.z, qa.w),
+                          make_float2(qb.x, qb.y), make_float2(qb.z, qb.w), X, at, pt.w, qt.w, AT, sv, sd, sp, zs);
+          }
+#pragma unroll
+          for (int m = 0; m < 3; ++m) sdv[m] = zs[m].x + zs[m].y;
+        }
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          sdv[m] *= (float)HighOrder::kZd;
+          sd[m] = __fmul2_rn(sd[m], dup2(-3.f));
+        }
+      } else if (far) {
         float2 B3[3];
-        far_b3(pt.x - rx, pt.y - ry, pt.z - rz, AT3, B3);
+        far_b3(pt.x - rx, pt.y - ry, pt.z - rz, AT, B3);
 #pragma unroll 2
         for (int r = 0; r < npr; ++r) {
           const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1],
                        na = st.N[2 * r], nb = st.N[2 * r + 1];
           far_pair2(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y),
                     make_float2(qa.x, qa.y), make_float2(qa.z, qa.w), make_float2(qb.x, qb.y),
-                    make_float2(na.x, na.y), make_float2(na.z, na.w), make_float2(nb.x, nb.y), X, AT3, B3, sv, sd, sp);
+                    make_float2(na.x, na.y), make_float2(na.z, na.w), make_float2(nb.x, nb.y), X, AT, B3, sv, sd, sp);
         }
       } else {
         float2 sdv2[3] = {dup2(0.f), dup2(0.f), dup2(0.f)};
@@ -199,20 +277,9 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
       red[(w * 6 + 3 + m) * TT + lane] = (double)dh[m] + (double)dl[m];
     }
     __syncthreads();
-    // the CTA of the tile's last row also clears the partials no CTA has
-    const int clear = row + nrows == first + rps ? a.nch : c + 1;
-    for (int e = threadIdx.x; e < 6 * TT; e += 32 * W) {
-      double v = 0.0;
-#pragma unroll
-      for (int k = 0; k < W; ++k) v += red[k * 6 * TT + e];
-      const int64_t i = t0 + e % TT;
-      if (i >= tend) continue;
-      double *o = a.partial + (e / TT) * a.cap + i;
-      o[c * 6 * a.cap] = v * kInv4Pi;
-      for (int k = c + 1; k < clear; ++k) o[k * 6 * a.cap] = 0.0;
-    }
+    row_run_sums(run, red, a.partial, a.cap, a.nch);
     __syncthreads();  // before the next tile's slices overwrite the sums
-    row += nrows;
+    row += run.nrows;
   }
 }
 

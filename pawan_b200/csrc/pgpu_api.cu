@@ -74,7 +74,9 @@ template <typename T> PairFn<T> pair_fn(int s, int ker, bool split) {
 // source per lane, with or without split positions, and 64-source ones.
 constexpr int kSliceLen[] = {32, 64};
 constexpr int kNumSlices = 2;
-PairFn<float> slices_fn(int v, bool split) {
+PairFn<float> slices_fn(int v, int ker, bool split) {
+  if (ker == PGPU_KERNEL_HIGHORDER)
+    return v == 0 ? pair_slices_kernel<1, false, kHighOrder> : pair_slices_kernel<2, false, kHighOrder>;
   if (split) return pair_slices_kernel<1, true>;
   return v == 0 ? pair_slices_kernel<1, false> : pair_slices_kernel<2, false>;
 }
@@ -336,10 +338,10 @@ int freeze(pgpu_ctx *c) {
   CK(cudaMemsetAsync(c->d_nfull, 0, sizeof(unsigned long long), c->st));
   CK(cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->st));
   for (int s = 0; s < kNumShapes; ++s) c->grid[s] = fp64(c) ? occupancy<double>(c, s) : occupancy<float>(c, s);
-  if (uses_boxes(c)) {
+  if (!fp64(c)) {
     for (int v = 0; v < kNumSlices; ++v) {
       int nb = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, slices_fn(v, uses_split(c)), 32 * kSliceWarps, 0) != cudaSuccess ||
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, slices_fn(v, c->cfg.kernel, uses_split(c)), 32 * kSliceWarps, 0) != cudaSuccess ||
           nb < 1)
         nb = 1;
       c->grid_slices[v] = nb * c->sms;
@@ -499,9 +501,11 @@ std::vector<PlanEntry> build_slices_plan(const pgpu_ctx *c, int variant, int *nc
 // the others slices while all systems together have fewer than 48,000 targets
 // (16 rings of 2000-32,000, 160,000 in all: 5.8 ms in tiles, 6.3 ms in slices),
 // 64-source ones above 45 million pairs.  A shape or chunk count that was asked
-// for, and a tuned shape, keep the tiles.
+// for, and a tuned shape, keep the tiles.  The high-order kernel's full terms
+// for every pair take the slices at any size (1000 particles: 14 against 52 us
+// in 256 x 1 tiles; 60,000: 6.4 against 8.1 ms; 400,000: 275 against 345 ms)).
 int choose_slices(const pgpu_ctx *c) {
-  if (!c->auto_shape || c->cfg.chunks > 0 || !uses_boxes(c) || c->sur) return -1;
+  if (!c->auto_shape || c->cfg.chunks > 0 || fp64(c) || c->sur) return -1;
   if (uses_split(c)) return 0;
   double pairs = 0.0, targets = 0.0;
   for (int s = 0; s < (int)c->sys.size(); ++s) {
@@ -509,7 +513,7 @@ int choose_slices(const pgpu_ctx *c) {
     pairs += tn * (double)sys_n(c, s);
     targets += tn;
   }
-  if (targets > 48000.0) return -1;
+  if (targets > 48000.0 && c->cfg.kernel == PGPU_KERNEL_GAUSSIAN) return -1;
   return pairs < 4.5e7 ? 0 : 1;
 }
 
@@ -619,10 +623,10 @@ template <typename T> int launch_pair(pgpu_ctx *c, int slot) {
   if (c->timing && slot >= 0) CK(cudaEventRecordWithFlags(c->ev[slot][0], c->st, flags));
   if (c->slices >= 0) {
     if constexpr (sizeof(T) == 4) {
-      slices_fn(c->slices, uses_split(c))<<<c->grid_slices[c->slices], 32 * kSliceWarps, 0, c->st>>>(a);
-      CK(cudaGetLastError());
-      c->launches++;
+      slices_fn(c->slices, c->cfg.kernel, uses_split(c))<<<c->grid_slices[c->slices], 32 * kSliceWarps, 0, c->st>>>(a);
     }
+    CK(cudaGetLastError());
+    c->launches++;
   } else if (c->groups.empty()) {
     pair_fn<T>(c->shape, c->cfg.kernel, uses_split(c))<<<c->grid[c->shape], kShapes[c->shape].block, 0, c->st>>>(a);
     CK(cudaGetLastError());
@@ -1404,6 +1408,7 @@ int pgpu_autotune(pgpu_ctx *c, int reps, int *block, int *tpt, double *ms_per_la
   if (!c->frozen) return fail(c, PGPU_EINVAL, "no particles were uploaded");
   if (reps < 1) reps = 1;
   c->sys_shape.clear();  // one shape for every system from here on
+  const bool auto_shape = c->auto_shape;
   c->auto_shape = false;
   const int saved = c->shape;
   double best = 1e300;
@@ -1430,6 +1435,24 @@ int pgpu_autotune(pgpu_ctx *c, int reps, int *block, int *tpt, double *ms_per_la
   }
   c->shape = best_s;
   c->plan_dirty = true;
+  if (auto_shape) {
+    // the row list stays where it beats every shape
+    c->auto_shape = true;
+    if ((r = upload_plan(c))) return r;
+    if (c->slices >= 0) {
+      for (int k = 0; k <= reps; ++k) {
+        if ((r = launch_eval(c, 0))) return r;
+        if ((r = collect_timing(c, 1))) return r;
+        if (k == 0) pgpu_pair_kernel_time(c, nullptr, nullptr);  // warm-up
+      }
+      double ms;
+      pgpu_pair_kernel_time(c, &ms, &nl);
+      c->auto_shape = ms / reps <= best;
+    } else {
+      c->auto_shape = false;
+    }
+    c->plan_dirty = true;
+  }
   if ((r = upload_plan(c))) return r;
   // The partial buffer now holds the last candidate's chunks: recompute the
   // rates of the current state with the chosen shape.

@@ -89,3 +89,29 @@ def test_rates_row_list_target_range(gpu, first, count):
     rv, ra = O.restate_rates(w, NU, targets=rows)
     assert np.abs(v[rows] - rv).max() <= 1e-5 * np.abs(rv).max()
     assert np.abs(a[rows] - ra).max() <= 1e-5 * np.abs(ra).max()
+
+
+@pytest.mark.parametrize("n", [25, 33, 257, 1000, 6700, 6720, 20011, 70003])
+def test_rates_row_list_highorder(gpu, n):
+    w = ring(n)
+    w.sigma[: n // 3] = 0.08
+    c, ids = context([w], capi.FP32C, kernel="highorder")
+    c.solve()
+    rows = np.unique(np.linspace(0, n - 1, 40).astype(np.int64))
+    v, a = c.rates(ids[0])
+    rv, ra = O.restate_rates(w, NU, targets=rows, kernel="highorder")
+    assert np.abs(v[rows] - rv).max() <= 1e-5 * np.abs(v).max()
+    assert np.abs(a[rows] - ra).max() <= 1e-5 * np.abs(a).max()
+
+
+def test_autotune_keeps_row_list_or_a_shape(gpu):
+    """After tuning, rates are the untuned ones to FP32 rounding, whichever kernel won."""
+    w = ring(6000)
+    for kernel in ("gaussian", "highorder"):
+        c, ids = context([w], capi.FP32C, kernel=kernel)
+        c.solve()
+        before = c.rates(ids[0])
+        (b, t), ms = c.autotune(reps=1)
+        assert (b, t) in ms
+        for x, y in zip(c.rates(ids[0]), before):
+            assert np.abs(x - y).max() <= 1e-5 * np.abs(y).max()
