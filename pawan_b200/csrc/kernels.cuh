@@ -350,9 +350,7 @@ __device__ __forceinline__ void pair_body_generic(const PairArgs<T> &a) {
               const T dx = xt[k][0] - p.x, dy = xt[k][1] - p.y, dz = xt[k][2] - p.z;
               const T r2 = dx * dx + dy * dy + dz * dz;
               // far limit: q' = r^3, F' = -3 r^5 (the -3 is in at3 and b3), no diffusion
-              T ir;
-              if constexpr (sizeof(T) == 4) ir = fast_rsqrt(r2);
-              else ir = rsqrt(r2);
+              const T ir = fast_rsqrt(r2);
               const T A = ir * ir;
               const T qq = A * ir;
               sp[k][0] += qq * q.x; sp[k][1] += qq * q.y; sp[k][2] += qq * q.z;
@@ -407,13 +405,13 @@ __device__ __forceinline__ void pair_body_generic(const PairArgs<T> &a) {
               // below 1e-16 of q and F); the closed form runs under a vote
               const T s2 = hst[k] + p.w;
               const bool near = r2 < T(kFarU64) * s2;
-              const T ir = rsqrt(r2);
+              const T ir = fast_rsqrt(r2);
               const T A = ir * ir;
               qq = A * ir;
               FF = T(-3) * qq * A;
               if (__any_sync(0xffffffffu, near)) {
                 if (near) {
-                  const PairTerms<T> pt = pair_terms(r2, s2);
+                  const PairTerms<T> pt = pair_terms(r2, s2, ir, fast_rsqrt(s2));
                   qq = pt.q; FF = pt.F;
                   sdv[k][0] += pt.zd * (vt[k] * q.x - q.w * at[k][0]);
                   sdv[k][1] += pt.zd * (vt[k] * q.y - q.w * at[k][1]);
@@ -500,6 +498,7 @@ __device__ __forceinline__ void pair_body_generic(const PairArgs<T> &a) {
 
 #include "pair_f32.cuh"
 #include "pair_slices.cuh"
+#include "pair_slices64.cuh"
 
 namespace pgpu {
 
@@ -811,10 +810,10 @@ __device__ __forceinline__ void diag_body_generic(const DiagArgs<T> &a) {
           }
         } else {
           const bool near = r2 < T(kFarU64) * s2;
-          const T ir = rsqrt(r2);
+          const T ir = fast_rsqrt(r2);
           kq = ir * ir * ir;
           if (__any_sync(0xffffffffu, near && use)) {
-            if (near && use) kq = pair_terms(r2, s2).q;
+            if (near && use) kq = pair_terms(r2, s2, ir, fast_rsqrt(s2)).q;
           }
         }
         const T cx = qt.y * q.z - qt.z * q.y, cy = qt.z * q.x - qt.x * q.z, cz = qt.x * q.y - qt.y * q.x;
@@ -825,7 +824,7 @@ __device__ __forceinline__ void diag_body_generic(const DiagArgs<T> &a) {
         T ir;
         // the enstrophy terms carry R^-4.5: a refined root keeps their FP32 error at rounding level
         if constexpr (sizeof(T) == 4) ir = KER == kHighOrder ? rsqrt_nr(rs) : fast_rsqrt(rs);
-        else ir = rsqrt(rs);
+        else ir = fast_rsqrt(rs);
         const T ir3 = ir * ir * ir;
         if (use) {
           hh -= kq * (dx * cx + dy * cy + dz * cz);
@@ -1211,7 +1210,7 @@ __global__ void __launch_bounds__(kProbeBlock) probe_kernel(const double *x0, co
     const double xs = x0[jj], ys = x0[cap + jj], zs = x0[2 * cap + jj];
     const double ax = valid ? x0[3 * cap + jj] : 0.0, ay = valid ? x0[4 * cap + jj] : 0.0,
                  az = valid ? x0[5 * cap + jj] : 0.0;
-    const double s2 = sig[jj] * sig[jj];
+    const double s2 = sig[jj] * sig[jj], is = fast_rsqrt(s2);
 #pragma unroll
     for (int k = 0; k < kProbePoints; ++k) {
       if (k >= np) break;
@@ -1225,7 +1224,7 @@ __global__ void __launch_bounds__(kProbeBlock) probe_kernel(const double *x0, co
         const double ir = fast_rsqrt(r2);
         q = ir * ir * ir;
         if (__any_sync(0xffffffffu, near)) {
-          if (near) q = pair_terms(r2, s2).q;
+          if (near) q = pair_terms(r2, s2, ir, is).q;
         }
       }
       if (valid) {

@@ -69,13 +69,11 @@ constexpr double kInv2Pi15 = 0.06349363593424097;     // (2 pi)^-1.5
 #define PGPU_T7 -8.158416875522139e-08
 #define PGPU_T8 4.613390495086924e-09
 
-// Threshold on u below which the series is used.  FP32: the closed form keeps
+// Threshold on u below which the FP32 series is used: the closed form keeps
 // ~1e-6 relative accuracy for F at u = 1, and 9 terms of the series are
-// accurate to ~1e-8 on [0, 1].  FP64: at u = 1e-2 the closed form keeps
-// ~3e-14 and 9 terms are exact to rounding.
+// accurate to ~1e-8 on [0, 1].
 template <typename T> struct SeriesCut;
 template <> struct SeriesCut<float> { static constexpr float value = 1.0f; };
-template <> struct SeriesCut<double> { static constexpr double value = 1.0e-2; };
 
 __device__ __forceinline__ float fast_rsqrt(float x) {
   float y;
@@ -93,12 +91,15 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // f(y) = 1/y^2 - x: with e = 1 - x y^2, y + y e (1/2 + 3/8 e), whose error is
 // e^3 / 3 or so.  Five FP64 operations; arguments that are not positive normal
 // numbers (zero, subnormal, infinite, NaN) take the library function.
-__device__ __forceinline__ double fast_rsqrt(double x) {
-  if ((unsigned)__double2hiint(x) - 0x00100000u >= 0x7fe00000u) return rsqrt(x);
+__device__ __forceinline__ double rsqrt_normal(double x) {  // x positive and normal
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma(-(x * y), y, 1.0);
   return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double fast_rsqrt(double x) {
+  if ((unsigned)__double2hiint(x) - 0x00100000u >= 0x7fe00000u) return rsqrt(x);
+  return rsqrt_normal(x);
 }
 
 template <typename T> struct PairTerms {
@@ -143,35 +144,64 @@ __device__ __forceinline__ PairTerms<float> pair_terms(float r2, float s2) {
   return o;
 }
 
-__device__ __forceinline__ PairTerms<double> pair_terms(double r2, double s2) {
+// FP64 closed form.  erf(y) = 1 - e^{-y^2} erfcx(y), y = sqrt(u/2), so that the
+// exponential of zeta serves both, with erfcx(y) = z P(t), z = 1/y =
+// sqrt2 sigma / rho, t = a z + b: P is the project's own degree-20 fit on
+// u in [1, 100] (t in [-1, 1]; least squares on 240 Chebyshev nodes of the
+// 50-digit erfcx, weighted by e^{-y^2} z, so that what the fit adds to erf is
+// below 7e-17).  Beyond u = 100 the term vanishes with e^{-u/2}.  Below u = 1,
+// where q and F of the closed form lose digits (a factor 15 / u^2 in F), the
+// series T gives F, and q follows without cancellation from F's definition,
+// zeta = 3 q + rho^2 F: S(u) = (e^{-u/2} + u T(u)) / 3.  About 60 FP64
+// operations with the roots, exp among them, against about 110 with CUDA's erf,
+// a square root and a division.
+__device__ constexpr double kErfcx64A = 1.5713484026367723;
+__device__ constexpr double kErfcx64B = -1.2222222222222223;
+__device__ constexpr double kErfcx64[21] = {
+    0.4634919981480707, -0.10686061498450462, 0.009106052635940233, 0.009011055439719284,
+    -0.007452171273763995, 0.0036207233597456696, -0.0011820612736484748, 0.00011092787605912042,
+    0.00020382647105256032, -0.00021071103322171375, 0.0001363408811237386, -6.737510924443525e-05,
+    2.419868421912903e-05, -3.1339025280591335e-06, -4.520829552394345e-06, 5.718065614463207e-06,
+    -4.409989858243718e-06, 2.5153884431436396e-06, -1.0165488900277692e-06, 2.5566286437268863e-07,
+    -2.96895951028469e-08};
+__device__ constexpr double kSeriesT64[15] = {  // (-1)^m / (2^m m! (2m + 5))
+    0.2, -0.07142857142857142, 0.013888888888888888, -0.001893939393939394,
+    0.00020032051282051281, -1.736111111111111e-05, 1.2765522875816993e-06, -8.158416875522139e-08,
+    4.613390495086924e-09, -2.340125613449889e-10, 1.0764577821869489e-11, -4.5305462213255424e-13,
+    1.7575394824107708e-14, -6.323653224554882e-16, 2.121571969277071e-17};
+
+// ir = 1/rho (any value at rho = 0), is = 1/sigma.
+__device__ __forceinline__ PairTerms<double> pair_terms(double r2, double s2, double ir, double is) {
   PairTerms<double> o;
-  const double is = rsqrt(s2);
   const double is2 = is * is;
   const double u = r2 * is2;
   const double E = exp(-0.5 * u);
   const double zk = kK1 * is * is2;
   const double z = zk * E;
-  if (u < SeriesCut<double>::value) {
-    double S = PGPU_S8;
-    S = fma(S, u, PGPU_S7); S = fma(S, u, PGPU_S6); S = fma(S, u, PGPU_S5); S = fma(S, u, PGPU_S4);
-    S = fma(S, u, PGPU_S3); S = fma(S, u, PGPU_S2); S = fma(S, u, PGPU_S1); S = fma(S, u, PGPU_S0);
-    double Tt = PGPU_T8;
-    Tt = fma(Tt, u, PGPU_T7); Tt = fma(Tt, u, PGPU_T6); Tt = fma(Tt, u, PGPU_T5); Tt = fma(Tt, u, PGPU_T4);
-    Tt = fma(Tt, u, PGPU_T3); Tt = fma(Tt, u, PGPU_T2); Tt = fma(Tt, u, PGPU_T1); Tt = fma(Tt, u, PGPU_T0);
-    const double m = r2 > 0.0 ? 1.0 : 0.0;
+  if (u < 1.0) {
+    double T = kSeriesT64[14];
+#pragma unroll
+    for (int m = 13; m >= 0; --m) T = fma(T, u, kSeriesT64[m]);
+    const double S = fma(u, T, E) * (1.0 / 3.0);
+    const double m = r2 > 0.0 ? 1.0 : 0.0;  // self pair contributes nothing
     o.q = zk * S * m;
-    o.F = -zk * is2 * Tt * m;
+    o.F = -zk * is2 * T * m;
     o.zd = z * is2 * m;
   } else {
-    const double rho = sqrt(r2);
-    const double ir = 1.0 / rho;
-    const double ir2 = ir * ir;
-    const double er = erf(rho * is * 0.70710678118654752440);
-    o.q = ir2 * (er * ir - kK1 * is * E);
-    o.F = (z - 3.0 * o.q) * ir2;
+    const double A = ir * ir;
+    const double zs = 1.41421356237309504880 * s2 * is;  // sqrt2 sigma
+    const double t = fma(kErfcx64A * zs, ir, kErfcx64B);
+    double P = kErfcx64[20];
+#pragma unroll
+    for (int m = 19; m >= 0; --m) P = fma(P, t, kErfcx64[m]);
+    o.q = fma(-(E * A), fma(zs * A, P, kK1 * is), A * ir);
+    o.F = fma(-3.0, o.q, z) * A;
     o.zd = z * is2;
   }
   return o;
+}
+__device__ __forceinline__ PairTerms<double> pair_terms(double r2, double s2) {
+  return pair_terms(r2, s2, fast_rsqrt(r2), fast_rsqrt(s2));
 }
 
 // ---------------------------------------------------------------- high-order algebraic kernel
@@ -225,7 +255,7 @@ __device__ __forceinline__ PairTerms<float> pair_terms_ho(float r2, float s2) {
 
 __device__ __forceinline__ PairTerms<double> pair_terms_ho(double r2, double s2) {
   const double m = r2 > 0.0 ? 1.0 : 0.0;
-  const double iR = 1.0 / sqrt(r2 + s2);
+  const double iR = fast_rsqrt(r2 + s2);
   const double iR2 = iR * iR;
   const double iR5 = iR2 * iR2 * iR;
   const double iR7 = iR5 * iR2;

@@ -81,6 +81,14 @@ PairFn<float> slices_fn(int v, int ker, bool split) {
   return v == 0 ? pair_slices_kernel<1, false> : pair_slices_kernel<2, false>;
 }
 
+// The same row list in FP64 (pair_slices64.cuh), with its dynamic shared memory.
+PairFn<double> slices64_fn(int v, int ker) {
+  if (ker == PGPU_KERNEL_HIGHORDER)
+    return v == 0 ? pair_slices64_kernel<1, kHighOrder> : pair_slices64_kernel<2, kHighOrder>;
+  return v == 0 ? pair_slices64_kernel<1, kGaussian> : pair_slices64_kernel<2, kGaussian>;
+}
+size_t slices64_bytes(int v) { return v == 0 ? slices64_smem<1>() : slices64_smem<2>(); }
+
 struct WakeRec {
   int sys;
   int64_t cap, n, off;
@@ -338,14 +346,19 @@ int freeze(pgpu_ctx *c) {
   CK(cudaMemsetAsync(c->d_nfull, 0, sizeof(unsigned long long), c->st));
   CK(cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->st));
   for (int s = 0; s < kNumShapes; ++s) c->grid[s] = fp64(c) ? occupancy<double>(c, s) : occupancy<float>(c, s);
-  if (!fp64(c)) {
-    for (int v = 0; v < kNumSlices; ++v) {
-      int nb = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, slices_fn(v, c->cfg.kernel, uses_split(c)), 32 * kSliceWarps, 0) != cudaSuccess ||
-          nb < 1)
-        nb = 1;
-      c->grid_slices[v] = nb * c->sms;
+  for (int v = 0; v < kNumSlices; ++v) {
+    int nb = 0;
+    cudaError_t e;
+    if (fp64(c)) {
+      const PairFn<double> fn = slices64_fn(v, c->cfg.kernel);
+      CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slices64_bytes(v)));
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 32 * kSliceWarps, slices64_bytes(v));
+    } else {
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, slices_fn(v, c->cfg.kernel, uses_split(c)),
+                                                        32 * kSliceWarps, 0);
     }
+    if (e != cudaSuccess || nb < 1) nb = 1;
+    c->grid_slices[v] = nb * c->sms;
   }
   c->frozen = true;
   c->plan_dirty = true;
@@ -503,9 +516,13 @@ std::vector<PlanEntry> build_slices_plan(const pgpu_ctx *c, int variant, int *nc
 // 64-source ones above 45 million pairs.  A shape or chunk count that was asked
 // for, and a tuned shape, keep the tiles.  The high-order kernel's full terms
 // for every pair take the slices at any size (1000 particles: 14 against 52 us
-// in 256 x 1 tiles; 60,000: 6.4 against 8.1 ms; 400,000: 275 against 345 ms)).
+// in 256 x 1 tiles; 60,000: 6.4 against 8.1 ms; 400,000: 275 against 345 ms), and
+// so does FP64 (5000 particles: 161 against 301 us in 128 x 1 tiles; 60,001:
+// 11.0 against 12.0 ms; 200,000: 121 against 125 ms; high-order 60,001: 12.5
+// against 14.2 ms), there too with 32-source slices below 45 million pairs
+// (10,000 particles: 562 against 583 us), 64-source ones above.
 int choose_slices(const pgpu_ctx *c) {
-  if (!c->auto_shape || c->cfg.chunks > 0 || fp64(c) || c->sur) return -1;
+  if (!c->auto_shape || c->cfg.chunks > 0 || c->sur) return -1;
   if (uses_split(c)) return 0;
   double pairs = 0.0, targets = 0.0;
   for (int s = 0; s < (int)c->sys.size(); ++s) {
@@ -513,7 +530,7 @@ int choose_slices(const pgpu_ctx *c) {
     pairs += tn * (double)sys_n(c, s);
     targets += tn;
   }
-  if (targets > 48000.0 && c->cfg.kernel == PGPU_KERNEL_GAUSSIAN) return -1;
+  if (targets > 48000.0 && c->cfg.kernel == PGPU_KERNEL_GAUSSIAN && !fp64(c)) return -1;
   return pairs < 4.5e7 ? 0 : 1;
 }
 
@@ -624,6 +641,9 @@ template <typename T> int launch_pair(pgpu_ctx *c, int slot) {
   if (c->slices >= 0) {
     if constexpr (sizeof(T) == 4) {
       slices_fn(c->slices, c->cfg.kernel, uses_split(c))<<<c->grid_slices[c->slices], 32 * kSliceWarps, 0, c->st>>>(a);
+    } else {
+      slices64_fn(c->slices, c->cfg.kernel)
+          <<<c->grid_slices[c->slices], 32 * kSliceWarps, slices64_bytes(c->slices), c->st>>>(a);
     }
     CK(cudaGetLastError());
     c->launches++;

@@ -115,3 +115,35 @@ def test_autotune_keeps_row_list_or_a_shape(gpu):
         assert (b, t) in ms
         for x, y in zip(c.rates(ids[0]), before):
             assert np.abs(x - y).max() <= 1e-5 * np.abs(y).max()
+
+
+@pytest.mark.parametrize("kernel", ["gaussian", "highorder"])
+@pytest.mark.parametrize("n", [25, 31, 33, 255, 257, 1000, 6700, 6720, 20011])
+def test_rates_row_list_fp64(gpu, n, kernel):
+    """FP64 row list with cores from overlapping to far apart, so that the series, the closed form and the far limit all
+    occur; the closed form's F keeps 15 eps at worst (u = 1), so 1e-12 leaves a margin of a few hundred for the sums."""
+    w = ring(n)
+    w.sigma[: n // 3] = 0.02
+    w.sigma[n // 3: n // 2] = 0.3
+    c, ids = context([w], capi.FP64, kernel=kernel)
+    c.solve()
+    rows = np.unique(np.linspace(0, n - 1, 40).astype(np.int64))
+    v, a = c.rates(ids[0])
+    rv, ra = O.restate_rates(w, NU, targets=rows, kernel=kernel)
+    assert np.abs(v[rows] - rv).max() <= 1e-12 * np.abs(v).max()
+    assert np.abs(a[rows] - ra).max() <= 1e-12 * np.abs(a).max()
+
+
+def test_rates_fp64_far_positions(gpu):
+    """Positions beyond the range of FP32 boxes: the far limit's unchecked root is not taken."""
+    w = ring(400)
+    w.pos[7] = [1e30, 2e25, -3e28]
+    w.pos[300] = [1e170, 0.0, 0.0]
+    c, ids = context([w], capi.FP64)
+    c.solve()
+    v, a = c.rates(ids[0])
+    rows = np.array([0, 8, 100, 399])
+    rest = cases.Wake(*(np.delete(x, [7, 300], axis=0) for x in (w.pos, w.alpha, w.sigma, w.vol)))
+    rv, ra = O.restate_rates(rest, NU, targets=np.array([0, 7, 99, 397]))
+    assert np.abs(v[rows] - rv).max() <= 1e-12 * np.abs(rv).max()
+    assert np.abs(a[rows] - ra).max() <= 1e-12 * np.abs(ra).max()
