@@ -74,19 +74,21 @@ __device__ __forceinline__ RowRun row_run(const PlanEntry *plan, int nsys, int64
   r.last = row + r.nrows == r.first + rps;
   return r;
 }
-// The CTA's sums of a tile, red[warp][component][target], in warp order into
-// its partial; the CTA of the tile's last row also clears the partials that
-// no CTA has.
-__device__ __forceinline__ void row_run_sums(const RowRun &r, const double *red, double *partial, int64_t cap, int nch) {
+// The CTA's sums of a tile, red[warp][component][target] (NC components), in
+// warp order and times `scale` into its partial; the CTA of the tile's last row
+// also clears the partials that no CTA has.
+template <int NC>
+__device__ __forceinline__ void row_run_sums(const RowRun &r, const double *red, double scale, double *partial,
+                                             int64_t cap, int nch) {
   const int clear = r.last ? nch : r.c + 1;
-  for (int e = threadIdx.x; e < 6 * 32; e += 32 * kSliceWarps) {
+  for (int e = threadIdx.x; e < NC * 32; e += 32 * kSliceWarps) {
     double v = 0.0;
 #pragma unroll
-    for (int k = 0; k < kSliceWarps; ++k) v += red[k * 6 * 32 + e];
+    for (int k = 0; k < kSliceWarps; ++k) v += red[k * NC * 32 + e];
     const int64_t i = r.t0 + e % 32;
     if (i >= r.tend) continue;
     double *o = partial + (e / 32) * cap + i;
-    o[r.c * 6 * cap] = v * kInv4Pi;
+    o[r.c * 6 * cap] = v * scale;
     for (int k = r.c + 1; k < clear; ++k) o[k * 6 * cap] = 0.0;
   }
 }
@@ -277,7 +279,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
       red[(w * 6 + 3 + m) * TT + lane] = (double)dh[m] + (double)dl[m];
     }
     __syncthreads();
-    row_run_sums(run, red, a.partial, a.cap, a.nch);
+    row_run_sums<6>(run, red, kInv4Pi, a.partial, a.cap, a.nch);
     __syncthreads();  // before the next tile's slices overwrite the sums
     row += run.nrows;
   }

@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices64_kernel(Pair
 #pragma unroll
     for (int m = 0; m < 6; ++m) hi[32 * m] += lo[32 * m];
     __syncthreads();
-    row_run_sums(run, sums_hi, a.partial, a.cap, a.nch);
+    row_run_sums<6>(run, sums_hi, kInv4Pi, a.partial, a.cap, a.nch);
     __syncthreads();  // before the next tile's sums
     row += run.nrows;
   }

@@ -383,16 +383,14 @@ bool restricted(const pgpu_ctx *c) {
   return false;
 }
 
-// Work list: systems by decreasing work, target tiles x source chunks each.
-// With own_targets, only each system's owned targets are listed (all
-// particles stay sources); otherwise every particle is a target.
-std::vector<PlanEntry> build_plan(const pgpu_ctx *c, const std::vector<int> &systems, int shape, int nch,
-                                  bool own_targets = true) {
+// Work list: systems by decreasing work, tiles of the owned targets x source
+// chunks each.
+std::vector<PlanEntry> build_plan(const pgpu_ctx *c, const std::vector<int> &systems, int shape, int nch) {
   const int64_t TT = (int64_t)kShapes[shape].block * kShapes[shape].tpt;
   const int64_t TILE = kShapes[shape].block;
   std::vector<std::pair<int64_t, int>> order;
   for (int s : systems) {
-    const int64_t tn = own_targets ? owned(c, s).second : sys_n(c, s);
+    const int64_t tn = owned(c, s).second;
     order.push_back({tn * sys_n(c, s), s});
   }
   std::stable_sort(order.begin(), order.end(), [](auto &a, auto &b) { return a.first > b.first; });
@@ -400,7 +398,7 @@ std::vector<PlanEntry> build_plan(const pgpu_ctx *c, const std::vector<int> &sys
   int64_t item = 0;
   for (auto &o : order) {
     const int64_t n = sys_n(c, o.second);
-    const auto t = own_targets ? owned(c, o.second) : std::make_pair<int64_t, int64_t>(0, sys_n(c, o.second));
+    const auto t = owned(c, o.second);
     if (n <= 0 || t.second <= 0) continue;
     PlanEntry e;
     e.off = c->sys[o.second].off;
@@ -460,15 +458,15 @@ int launch_layout(const pgpu_ctx *c) {
 }
 
 // Work list of the slices kernel over every system, in the context's order:
-// rows per system, an equal run of rows per CTA, and in *nch the partials a
-// tile's rows can be split over.
-std::vector<PlanEntry> build_slices_plan(const pgpu_ctx *c, int variant, int *nch) {
+// rows per system, an equal run of rows per CTA of a grid of `grid`, and in
+// *nch the partials a tile's rows can be split over.
+std::vector<PlanEntry> build_slices_plan(const pgpu_ctx *c, int variant, int grid, bool own_targets, int *nch) {
   const int64_t TT = 32, RS = (int64_t)kSliceLen[variant] * kSliceWarps;  // targets and sources per row
   std::vector<PlanEntry> plan;
   int64_t rows = 0, rps_max = 1;
   for (int s = 0; s < (int)c->sys.size(); ++s) {
     const int64_t n = sys_n(c, s);
-    const auto t = owned(c, s);
+    const auto t = own_targets ? owned(c, s) : std::make_pair<int64_t, int64_t>(0, sys_n(c, s));
     if (n <= 0 || t.second <= 0) continue;
     PlanEntry e;
     e.off = c->sys[s].off;
@@ -491,7 +489,7 @@ std::vector<PlanEntry> build_slices_plan(const pgpu_ctx *c, int variant, int *nc
   sentinel.item_start = rows;
   // at most kMaxChunks partials per tile: a tile's rows start anywhere in a CTA's run
   sentinel.chunk = std::max<int64_t>(
-      1, std::max(ceil_div(rows, c->grid_slices[variant]), ceil_div(rps_max, kMaxChunks - 1)));
+      1, std::max(ceil_div(rows, grid), ceil_div(rps_max, kMaxChunks - 1)));
   *nch = 1;
   for (const PlanEntry &e : plan)
     *nch = std::max(*nch, (int)std::min(e.chunk, ceil_div(e.chunk, sentinel.chunk) + 1));
@@ -552,7 +550,7 @@ int upload_plan(pgpu_ctx *c) {
   std::vector<PlanEntry> plan;
   c->slices = c->groups.empty() ? choose_slices(c) : -1;
   if (c->slices >= 0) {
-    plan = build_slices_plan(c, c->slices, &c->nch);
+    plan = build_slices_plan(c, c->slices, c->grid_slices[c->slices], true, &c->nch);
     plan.resize(ns + 1, plan.back());
   } else if (c->groups.empty()) {
     // the surrogate writes one chunk of rates per evaluation
@@ -1072,7 +1070,7 @@ int pgpu_diagnose_partial(pgpu_ctx *c, int32_t system, double *fields) {
   // rows: the owned targets (all of them without a target range); each
   // unordered pair is summed from its lower index, so the ranks' row ranges
   // together cover every pair once
-  std::vector<PlanEntry> plan = build_plan(c, {system}, shape, nch, true);
+  std::vector<PlanEntry> plan = build_plan(c, {system}, shape, nch);
   CK(cudaMemcpyAsync(c->d_plan_diag, plan.data(), plan.size() * sizeof(PlanEntry), cudaMemcpyHostToDevice, c->st));
   CK(cudaStreamSynchronize(c->st));
   const bool quad = plan.size() > 1;
@@ -1235,25 +1233,24 @@ int pgpu_influence(pgpu_ctx *c) {
       return fail(c, PGPU_ENOMEM, "cudaMalloc of the vorticity field failed: %s", cudaGetErrorString(e));
     }
   }
-  // every particle of every system is a target, 256-target tiles
-  const int shape = 2, block = 256;
-  int64_t tiles = 0;
-  std::vector<int> all(c->sys.size());
-  for (size_t s = 0; s < all.size(); ++s) {
-    all[s] = (int)s;
-    tiles += ceil_div(sys_n(c, (int)s), block);
-  }
-  const int nch = (int)std::max<int64_t>(1, std::min<int64_t>(kMaxChunks, ceil_div(8LL * c->sms, std::max<int64_t>(1, tiles))));
-  std::vector<PlanEntry> plan = build_plan(c, all, shape, nch, false);
+  // every particle of every system is a target; slice length as choose_slices
+  double pairs = 0.0;
+  for (size_t k = 0; k < c->sys.size(); ++k) pairs += (double)sys_n(c, (int)k) * (double)sys_n(c, (int)k);
+  const int v = pairs < 4.5e7 ? 0 : 1;
+  const bool ho = c->cfg.kernel == PGPU_KERNEL_HIGHORDER;
+  auto fn = v == 0 ? (ho ? field_kernel<1, kHighOrder> : field_kernel<1, kGaussian>)
+                   : (ho ? field_kernel<2, kHighOrder> : field_kernel<2, kGaussian>);
+  int nb = 0, nch = 1;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 32 * kSliceWarps, 0));
+  const int grid = std::max(1, nb) * c->sms;
+  std::vector<PlanEntry> plan = build_slices_plan(c, v, grid, false, &nch);
+  const bool any = plan.size() > 1;
   plan.resize(c->sys.size() + 1, plan.back());
   CK(cudaMemcpyAsync(c->d_plan_field, plan.data(), plan.size() * sizeof(PlanEntry), cudaMemcpyHostToDevice, c->st));
   CK(cudaStreamSynchronize(c->st));  // the plan vector is pageable host memory
-  if (plan.size() > 1 && plan.front().n > 0) {
-    int grid = 0;
-    FieldArgs a{c->x0, c->sig, c->partial, c->d_plan_field, (int)c->sys.size(), nch, c->cap, c->d_counters};
-    auto fn = c->cfg.kernel == PGPU_KERNEL_HIGHORDER ? field_kernel<256, kHighOrder> : field_kernel<256, kGaussian>;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&grid, fn, block, 0));
-    fn<<<std::max(1, grid) * c->sms, block, 0, c->st>>>(a);
+  if (any) {
+    FieldArgs a{c->x0, c->sig, c->partial, c->d_plan_field, (int)c->sys.size(), nch, c->cap};
+    fn<<<grid, 32 * kSliceWarps, 0, c->st>>>(a);
     CK(cudaGetLastError());
     c->launches++;
   }

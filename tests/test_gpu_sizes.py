@@ -147,3 +147,24 @@ def test_rates_fp64_far_positions(gpu):
     rv, ra = O.restate_rates(rest, NU, targets=np.array([0, 7, 99, 397]))
     assert np.abs(v[rows] - rv).max() <= 1e-12 * np.abs(rv).max()
     assert np.abs(a[rows] - ra).max() <= 1e-12 * np.abs(ra).max()
+
+
+@pytest.mark.parametrize("kernel", ["gaussian", "highorder"])
+@pytest.mark.parametrize("n", [25, 33, 255, 257, 3000, 6720, 12011])
+def test_field_row_list(gpu, n, kernel):
+    """Slices of one and of several radii, some beyond the reach of the exponential."""
+    w = ring(n, sigma=0.02)
+    w.sigma[: n // 3] = 0.011
+    other = ring(40)
+    c, ids = context([w, other], capi.FP32C, kernel=kernel)
+    for k, x in zip(ids, (w, other)):
+        f, ref = c.vorticity_field(k), O.restate_vorticity_field(x, kernel=kernel)
+        assert np.abs(f - ref).max() <= 1e-11 * np.abs(ref).max()
+
+
+def test_field_keeps_non_finite_strengths(gpu):
+    """A strength that is not finite reaches every target, also those beyond the exponential's reach (0 x inf)."""
+    w = ring(3000, sigma=0.01)
+    w.alpha[17, 1] = np.inf
+    c, ids = context([w], capi.FP32C)
+    assert np.isnan(c.vorticity_field(ids[0])[1600, 1])
