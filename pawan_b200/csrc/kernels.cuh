@@ -77,6 +77,10 @@ template <typename T> struct PairArgs {
   // residuals (x - (float)x, y - (float)y, z - (float)z, 0) of every
   // particle, added to the pair differences in tiles with near pairs.
   const float4 *L = nullptr;
+  // Slices kernel: targets t of the plan are the particles off + targets[t]
+  // of the system, and their sums go to partial rows t (a plan with toff =
+  // -off, and cap the number of targets).  nullptr: the particles themselves.
+  const int *targets = nullptr;
 };
 
 // Slots per precomputed source box (divides every pair-kernel tile).

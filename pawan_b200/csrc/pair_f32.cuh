@@ -198,8 +198,9 @@ __device__ __forceinline__ void far_b3(float xr0, float xr1, float xr2, const fl
 // q (alpha_t x alpha_s) for the stretching (nearly parallel neighbours along a
 // filament) and the diffusion v_t a_s - v_s a_t.  uni: the sigma factors where
 // one sigma serves every pair (72 FP32 operations per pair, 63 with them), or
-// null.  All lanes of the warp together (it votes).
-template <bool SPLIT>
+// null.  CROSS: sp sums q (alpha_t x alpha_s), else q alpha_s (six operations
+// less).  All lanes of the warp together (it votes).
+template <bool SPLIT, bool CROSS = true>
 __device__ __forceinline__ void mid_pair2(float2 px, float2 py, float2 pz, float2 ph, float2 ax, float2 ay, float2 az,
                                           float2 av, float2 lx, float2 ly, float2 lz, const float2 *X, const float *xl,
                                           const float *at, float hst, float h50, float vt, const MidSigma2 *uni,
@@ -241,12 +242,18 @@ __device__ __forceinline__ void mid_pair2(float2 px, float2 py, float2 pz, float
   sd[0] = __ffma2_rn(fd, dx, sd[0]);
   sd[1] = __ffma2_rn(fd, dy, sd[1]);
   sd[2] = __ffma2_rn(fd, dz, sd[2]);
-  const float2 cx = __ffma2_rn(dup2(at[1]), az, __fmul2_rn(dup2(-at[2]), ay));
-  const float2 cy = __ffma2_rn(dup2(at[2]), ax, __fmul2_rn(dup2(-at[0]), az));
-  const float2 cz = __ffma2_rn(dup2(at[0]), ay, __fmul2_rn(dup2(-at[1]), ax));
-  sp[0] = __ffma2_rn(t.q, cx, sp[0]);
-  sp[1] = __ffma2_rn(t.q, cy, sp[1]);
-  sp[2] = __ffma2_rn(t.q, cz, sp[2]);
+  if constexpr (CROSS) {
+    const float2 cx = __ffma2_rn(dup2(at[1]), az, __fmul2_rn(dup2(-at[2]), ay));
+    const float2 cy = __ffma2_rn(dup2(at[2]), ax, __fmul2_rn(dup2(-at[0]), az));
+    const float2 cz = __ffma2_rn(dup2(at[0]), ay, __fmul2_rn(dup2(-at[1]), ax));
+    sp[0] = __ffma2_rn(t.q, cx, sp[0]);
+    sp[1] = __ffma2_rn(t.q, cy, sp[1]);
+    sp[2] = __ffma2_rn(t.q, cz, sp[2]);
+  } else {
+    sp[0] = __ffma2_rn(t.q, ax, sp[0]);
+    sp[1] = __ffma2_rn(t.q, ay, sp[1]);
+    sp[2] = __ffma2_rn(t.q, az, sp[2]);
+  }
   const float2 VT = dup2(vt);
   sdv[0] = __ffma2_rn(t.zd, __ffma2_rn(av, dup2(-at[0]), __fmul2_rn(VT, ax)), sdv[0]);
   sdv[1] = __ffma2_rn(t.zd, __ffma2_rn(av, dup2(-at[1]), __fmul2_rn(VT, ay)), sdv[1]);
@@ -254,8 +261,9 @@ __device__ __forceinline__ void mid_pair2(float2 px, float2 py, float2 pz, float
 }
 
 // Folds one compensation group of a target into its (hi, lo) sums.  Far
-// groups summed q alpha_s and q n_s (xr = x_t - ref), the others
-// q (alpha_t x alpha_s) and q w.
+// groups summed q alpha_s and q n_s (xr = x_t - ref), the others q w and, with
+// CROSS, q (alpha_t x alpha_s), else q alpha_s.
+template <bool CROSS = true>
 __device__ __forceinline__ void fold_group_f32(bool far, float xr0, float xr1, float xr2, const float *at, float nu2,
                                                const float2 *sv, const float2 *sd, const float2 *sp, const float *sdv,
                                                float *vh, float *vl, float *dh, float *dl) {
@@ -274,6 +282,8 @@ __device__ __forceinline__ void fold_group_f32(bool far, float xr0, float xr1, f
     svs[0] = sps[1] * xr2 - sps[2] * xr1 + n0;
     svs[1] = sps[2] * xr0 - sps[0] * xr2 + n1;
     svs[2] = sps[0] * xr1 - sps[1] * xr0 + n2;
+  }
+  if (far || !CROSS) {
     c0 = at[1] * sps[2] - at[2] * sps[1];
     c1 = at[2] * sps[0] - at[0] * sps[2];
     c2 = at[0] * sps[1] - at[1] * sps[0];

@@ -98,6 +98,60 @@ template <int SL, bool SPLIT> struct SliceStage {
   float4 L[SPLIT ? 32 * SL : 1];
 };
 
+// Source k of a slice (position p, strength and volume q), its n_s taken
+// about the slice's reference point.
+template <int SL, bool SPLIT>
+__device__ __forceinline__ void stage_source(SliceStage<SL, SPLIT> &st, int k, float4 p, float4 q, float rx, float ry,
+                                             float rz) {
+  const int e = (k >> 1) * 8 + (k & 1);
+  float *dp = reinterpret_cast<float *>(st.P) + e, *dq = reinterpret_cast<float *>(st.Q) + e,
+        *dn = reinterpret_cast<float *>(st.N) + e;
+  dp[0] = p.x; dp[2] = p.y; dp[4] = p.z; dp[6] = p.w;
+  dq[0] = q.x; dq[2] = q.y; dq[4] = q.z; dq[6] = q.w;
+  const float px = p.x - rx, py = p.y - ry, pz = p.z - rz;
+  dn[0] = py * q.z - pz * q.y;
+  dn[2] = pz * q.x - px * q.z;
+  dn[4] = px * q.y - py * q.x;
+}
+
+// The Gaussian sums of one target over npr source pairs of a staged slice:
+// the far limit, or the closed form (its diffusion into sdv).
+template <int SL, bool SPLIT>
+__device__ __forceinline__ void far_slice(const SliceStage<SL, SPLIT> &st, int npr, const float2 *X, const float2 *AT,
+                                          float xr0, float xr1, float xr2, float2 *sv, float2 *sd, float2 *sp) {
+  float2 B3[3];
+  far_b3(xr0, xr1, xr2, AT, B3);
+#pragma unroll 2
+  for (int r = 0; r < npr; ++r) {
+    const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1], na = st.N[2 * r],
+                 nb = st.N[2 * r + 1];
+    far_pair2(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y), make_float2(qa.x, qa.y),
+              make_float2(qa.z, qa.w), make_float2(qb.x, qb.y), make_float2(na.x, na.y), make_float2(na.z, na.w),
+              make_float2(nb.x, nb.y), X, AT, B3, sv, sd, sp);
+  }
+}
+template <bool SPLIT, bool CROSS, int SL>
+__device__ __forceinline__ void mid_slice(const SliceStage<SL, SPLIT> &st, int npr, const float2 *X, const float *xl,
+                                          const float *at, float hst, float vt, const MidSigma2 *uni, float2 *sv,
+                                          float2 *sd, float2 *sp, float *sdv, unsigned &nfull) {
+  float2 sdv2[3] = {dup2(0.f), dup2(0.f), dup2(0.f)};
+#pragma unroll 2
+  for (int r = 0; r < npr; ++r) {
+    const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1];
+    float2 lx = dup2(0.f), ly = lx, lz = lx;
+    if constexpr (SPLIT) {
+      const float4 la = st.L[2 * r], lb = st.L[2 * r + 1];
+      lx = make_float2(la.x, la.y); ly = make_float2(la.z, la.w); lz = make_float2(lb.x, lb.y);
+    }
+    mid_pair2<SPLIT, CROSS>(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y),
+                            make_float2(pb.z, pb.w), make_float2(qa.x, qa.y), make_float2(qa.z, qa.w),
+                            make_float2(qb.x, qb.y), make_float2(qb.z, qb.w), lx, ly, lz, X, xl, at, hst, kFarU * hst,
+                            vt, uni, sv, sd, sp, sdv2, nfull);
+  }
+#pragma unroll
+  for (int m = 0; m < 3; ++m) sdv[m] = sdv2[m].x + sdv2[m].y;
+}
+
 template <int SL, bool SPLIT, int KER = kGaussian>
 __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairArgs<float> a) {
   constexpr int W = kSliceWarps, S = 32 * SL, TT = 32;
@@ -129,7 +183,8 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
     int64_t sb = run.pe.off + (g * W + w) * S;
     if (sb < s1) fetch(sb);
 
-    const int64_t ti = min(run.t0 + lane, run.tend - 1);
+    int64_t ti = min(run.t0 + lane, run.tend - 1);
+    if (a.targets) ti = run.pe.off + a.targets[ti];
     const float4 pt = a.P[ti], qt = a.Q[ti];
     float4 lt = pad_Q<float>();
     if constexpr (SPLIT) lt = a.L[ti];
@@ -166,18 +221,10 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
       float hmin = 3.0e38f;
 #pragma unroll
       for (int j = 0; j < SL; ++j) {
-        const int e = ((lane + 32 * j) >> 1) * 8 + (lane & 1);
-        float *dp = reinterpret_cast<float *>(st.P) + e, *dq = reinterpret_cast<float *>(st.Q) + e,
-              *dn = reinterpret_cast<float *>(st.N) + e;
         const float4 p = gp[j], q = gq[j];
-        dp[0] = p.x; dp[2] = p.y; dp[4] = p.z; dp[6] = p.w;
-        dq[0] = q.x; dq[2] = q.y; dq[4] = q.z; dq[6] = q.w;
-        const float px = p.x - rx, py = p.y - ry, pz = p.z - rz;
-        dn[0] = py * q.z - pz * q.y;
-        dn[2] = pz * q.x - px * q.z;
-        dn[4] = px * q.y - py * q.x;
+        stage_source(st, lane + 32 * j, p, q, rx, ry, rz);
         if constexpr (SPLIT) {
-          float *dl_ = reinterpret_cast<float *>(st.L) + e;
+          float *dl_ = reinterpret_cast<float *>(st.L) + ((lane + 32 * j) >> 1) * 8 + (lane & 1);
           dl_[0] = gl[j].x; dl_[2] = gl[j].y; dl_[4] = gl[j].z;
         }
         if (cur + lane + 32 * j < s1) {
@@ -228,44 +275,15 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
           sd[m] = __fmul2_rn(sd[m], dup2(-3.f));
         }
       } else if (far) {
-        float2 B3[3];
-        far_b3(pt.x - rx, pt.y - ry, pt.z - rz, AT, B3);
-#pragma unroll 2
-        for (int r = 0; r < npr; ++r) {
-          const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1],
-                       na = st.N[2 * r], nb = st.N[2 * r + 1];
-          far_pair2(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y),
-                    make_float2(qa.x, qa.y), make_float2(qa.z, qa.w), make_float2(qb.x, qb.y),
-                    make_float2(na.x, na.y), make_float2(na.z, na.w), make_float2(nb.x, nb.y), X, AT, B3, sv, sd, sp);
-        }
-      } else {
-        float2 sdv2[3] = {dup2(0.f), dup2(0.f), dup2(0.f)};
-        auto mid = [&](const MidSigma2 *uni) {
-#pragma unroll 2
-          for (int r = 0; r < npr; ++r) {
-            const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1];
-            float2 lx = dup2(0.f), ly = lx, lz = lx;
-            if constexpr (SPLIT) {
-              const float4 la = st.L[2 * r], lb = st.L[2 * r + 1];
-              lx = make_float2(la.x, la.y); ly = make_float2(la.z, la.w); lz = make_float2(lb.x, lb.y);
-            }
-            mid_pair2<SPLIT>(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y),
-                             make_float2(pb.z, pb.w), make_float2(qa.x, qa.y), make_float2(qa.z, qa.w),
-                             make_float2(qb.x, qb.y), make_float2(qb.z, qb.w), lx, ly, lz, X, xl, at, pt.w,
-                             kFarU * pt.w, qt.w, uni, sv, sd, sp, sdv2, nfull);
-          }
-        };
+        far_slice(st, npr, X, AT, pt.x - rx, pt.y - ry, pt.z - rz, sv, sd, sp);
+      } else if (warp_min(hmin) == sbox.hs && thmin == tb.hs) {
         // one sigma for all of the slice's pairs, as in every wake shed with
         // one radius: its factors leave the loop (an odd tail's padding
         // source carries no strength, so its sigma does not matter)
-        if (warp_min(hmin) == sbox.hs && thmin == tb.hs) {
-          const MidSigma2 g = mid_sigma2(dup2(tb.hs + sbox.hs));
-          mid(&g);
-        } else {
-          mid(nullptr);
-        }
-#pragma unroll
-        for (int m = 0; m < 3; ++m) sdv[m] = sdv2[m].x + sdv2[m].y;
+        const MidSigma2 g = mid_sigma2(dup2(tb.hs + sbox.hs));
+        mid_slice<SPLIT, true>(st, npr, X, xl, at, pt.w, qt.w, &g, sv, sd, sp, sdv, nfull);
+      } else {
+        mid_slice<SPLIT, true>(st, npr, X, xl, at, pt.w, qt.w, nullptr, sv, sd, sp, sdv, nfull);
       }
       fold_group_f32(far, pt.x - rx, pt.y - ry, pt.z - rz, at, a.nu2, sv, sd, sp, sdv, vh, vl, dh, dl);
     }

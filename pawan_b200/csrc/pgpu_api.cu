@@ -457,25 +457,23 @@ int launch_layout(const pgpu_ctx *c) {
   return 1000 + mask;
 }
 
-// Work list of the slices kernel over every system, in the context's order:
-// rows per system, an equal run of rows per CTA of a grid of `grid`, and in
-// *nch the partials a tile's rows can be split over.
-std::vector<PlanEntry> build_slices_plan(const pgpu_ctx *c, int variant, int grid, bool own_targets, int *nch) {
-  const int64_t TT = 32, RS = (int64_t)kSliceLen[variant] * kSliceWarps;  // targets and sources per row
+// Work list of the slices kernel: systems added one by one, then closed for a
+// grid of `grid` CTAs with an equal run of rows each; nch is the number of
+// partials a tile's rows can be split over.
+struct SlicesPlan {
   std::vector<PlanEntry> plan;
   int64_t rows = 0, rps_max = 1;
-  for (int s = 0; s < (int)c->sys.size(); ++s) {
-    const int64_t n = sys_n(c, s);
-    const auto t = own_targets ? owned(c, s) : std::make_pair<int64_t, int64_t>(0, sys_n(c, s));
-    if (n <= 0 || t.second <= 0) continue;
+  int nch = 1;
+  void add(int variant, int64_t off, int64_t n, int64_t toff, int64_t tn) {
+    if (n <= 0 || tn <= 0) return;
     PlanEntry e;
-    e.off = c->sys[s].off;
+    e.off = off;
     e.n = n;
     e.item_start = rows;
-    e.tiles = ceil_div(t.second, TT);
-    e.chunk = ceil_div(n, RS);
-    e.toff = t.first;
-    e.tn = t.second;
+    e.tiles = ceil_div(tn, 32);
+    e.chunk = ceil_div(n, (int64_t)kSliceLen[variant] * kSliceWarps);
+    e.toff = toff;
+    e.tn = tn;
     // a step near the golden section of the rows, coprime to their number,
     // scatters any run of rows over the system
     e.mult = std::max<int64_t>(1, (int64_t)(0.618 * (double)e.chunk));
@@ -485,16 +483,28 @@ std::vector<PlanEntry> build_slices_plan(const pgpu_ctx *c, int variant, int gri
     rps_max = std::max(rps_max, e.chunk);
     plan.push_back(e);
   }
-  PlanEntry sentinel{};
-  sentinel.item_start = rows;
-  // at most kMaxChunks partials per tile: a tile's rows start anywhere in a CTA's run
-  sentinel.chunk = std::max<int64_t>(
-      1, std::max(ceil_div(rows, grid), ceil_div(rps_max, kMaxChunks - 1)));
-  *nch = 1;
-  for (const PlanEntry &e : plan)
-    *nch = std::max(*nch, (int)std::min(e.chunk, ceil_div(e.chunk, sentinel.chunk) + 1));
-  plan.push_back(sentinel);
-  return plan;
+  void close(int grid, size_t entries) {
+    PlanEntry sentinel{};
+    sentinel.item_start = rows;
+    // at most kMaxChunks partials per tile: a tile's rows start anywhere in a CTA's run
+    sentinel.chunk = std::max<int64_t>(1, std::max(ceil_div(rows, grid), ceil_div(rps_max, kMaxChunks - 1)));
+    nch = 1;
+    for (const PlanEntry &e : plan)
+      nch = std::max(nch, (int)std::min(e.chunk, ceil_div(e.chunk, sentinel.chunk) + 1));
+    plan.resize(entries, sentinel);
+  }
+};
+
+// Every system of the context, its owned targets or all of them.
+SlicesPlan build_slices_plan(const pgpu_ctx *c, int variant, int grid, bool own_targets) {
+  SlicesPlan p;
+  for (int s = 0; s < (int)c->sys.size(); ++s) {
+    const int64_t n = sys_n(c, s);
+    const auto t = own_targets ? owned(c, s) : std::make_pair<int64_t, int64_t>(0, sys_n(c, s));
+    p.add(variant, c->sys[s].off, n, t.first, t.second);
+  }
+  p.close(grid, c->sys.size() + 1);
+  return p;
 }
 
 // Variant of the slices kernel for the context's next evaluations, -1 for the
@@ -550,8 +560,9 @@ int upload_plan(pgpu_ctx *c) {
   std::vector<PlanEntry> plan;
   c->slices = c->groups.empty() ? choose_slices(c) : -1;
   if (c->slices >= 0) {
-    plan = build_slices_plan(c, c->slices, c->grid_slices[c->slices], true, &c->nch);
-    plan.resize(ns + 1, plan.back());
+    SlicesPlan p = build_slices_plan(c, c->slices, c->grid_slices[c->slices], true);
+    plan = std::move(p.plan);
+    c->nch = p.nch;
   } else if (c->groups.empty()) {
     // the surrogate writes one chunk of rates per evaluation
     c->nch = c->sur ? 1 : choose_nch(c, c->shape);
@@ -1240,15 +1251,14 @@ int pgpu_influence(pgpu_ctx *c) {
   const bool ho = c->cfg.kernel == PGPU_KERNEL_HIGHORDER;
   auto fn = v == 0 ? (ho ? field_kernel<1, kHighOrder> : field_kernel<1, kGaussian>)
                    : (ho ? field_kernel<2, kHighOrder> : field_kernel<2, kGaussian>);
-  int nb = 0, nch = 1;
+  int nb = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 32 * kSliceWarps, 0));
   const int grid = std::max(1, nb) * c->sms;
-  std::vector<PlanEntry> plan = build_slices_plan(c, v, grid, false, &nch);
-  const bool any = plan.size() > 1;
-  plan.resize(c->sys.size() + 1, plan.back());
-  CK(cudaMemcpyAsync(c->d_plan_field, plan.data(), plan.size() * sizeof(PlanEntry), cudaMemcpyHostToDevice, c->st));
+  const SlicesPlan p = build_slices_plan(c, v, grid, false);
+  const int nch = p.nch;
+  CK(cudaMemcpyAsync(c->d_plan_field, p.plan.data(), p.plan.size() * sizeof(PlanEntry), cudaMemcpyHostToDevice, c->st));
   CK(cudaStreamSynchronize(c->st));  // the plan vector is pageable host memory
-  if (any) {
+  if (p.rows > 0) {
     FieldArgs a{c->x0, c->sig, c->partial, c->d_plan_field, (int)c->sys.size(), nch, c->cap};
     fn<<<grid, 32 * kSliceWarps, 0, c->st>>>(a);
     CK(cudaGetLastError());

@@ -257,50 +257,6 @@ __device__ __forceinline__ void far_features(const float *v, const float *x, con
   ss = am * tm * ir * ir * ir * q2;
 }
 
-// One ordered pair with the FP32 three-regime terms of the direct kernel,
-// accumulated into CG-group partial sums.  Must be called by all lanes of a
-// warp together (it votes).
-__device__ __forceinline__ void pair_accum_f32(const float4 p, const float4 q, const float *xt, const float *at,
-                                               float hst, float h50, float vt, float *sv, float *sd, float *sp,
-                                               float *sdv) {
-  const float dx = xt[0] - p.x, dy = xt[1] - p.y, dz = xt[2] - p.z;
-  const float r2 = dx * dx + dy * dy + dz * dz;
-  const bool near = fmaf(-kFarU, p.w, r2) < h50;
-  const float ir = fast_rsqrt(r2);
-  const float A = ir * ir;
-  float qq = A * ir, FF = -3.0f * qq * A, zd = 0.f;
-  bool diffuse = false;
-  if (__any_sync(0xffffffffu, near)) {
-    if (near) {
-      const PairTerms<float> pt = pair_terms_near(r2, hst + p.w);
-      qq = pt.q; FF = pt.F; zd = pt.zd;
-      diffuse = true;
-    }
-  }
-  const float wx = q.y * dz - q.z * dy, wy = q.z * dx - q.x * dz, wz = q.x * dy - q.y * dx;
-  sv[0] += qq * wx; sv[1] += qq * wy; sv[2] += qq * wz;
-  const float fd = FF * (at[0] * wx + at[1] * wy + at[2] * wz);
-  sd[0] += fd * dx; sd[1] += fd * dy; sd[2] += fd * dz;
-  sp[0] += qq * q.x; sp[1] += qq * q.y; sp[2] += qq * q.z;
-  if (diffuse) {
-    sdv[0] += zd * (vt * q.x - q.w * at[0]);
-    sdv[1] += zd * (vt * q.y - q.w * at[1]);
-    sdv[2] += zd * (vt * q.z - q.w * at[2]);
-  }
-}
-
-__device__ __forceinline__ void fold_group(const float *at, float nu2, float *sv, float *sd, float *sp, float *sdv,
-                                           float *vh, float *vl, float *dh, float *dl) {
-  const float e[3] = {at[1] * sp[2] - at[2] * sp[1] + sd[0] + nu2 * sdv[0],
-                      at[2] * sp[0] - at[0] * sp[2] + sd[1] + nu2 * sdv[1],
-                      at[0] * sp[1] - at[1] * sp[0] + sd[2] + nu2 * sdv[2]};
-  for (int m = 0; m < 3; ++m) {
-    two_sum_acc(vh[m], vl[m], sv[m]);
-    two_sum_acc(dh[m], dl[m], e[m]);
-    sv[m] = sd[m] = sp[m] = sdv[m] = 0.f;
-  }
-}
-
 struct TreeEvalArgs {
   const CellData *cd;
   const TreeCell *cells;
@@ -321,9 +277,6 @@ struct TreeEvalArgs {
   int own_lo, own_hi;
 };
 
-constexpr int kTreeBlock = 256;  // sampled-check kernel
-
-
 // Warp-independent form: every warp takes work items (target leaf, slice of
 // 32 of its targets) from an atomic counter and stages its own source tiles,
 // synchronising only within the warp.  Leaves average ~130 particles, so
@@ -336,8 +289,10 @@ constexpr int kWarpsPerCta = 4;
 // Per-warp shared buffers (all carved from dynamic shared memory, after the
 // packed network when the correction is on).
 struct WarpSmem {
-  float sc[kWarpCells][kCellFloats];
-  float4 sP[kWarpTile], sQ[kWarpTile];
+  union {
+    float sc[kWarpCells][kCellFloats];
+    SliceStage<kWarpTile / 32, false> near;
+  };
 };
 struct WarpSmemMlp {
   __nv_bfloat16 sF[32][kInPad + 8];
@@ -418,24 +373,23 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
         two_sum_acc(dh[m], dl[m], ss[m]);
       }
     }
-    // Near field, two sources per packed FP32 instruction (lane .x the even
-    // source of a pair, .y the odd one; pair-interleaved staging as in the
-    // direct kernel).  A 64-source sub-tile whose box is far from the warp's
-    // 32 targets (every pair at u >= 50) takes the far limit; the others take
-    // the closed form for every pair, and lanes at u < 1, the self pair among
-    // them, the series.  On the 4M coaxial rings the all-far sub-tiles cut
-    // the evaluation from 933 to 869 ms; boxes per 32-source half cut fewer
-    // pairs than their second reduction cost (877 ms).
+    // Near field: the slices of pair_slices.cuh over the leaf's runs.  Slices
+    // far from the warp's targets (every pair at u >= 50) take the far limit,
+    // the others the closed form, with sigma's factors out of the loop where
+    // one radius serves the slice.  It is most of the evaluation (about 28,000
+    // near particles per target on the 1M coaxial rings) and bound by the FP32
+    // pipe: the evaluation takes 105 ms, and 116 ms with 64-source slices boxed
+    // by shuffles and sigma's factors per pair.
     const float2 X2[3] = {dup2(xt[0]), dup2(xt[1]), dup2(xt[2])};
-    const float2 AT2[3] = {dup2(at[0]), dup2(at[1]), dup2(at[2])};
-    const float2 NAT2[3] = {dup2(-at[0]), dup2(-at[1]), dup2(-at[2])};
-    const float2 HS2 = dup2(hst), VT2 = dup2(vt), M1 = dup2(-1.f);
     const float2 AT3[3] = {dup2(-3.f * at[0]), dup2(-3.f * at[1]), dup2(-3.f * at[2])};
-    // bounding box of the warp's targets, for the per-sub-tile all-far test
     WarpBox tb;
     tb.init();
     tb.add(xt[0], xt[1], xt[2], hst);
-    tb.reduce();
+    reduce_box(tb);
+    const float thmin = warp_min(hst);
+    constexpr int SL = kWarpTile / 32;
+    auto &st = ws.near;
+    unsigned nfull = 0;
     const int no = a.near_off[li], nn = a.near_cnt[li];
     for (int ni = 0; ni < nn; ++ni) {
       const int2 run = a.near_runs[no + ni];
@@ -443,123 +397,41 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
         __syncwarp();
         WarpBox sbx;
         sbx.init();
-        for (int k = lane; k < kWarpTile; k += 32) {
-          const int j = sb + k;
-          const float4 p = j < run.y ? a.Ps[j] : pad_P<float>();
-          const float4 q = j < run.y ? a.Qs[j] : pad_Q<float>();
-          if (j < run.y) sbx.add(p.x, p.y, p.z, p.w);
-          float *dp = reinterpret_cast<float *>(ws.sP) + (k >> 1) * 8 + (k & 1);
-          float *dq = reinterpret_cast<float *>(ws.sQ) + (k >> 1) * 8 + (k & 1);
-          dp[0] = p.x; dp[2] = p.y; dp[4] = p.z; dp[6] = p.w;
-          dq[0] = q.x; dq[2] = q.y; dq[4] = q.z; dq[6] = q.w;
+        float hmin = 3.0e38f, rx = 0.f, ry = 0.f, rz = 0.f;
+#pragma unroll
+        for (int j = 0; j < SL; ++j) {
+          const int i = sb + lane + 32 * j;
+          const float4 p = i < run.y ? a.Ps[i] : pad_P<float>();
+          const float4 q = i < run.y ? a.Qs[i] : pad_Q<float>();
+          if (j == 0) {
+            rx = __shfl_sync(0xffffffffu, p.x, 0);
+            ry = __shfl_sync(0xffffffffu, p.y, 0);
+            rz = __shfl_sync(0xffffffffu, p.z, 0);
+          }
+          stage_source(st, lane + 32 * j, p, q, rx, ry, rz);
+          if (i < run.y) {
+            sbx.add(p.x, p.y, p.z, p.w);
+            hmin = fminf(hmin, p.w);
+          }
         }
-        sbx.reduce();
-        // every pair of the warp's targets with this sub-tile at u >= 50: the
-        // far limit (q = 1/rho^3, F = -3/rho^5, no diffusion), as the direct
-        // kernel's all-far tiles
+        reduce_box(sbx);
         const bool far_tile = all_far(tb, sbx);
         __syncwarp();
         // source pairs; an odd tail pairs with a padding source (zero strength, far away)
         const int npr = (min(kWarpTile, run.y - sb) + 1) >> 1;
+        float2 sv[3], sd[3], sp[3];
+        float sdv[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int m = 0; m < 3; ++m) sv[m] = sd[m] = sp[m] = dup2(0.f);
         if (far_tile) {
-          for (int g = 0; g < npr; g += 16) {
-            float2 sv2[3], sd2[3], sp2[3];
-            for (int m = 0; m < 3; ++m) { sv2[m] = sd2[m] = sp2[m] = dup2(0.f); }
-            const int ge = min(npr, g + 16);
-            for (int r = g; r < ge; ++r) {
-              const float4 pa = ws.sP[2 * r], pb = ws.sP[2 * r + 1];
-              const float4 qa = ws.sQ[2 * r], qb = ws.sQ[2 * r + 1];
-              const float2 dx = __ffma2_rn(make_float2(pa.x, pa.y), M1, X2[0]);
-              const float2 dy = __ffma2_rn(make_float2(pa.z, pa.w), M1, X2[1]);
-              const float2 dz = __ffma2_rn(make_float2(pb.x, pb.y), M1, X2[2]);
-              const float2 ax = make_float2(qa.x, qa.y), ay = make_float2(qa.z, qa.w), az = make_float2(qb.x, qb.y);
-              float2 r2 = __fmul2_rn(dx, dx);
-              r2 = __ffma2_rn(dy, dy, r2);
-              r2 = __ffma2_rn(dz, dz, r2);
-              const float2 ir = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
-              const float2 A = __fmul2_rn(ir, ir);
-              const float2 qq = __fmul2_rn(A, ir);
-              const float2 qA = __fmul2_rn(qq, A);
-              const float2 wx = make_float2(ay.x * dz.x - az.x * dy.x, ay.y * dz.y - az.y * dy.y);
-              const float2 wy = make_float2(az.x * dx.x - ax.x * dz.x, az.y * dx.y - ax.y * dz.y);
-              const float2 wz = make_float2(ax.x * dy.x - ay.x * dx.x, ax.y * dy.y - ay.y * dx.y);
-              sv2[0] = __ffma2_rn(qq, wx, sv2[0]);
-              sv2[1] = __ffma2_rn(qq, wy, sv2[1]);
-              sv2[2] = __ffma2_rn(qq, wz, sv2[2]);
-              float2 dot = __fmul2_rn(AT3[0], wx);
-              dot = __ffma2_rn(AT3[1], wy, dot);
-              dot = __ffma2_rn(AT3[2], wz, dot);
-              const float2 fd = __fmul2_rn(qA, dot);
-              sd2[0] = __ffma2_rn(fd, dx, sd2[0]);
-              sd2[1] = __ffma2_rn(fd, dy, sd2[1]);
-              sd2[2] = __ffma2_rn(fd, dz, sd2[2]);
-              sp2[0] = __ffma2_rn(qq, ax, sp2[0]);
-              sp2[1] = __ffma2_rn(qq, ay, sp2[1]);
-              sp2[2] = __ffma2_rn(qq, az, sp2[2]);
-            }
-            float sv[3], sd[3], sp[3], sdv[3] = {0.f, 0.f, 0.f};
-            for (int m = 0; m < 3; ++m) {
-              sv[m] = sv2[m].x + sv2[m].y;
-              sd[m] = sd2[m].x + sd2[m].y;
-              sp[m] = sp2[m].x + sp2[m].y;
-            }
-            fold_group(at, a.nu2, sv, sd, sp, sdv, vh, vl, dh, dl);
-          }
-          continue;
+          far_slice(st, npr, X2, AT3, xt[0] - rx, xt[1] - ry, xt[2] - rz, sv, sd, sp);
+        } else if (warp_min(hmin) == sbx.hs && thmin == tb.hs) {
+          const MidSigma2 g = mid_sigma2(dup2(tb.hs + sbx.hs));
+          mid_slice<false, false>(st, npr, X2, xt, at, hst, vt, &g, sv, sd, sp, sdv, nfull);
+        } else {
+          mid_slice<false, false>(st, npr, X2, xt, at, hst, vt, nullptr, sv, sd, sp, sdv, nfull);
         }
-        for (int g = 0; g < npr; g += 16) {
-          float2 sv2[3], sd2[3], sp2[3], sdv2[3];
-          for (int m = 0; m < 3; ++m) { sv2[m] = sd2[m] = sp2[m] = sdv2[m] = dup2(0.f); }
-          const int ge = min(npr, g + 16);
-          for (int r = g; r < ge; ++r) {
-            const float4 pa = ws.sP[2 * r], pb = ws.sP[2 * r + 1];
-            const float4 qa = ws.sQ[2 * r], qb = ws.sQ[2 * r + 1];
-            const float2 dx = __ffma2_rn(make_float2(pa.x, pa.y), M1, X2[0]);
-            const float2 dy = __ffma2_rn(make_float2(pa.z, pa.w), M1, X2[1]);
-            const float2 dz = __ffma2_rn(make_float2(pb.x, pb.y), M1, X2[2]);
-            const float2 ax = make_float2(qa.x, qa.y), ay = make_float2(qa.z, qa.w), az = make_float2(qb.x, qb.y);
-            float2 r2 = __fmul2_rn(dx, dx);
-            r2 = __ffma2_rn(dy, dy, r2);
-            r2 = __ffma2_rn(dz, dz, r2);
-            const float2 s2 = __fadd2_rn(HS2, make_float2(pb.z, pb.w));
-            PairTerms2 t = pair_terms_mid2(r2, mid_sigma2(s2));
-            const bool lx = r2.x < s2.x, ly = r2.y < s2.y;  // u < 1
-            if (__any_sync(0xffffffffu, lx || ly)) {
-              if (lx) { const PairTerms<float> e = pair_terms_near(r2.x, s2.x); t.q.x = e.q; t.F.x = e.F; t.zd.x = e.zd; }
-              if (ly) { const PairTerms<float> e = pair_terms_near(r2.y, s2.y); t.q.y = e.q; t.F.y = e.F; t.zd.y = e.zd; }
-            }
-            // w = alpha_s x d (scalar: the negated operand is free)
-            const float2 wx = make_float2(ay.x * dz.x - az.x * dy.x, ay.y * dz.y - az.y * dy.y);
-            const float2 wy = make_float2(az.x * dx.x - ax.x * dz.x, az.y * dx.y - ax.y * dz.y);
-            const float2 wz = make_float2(ax.x * dy.x - ay.x * dx.x, ax.y * dy.y - ay.y * dx.y);
-            sv2[0] = __ffma2_rn(t.q, wx, sv2[0]);
-            sv2[1] = __ffma2_rn(t.q, wy, sv2[1]);
-            sv2[2] = __ffma2_rn(t.q, wz, sv2[2]);
-            float2 dot = __fmul2_rn(AT2[0], wx);
-            dot = __ffma2_rn(AT2[1], wy, dot);
-            dot = __ffma2_rn(AT2[2], wz, dot);
-            const float2 fd = __fmul2_rn(t.F, dot);
-            sd2[0] = __ffma2_rn(fd, dx, sd2[0]);
-            sd2[1] = __ffma2_rn(fd, dy, sd2[1]);
-            sd2[2] = __ffma2_rn(fd, dz, sd2[2]);
-            sp2[0] = __ffma2_rn(t.q, ax, sp2[0]);
-            sp2[1] = __ffma2_rn(t.q, ay, sp2[1]);
-            sp2[2] = __ffma2_rn(t.q, az, sp2[2]);
-            // diffusion per pair: zeta (v_t a_s - v_s a_t), as in DIFFUSION (interaction_utils.h:358-369)
-            const float2 vs = make_float2(qb.z, qb.w);
-            sdv2[0] = __ffma2_rn(t.zd, __ffma2_rn(vs, NAT2[0], __fmul2_rn(VT2, ax)), sdv2[0]);
-            sdv2[1] = __ffma2_rn(t.zd, __ffma2_rn(vs, NAT2[1], __fmul2_rn(VT2, ay)), sdv2[1]);
-            sdv2[2] = __ffma2_rn(t.zd, __ffma2_rn(vs, NAT2[2], __fmul2_rn(VT2, az)), sdv2[2]);
-          }
-          float sv[3], sd[3], sp[3], sdv[3];
-          for (int m = 0; m < 3; ++m) {
-            sv[m] = sv2[m].x + sv2[m].y;
-            sd[m] = sd2[m].x + sd2[m].y;
-            sp[m] = sp2[m].x + sp2[m].y;
-            sdv[m] = sdv2[m].x + sdv2[m].y;
-          }
-          fold_group(at, a.nu2, sv, sd, sp, sdv, vh, vl, dh, dl);
-        }
+        fold_group_f32<false>(far_tile, xt[0] - rx, xt[1] - ry, xt[2] - rz, at, a.nu2, sv, sd, sp, sdv, vh, vl, dh, dl);
       }
     }
     if (mine) {
@@ -651,43 +523,6 @@ __global__ void slice_write_kernel(const int *cnt, const int *off, int nleaves, 
   const int li = blockIdx.x * blockDim.x + threadIdx.x;
   if (li < nleaves)
     for (int k = 0; k < cnt[li]; ++k) items[off[li] + k] = make_int2(li, k);
-}
-
-// Exact rates (direct FP32C sum over all n particles of the system) at nt
-// sampled targets, split over gridDim.y source chunks:
-// out[c][m][t], m = 0..5.
-__global__ void __launch_bounds__(kTreeBlock) sample_exact_kernel(const float4 *P, const float4 *Q, int64_t off,
-                                                                  int64_t n, const int *targets, int nt, float nu2,
-                                                                  double *out) {
-  __shared__ float4 sP[kTreeBlock], sQ[kTreeBlock];
-  const int tid = threadIdx.x;
-  const int ti = blockIdx.x * kTreeBlock + tid;
-  const int64_t t = off + targets[min(ti, nt - 1)];
-  const float4 pt = P[t], qt = Q[t];
-  const float xt[3] = {pt.x, pt.y, pt.z}, at[3] = {qt.x, qt.y, qt.z};
-  const float hst = pt.w, h50 = kFarU * pt.w, vt = qt.w;
-  float vh[3] = {0, 0, 0}, vl[3] = {0, 0, 0}, dh[3] = {0, 0, 0}, dl[3] = {0, 0, 0};
-  const int64_t per = (n + gridDim.y - 1) / gridDim.y;
-  const int64_t s0 = off + blockIdx.y * per, s1 = min(off + n, s0 + per);
-  for (int64_t sb = s0; sb < s1; sb += kTreeBlock) {
-    __syncthreads();
-    const int64_t j = sb + tid;
-    if (j < s1) { sP[tid] = P[j]; sQ[tid] = Q[j]; }
-    else { sP[tid] = pad_P<float>(); sQ[tid] = pad_Q<float>(); }
-    __syncthreads();
-    for (int g = 0; g < kTreeBlock; g += 32) {
-      float sv[3] = {}, sd[3] = {}, sp[3] = {}, sdv[3] = {};
-      for (int jj = 0; jj < 32; ++jj) pair_accum_f32(sP[g + jj], sQ[g + jj], xt, at, hst, h50, vt, sv, sd, sp, sdv);
-      fold_group(at, nu2, sv, sd, sp, sdv, vh, vl, dh, dl);
-    }
-  }
-  if (ti < nt) {
-    double *o = out + (int64_t)blockIdx.y * 6 * nt + ti;
-    for (int m = 0; m < 3; ++m) {
-      o[m * nt] = ((double)vh[m] + (double)vl[m]) * kInv4Pi;
-      o[(3 + m) * nt] = ((double)dh[m] + (double)dl[m]) * kInv4Pi;
-    }
-  }
 }
 
 // Max-norm errors of the surrogate rates (chunk 0 of partial) at the sampled
