@@ -690,29 +690,67 @@ __global__ void pack_kernel(const double *x0, const double *sig, const double *v
   }
 }
 
-// Host row-major (n, 3) position / strength + (n) radius / volume, staged in
-// device memory, scattered into the SoA state at slot offset `off`.
-static __global__ void scatter_kernel(const double *stage, int64_t n, int64_t off, int64_t cap, double *x0, double *sig,
-                               double *vol) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      x0[m * cap + off + i] = stage[3 * i + m];
-      x0[(3 + m) * cap + off + i] = stage[3 * n + 3 * i + m];
+// Host row-major layout <-> SoA.  A CTA takes kIoRows rows through shared
+// memory, so that both sides are read and written in whole segments: the
+// row-major side may be pinned host memory, mapped (uploads and downloads of a
+// few thousand particles need no copy of their own then).
+constexpr int kIoRows = 256;
+
+// Row-major (n, 3) positions and strengths, (n) radii and volumes, one after
+// another in `stage` -> SoA state at slot offset `off`, and the rows' source
+// records (and split-position residuals when L is set).
+template <typename T>
+__global__ void __launch_bounds__(kIoRows) upload_kernel(const double *stage, int64_t n, int64_t off, int64_t cap,
+                                                         double *x0, double *sig, double *vol, void *P, void *Q,
+                                                         float4 *L) {
+  __shared__ double s[6 * kIoRows];
+  for (int64_t b = blockIdx.x * (int64_t)kIoRows; b < n; b += (int64_t)gridDim.x * kIoRows) {
+    const int rows = (int)min((int64_t)kIoRows, n - b);
+    for (int t = threadIdx.x; t < 3 * rows; t += kIoRows) {
+      s[t] = stage[3 * b + t];
+      s[3 * kIoRows + t] = stage[3 * n + 3 * b + t];
     }
-    sig[off + i] = stage[6 * n + i];
-    vol[off + i] = stage[7 * n + i];
+    __syncthreads();
+    if ((int)threadIdx.x < rows) {
+      const int64_t j = b + threadIdx.x, i = off + j;
+      double y[6];
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        y[m] = s[3 * threadIdx.x + m];
+        y[3 + m] = s[3 * kIoRows + 3 * threadIdx.x + m];
+      }
+#pragma unroll
+      for (int m = 0; m < 6; ++m) x0[m * cap + i] = y[m];
+      const double sg = stage[6 * n + j], v = stage[7 * n + j];
+      sig[i] = sg;
+      vol[i] = v;
+      static_cast<v4_t<T> *>(P)[i] = make_v4<T>((T)y[0], (T)y[1], (T)y[2], (T)(0.5 * sg * sg));
+      static_cast<v4_t<T> *>(Q)[i] = make_v4<T>((T)y[3], (T)y[4], (T)y[5], (T)v);
+      if (L) L[i] = split_low(y[0], y[1], y[2]);
+    }
+    __syncthreads();
   }
 }
 
 // SoA [6][cap] (from slot offset `off`) -> row-major (n, 3) x 2.
-static __global__ void gather_kernel(const double *src, int64_t n, int64_t off, int64_t cap, double *stage) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+static __global__ void __launch_bounds__(kIoRows) gather_kernel(const double *src, int64_t n, int64_t off, int64_t cap,
+                                                                double *stage) {
+  __shared__ double s[6 * kIoRows];
+  for (int64_t b = blockIdx.x * (int64_t)kIoRows; b < n; b += (int64_t)gridDim.x * kIoRows) {
+    const int rows = (int)min((int64_t)kIoRows, n - b);
+    if ((int)threadIdx.x < rows) {
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      stage[3 * i + m] = src[m * cap + off + i];
-      stage[3 * n + 3 * i + m] = src[(3 + m) * cap + off + i];
+      for (int m = 0; m < 3; ++m) {
+        s[3 * threadIdx.x + m] = src[m * cap + off + b + threadIdx.x];
+        s[3 * kIoRows + 3 * threadIdx.x + m] = src[(3 + m) * cap + off + b + threadIdx.x];
+      }
     }
+    __syncthreads();
+    for (int t = threadIdx.x; t < 3 * rows; t += kIoRows) {
+      stage[3 * b + t] = s[t];
+      stage[3 * n + 3 * b + t] = s[3 * kIoRows + t];
+    }
+    __syncthreads();
   }
 }
 

@@ -113,7 +113,7 @@ struct pgpu_ctx {
   bool frozen = false;
   int64_t cap = 0;
   double *x0 = nullptr, *acc = nullptr, *rates = nullptr, *sig = nullptr, *vol = nullptr;
-  double *partial = nullptr, *stage = nullptr, *d_diag = nullptr;
+  double *partial = nullptr, *stage = nullptr;
   void *P = nullptr, *Q = nullptr;
   int64_t *d_sysoff = nullptr, *d_sysn = nullptr, *d_syst = nullptr;
   PlanEntry *d_plan = nullptr, *d_plan_diag = nullptr, *d_plan_field = nullptr;
@@ -127,7 +127,12 @@ struct pgpu_ctx {
   float4 *d_box = nullptr;  // FP32 source boxes per kBoxGran slots (box_kernel), FP32C Gaussian contexts
   float4 *d_L = nullptr;    // [cap] split-position residuals (pgpu_config.split_positions)
   int64_t pairs_acc = 0, selfs_acc = 0;  // ordered pairs and self pairs of the pair launches so far
-  int *d_flag = nullptr;
+  // Pinned host memory of the context, mapped: the non-finite flag the kernels
+  // set (h_flag), then a ring of io_bytes for small transfers (io_take), so
+  // that a call on a few thousand particles queues kernels and no copies.
+  unsigned char *h_io = nullptr;
+  size_t io_bytes = 0, io_pos = 0;
+  int *h_flag = nullptr;
   int diag_blocks = 0;
   int shape = 2;  // (256, 1) before autotuning: the high-order kernel's default (pgpu_create picks the Gaussian's)
   // Shapes per system chosen by pgpu_autotune_classes (empty: `shape` for
@@ -150,7 +155,8 @@ struct pgpu_ctx {
   double pair_ms = 0.0;
   int64_t pair_launches = 0;
   int64_t launches = 0;
-  std::map<std::tuple<int, double, int, int, bool>, cudaGraphExec_t> graphs;  // (scheme, dt, launch layout, nch, timing)
+  // (scheme, dt, launch layout, nch, timing, first event slot)
+  std::map<std::tuple<int, double, int, int, bool, int>, cudaGraphExec_t> graphs;
   std::vector<cudaGraph_t> graph_defs;
   // last error message: a fixed buffer under a mutex, since pgpu_snapshot_wait
   // may fail on a writer thread while the owning thread queues work
@@ -283,6 +289,40 @@ template <typename T> int occupancy(pgpu_ctx *c, int s) {
   return nb * c->sms;
 }
 
+// Largest ring of pinned memory for small transfers (pinning 2 MB takes 2 ms of
+// the first upload, 512 kB a quarter of that), and the largest transfer that
+// goes through it, in pieces of half a ring.  A larger one takes the driver's
+// own staging of pageable copies, whose time is the copy's.
+constexpr size_t kIoMax = 512 << 10;
+constexpr int64_t kIoRowsMax = 65536;
+
+// `bytes` of the context's pinned ring for work on its stream, nullptr if it is
+// larger than the ring.  When the ring is used up, waits for the stream, whose
+// work no longer needs any of it then.
+unsigned char *io_take(pgpu_ctx *c, size_t bytes) {
+  bytes = (bytes + 63) / 64 * 64;
+  if (bytes > c->io_bytes) return nullptr;
+  if (c->io_pos + bytes > c->io_bytes) {
+    if (cudaStreamSynchronize(c->st) != cudaSuccess) return nullptr;  // the next call on the stream reports it
+    c->io_pos = 0;
+  }
+  unsigned char *p = c->h_io + 64 + c->io_pos;
+  c->io_pos += bytes;
+  return p;
+}
+
+// Rows of a piece: half a ring of the 8 doubles an uploaded row takes.
+int64_t io_rows(const pgpu_ctx *c) { return std::max<int64_t>(1, (int64_t)(c->io_bytes / 128)); }
+
+// Queues a copy of host data to the device through the ring; data too large
+// for it is copied at once (the stream is waited for).
+cudaError_t put_data(pgpu_ctx *c, void *dst, const void *src, size_t bytes) {
+  unsigned char *h = io_take(c, bytes);
+  if (h) memcpy(h, src, bytes);
+  const cudaError_t e = cudaMemcpyAsync(dst, h ? h : src, bytes, cudaMemcpyHostToDevice, c->st);
+  return e != cudaSuccess || h ? e : cudaStreamSynchronize(c->st);
+}
+
 // Freeze the slot layout and allocate device memory (first upload).
 int freeze(pgpu_ctx *c) {
   if (c->frozen) return PGPU_OK;
@@ -333,9 +373,19 @@ int freeze(pgpu_ctx *c) {
     if ((r = alloc((void **)&c->d_L, cap * sizeof(float4)))) return r;
     CK(cudaMemsetAsync(c->d_L, 0, cap * sizeof(float4), c->st));
   }
-  if ((r = alloc((void **)&c->d_flag, sizeof(int)))) return r;
+  // at least the sums of one diagnostics call and a small work plan
+  c->io_bytes = std::min<size_t>(std::max<size_t>(8 * cap * sizeof(double), 64 << 10), kIoMax);
+  {
+    const cudaError_t e = cudaHostAlloc((void **)&c->h_io, 64 + c->io_bytes, cudaHostAllocMapped);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      c->h_io = nullptr;
+      return fail(c, PGPU_ENOMEM, "pinned transfer buffer of %zu bytes: %s", c->io_bytes, cudaGetErrorString(e));
+    }
+    c->h_flag = reinterpret_cast<int *>(c->h_io);
+    *c->h_flag = 0;
+  }
   c->diag_blocks = 2 * c->sms;
-  if ((r = alloc((void **)&c->d_diag, (size_t)c->diag_blocks * kDiagFields * sizeof(double)))) return r;
   CK(cudaMemsetAsync(c->x0, 0, 6 * cap * sizeof(double), c->st));
   CK(cudaMemsetAsync(c->acc, 0, 6 * cap * sizeof(double), c->st));
   CK(cudaMemsetAsync(c->rates, 0, 6 * cap * sizeof(double), c->st));
@@ -344,7 +394,6 @@ int freeze(pgpu_ctx *c) {
   CK(cudaMemsetAsync(c->partial, 0, (size_t)kMaxChunks * 6 * cap * sizeof(double), c->st));
   CK(cudaMemsetAsync(c->d_counters, 0, 4 * sizeof(unsigned int), c->st));
   CK(cudaMemsetAsync(c->d_nfull, 0, sizeof(unsigned long long), c->st));
-  CK(cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->st));
   for (int s = 0; s < kNumShapes; ++s) c->grid[s] = fp64(c) ? occupancy<double>(c, s) : occupancy<float>(c, s);
   for (int v = 0; v < kNumSlices; ++v) {
     int nb = 0;
@@ -584,9 +633,6 @@ int upload_plan(pgpu_ctx *c) {
   std::vector<int64_t> off(c->sys.size() + 1), n(c->sys.size());
   for (size_t s = 0; s < c->sys.size(); ++s) { off[s] = c->sys[s].off; n[s] = sys_n(c, (int)s); }
   off[c->sys.size()] = c->cap;
-  CK(cudaMemcpyAsync(c->d_plan, plan.data(), plan.size() * sizeof(PlanEntry), cudaMemcpyHostToDevice, c->st));
-  CK(cudaMemcpyAsync(c->d_sysoff, off.data(), off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, c->st));
-  CK(cudaMemcpyAsync(c->d_sysn, n.data(), n.size() * sizeof(int64_t), cudaMemcpyHostToDevice, c->st));
   std::vector<int64_t> t(2 * c->sys.size());
   for (size_t k = 0; k < c->sys.size(); ++k) {
     // an unrestricted system owns every slot, including particles appended later
@@ -594,9 +640,10 @@ int upload_plan(pgpu_ctx *c) {
     t[2 * k] = c->sys[k].t_count < 0 ? 0 : o.first;
     t[2 * k + 1] = c->sys[k].t_count < 0 ? INT64_MAX : o.first + o.second;
   }
-  CK(cudaMemcpyAsync(c->d_syst, t.data(), t.size() * sizeof(int64_t), cudaMemcpyHostToDevice, c->st));
-  // Pageable host sources: make sure the copies are done before the vectors go away.
-  CK(cudaStreamSynchronize(c->st));
+  CK(put_data(c, c->d_plan, plan.data(), plan.size() * sizeof(PlanEntry)));
+  CK(put_data(c, c->d_sysoff, off.data(), off.size() * sizeof(int64_t)));
+  CK(put_data(c, c->d_sysn, n.data(), n.size() * sizeof(int64_t)));
+  CK(put_data(c, c->d_syst, t.data(), t.size() * sizeof(int64_t)));
   c->plan_dirty = false;
   return PGPU_OK;
 }
@@ -683,7 +730,7 @@ int launch_stage(pgpu_ctx *c, int scheme, int stage, double dt) {
   s.sys_off = c->d_sysoff; s.sys_n = c->d_sysn; s.sys_t = c->d_syst; s.nsys = (int)c->sys.size();
   s.nch = c->nch; s.cap = c->cap; s.scheme = scheme; s.stage = stage; s.dt = dt;
   for (int m = 0; m < 3; ++m) s.vinf[m] = c->cfg.vinf[m];
-  s.flag = c->d_flag;
+  s.flag = c->h_flag;
   const int grid = (int)std::min<int64_t>(ceil_div(c->cap, kStageParticles), 10LL * c->sms);
   if (fp64(c)) stage_kernel<double><<<grid, kStageBlock, 0, c->st>>>(s);
   else stage_kernel<float><<<grid, kStageBlock, 0, c->st>>>(s);
@@ -712,10 +759,12 @@ int launch_eval(pgpu_ctx *c, int slot) {
   return fp64(c) ? launch_pair<double>(c, slot) : launch_pair<float>(c, slot);
 }
 
-int collect_timing(pgpu_ctx *c, int nslots) {
+// Reads the pair-kernel times of event slots [base, base + nslots), waiting for
+// the last of them.
+int collect_timing(pgpu_ctx *c, int nslots, int base = 0) {
   if (!c->timing || c->sur) return PGPU_OK;  // surrogate evaluations keep their own phase times
-  for (int k = 0; k < nslots; ++k) {
-    CK(cudaEventSynchronize(c->ev[k][1]));
+  CK(cudaEventSynchronize(c->ev[base + nslots - 1][1]));
+  for (int k = base; k < base + nslots; ++k) {
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, c->ev[k][0], c->ev[k][1]));
     c->pair_ms += ms;
@@ -726,10 +775,10 @@ int collect_timing(pgpu_ctx *c, int nslots) {
 
 int stages_of(int scheme) { return scheme == PGPU_RK4 ? 4 : scheme == PGPU_RK3 ? 3 : 1; }
 
-int record_step(pgpu_ctx *c, int scheme, double dt) {
+int record_step(pgpu_ctx *c, int scheme, double dt, int base = 0) {
   const int ns = stages_of(scheme);
   for (int k = 0; k < ns; ++k) {
-    int r = launch_eval(c, k);
+    int r = launch_eval(c, base + k);
     if (r) return r;
     if ((r = launch_stage(c, scheme, k, dt))) return r;
   }
@@ -746,15 +795,33 @@ int upload_rows(pgpu_ctx *c, const WakeRec &W, int64_t first, int64_t m, const d
                 const double *sigma, const double *vol) {
   if (m <= 0) return PGPU_OK;
   if (!pos || !alpha || !sigma || !vol) return fail(c, PGPU_EINVAL, "null particle array");
+  auto fn = fp64(c) ? upload_kernel<double> : upload_kernel<float>;
+  auto launch = [&](const double *rows, int64_t at, int64_t k) -> int {
+    const int grid = (int)std::min<int64_t>(ceil_div(k, kIoRows), 8LL * c->sms);
+    fn<<<grid, kIoRows, 0, c->st>>>(rows, k, W.off + first + at, c->cap, c->x0, c->sig, c->vol, c->P, c->Q, c->d_L);
+    CK(cudaGetLastError());
+    c->launches++;
+    return PGPU_OK;
+  };
+  if (m <= kIoRowsMax) {
+    const int64_t piece = io_rows(c);
+    for (int64_t at = 0; at < m; at += piece) {
+      const int64_t k = std::min(piece, m - at);
+      double *h = reinterpret_cast<double *>(io_take(c, 8 * k * sizeof(double)));
+      if (!h) return fail(c, PGPU_ECUDA, "waiting for the pinned transfer buffer failed");
+      memcpy(h, pos + 3 * at, 3 * k * sizeof(double));
+      memcpy(h + 3 * k, alpha + 3 * at, 3 * k * sizeof(double));
+      memcpy(h + 6 * k, sigma + at, k * sizeof(double));
+      memcpy(h + 7 * k, vol + at, k * sizeof(double));
+      if (int r = launch(h, at, k)) return r;
+    }
+    return PGPU_OK;
+  }
   CK(cudaMemcpyAsync(c->stage, pos, 3 * m * sizeof(double), cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(c->stage + 3 * m, alpha, 3 * m * sizeof(double), cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(c->stage + 6 * m, sigma, m * sizeof(double), cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(c->stage + 7 * m, vol, m * sizeof(double), cudaMemcpyHostToDevice, c->st));
-  const int grid = (int)std::min<int64_t>(ceil_div(m, 256), 16LL * c->sms);
-  scatter_kernel<<<grid, 256, 0, c->st>>>(c->stage, m, W.off + first, c->cap, c->x0, c->sig, c->vol);
-  CK(cudaGetLastError());
-  c->launches++;
-  return launch_pack(c, W.off + first, W.off + first + m);
+  return launch(c->stage, 0, m);
 }
 
 }  // namespace
@@ -822,12 +889,13 @@ int pgpu_destroy(pgpu_ctx *c) {
   surrogate_free(c);
   for (auto &g : c->graphs) cudaGraphExecDestroy(g.second);
   for (auto g : c->graph_defs) cudaGraphDestroy(g);
-  void *ptrs[] = {c->x0, c->acc, c->rates, c->sig, c->vol, c->partial, c->stage, c->d_diag, c->P, c->Q,
+  void *ptrs[] = {c->x0, c->acc, c->rates, c->sig, c->vol, c->partial, c->stage, c->P, c->Q,
                   c->d_sysoff, c->d_sysn, c->d_syst, c->d_plan, c->d_plan_diag, c->d_plan_field, c->d_field,
-                  c->d_counters, c->d_nfull, c->d_flag, c->d_merge, c->d_merge_tmp, c->d_box, c->d_L};
+                  c->d_counters, c->d_nfull, c->d_merge, c->d_merge_tmp, c->d_box, c->d_L};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (int k = 0; k < 8; ++k) { cudaEventDestroy(c->ev[k][0]); cudaEventDestroy(c->ev[k][1]); }
+  if (c->h_io) cudaFreeHost(c->h_io);
   if (c->st_copy) cudaStreamSynchronize(c->st_copy);
   for (int s = 0; s < 2; ++s) {
     if (c->d_snap[s]) cudaFree(c->d_snap[s]);
@@ -863,8 +931,8 @@ int pgpu_set_particles(pgpu_ctx *c, int32_t wake, int64_t n, const double *pos, 
   WakeRec &W = c->wakes[wake];
   if (n < 0 || n > W.cap) return fail(c, PGPU_EINVAL, "n=%lld exceeds the capacity %lld of wake %d", (long long)n, (long long)W.cap, wake);
   if ((r = upload_rows(c, W, 0, n, pos, alpha, sigma, vol))) return r;
+  if (W.n != n) c->plan_dirty = true;  // the work list depends on the sizes alone
   W.n = n;
-  c->plan_dirty = true;
   return PGPU_OK;
 }
 
@@ -893,13 +961,45 @@ int pgpu_get_num_particles(pgpu_ctx *c, int32_t wake, int64_t *n) {
 
 static int download_rows(pgpu_ctx *c, const double *src, const WakeRec &W, double *a, double *b) {
   if (W.n == 0) return PGPU_OK;
-  const int grid = (int)std::min<int64_t>(ceil_div(W.n, 256), 16LL * c->sms);
-  gather_kernel<<<grid, 256, 0, c->st>>>(src, W.n, W.off, c->cap, c->stage);
-  CK(cudaGetLastError());
-  c->launches++;
-  CK(cudaMemcpyAsync(a, c->stage, 3 * W.n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaMemcpyAsync(b, c->stage + 3 * W.n, 3 * W.n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
+  auto launch = [&](int64_t at, int64_t k, double *dst) -> int {
+    const int grid = (int)std::min<int64_t>(ceil_div(k, kIoRows), 8LL * c->sms);
+    gather_kernel<<<grid, kIoRows, 0, c->st>>>(src, k, W.off + at, c->cap, dst);
+    CK(cudaGetLastError());
+    c->launches++;
+    return PGPU_OK;
+  };
+  if (W.n > kIoRowsMax) {
+    if (int r = launch(0, W.n, c->stage)) return r;
+    CK(cudaMemcpyAsync(a, c->stage, 3 * W.n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(b, c->stage + 3 * W.n, 3 * W.n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    return PGPU_OK;
+  }
+  // two pieces in the ring at a time, then on to the caller's arrays
+  const int64_t piece = io_rows(c);
+  for (int64_t at = 0; at < W.n; at += 2 * piece) {
+    double *h[2] = {nullptr, nullptr};
+    for (int q = 0; q < 2; ++q) {
+      const int64_t lo = at + q * piece, k = std::min(piece, W.n - lo);
+      if (k <= 0) break;
+      h[q] = reinterpret_cast<double *>(io_take(c, 6 * k * sizeof(double)));
+      if (!h[q]) return fail(c, PGPU_ECUDA, "waiting for the pinned transfer buffer failed");
+      if (q == 1 && h[1] <= h[0]) {  // the ring started over and the first piece has landed: take it out first
+        memcpy(a + 3 * at, h[0], 3 * piece * sizeof(double));
+        memcpy(b + 3 * at, h[0] + 3 * piece, 3 * piece * sizeof(double));
+        h[0] = nullptr;
+      }
+      if (int r = launch(lo, k, h[q])) return r;
+    }
+    CK(cudaStreamSynchronize(c->st));
+    for (int q = 0; q < 2; ++q) {
+      const int64_t lo = at + q * piece, k = std::min(piece, W.n - lo);
+      if (!h[q]) continue;
+      memcpy(a + 3 * lo, h[q], 3 * k * sizeof(double));
+      memcpy(b + 3 * lo, h[q] + 3 * k, 3 * k * sizeof(double));
+    }
+    c->io_pos = 0;  // the stream is idle: nothing needs the ring any more
+  }
   return PGPU_OK;
 }
 
@@ -1038,31 +1138,41 @@ int pgpu_step(pgpu_ctx *c, int scheme, double dt, int32_t nsteps) {
     }
     return PGPU_OK;
   }
-  auto key = std::make_tuple(scheme, dt, launch_layout(c), c->nch, c->timing);
-  auto it = c->graphs.find(key);
-  if (it == c->graphs.end()) {
-    cudaGraph_t g;
-    CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-    const int64_t before = c->launches;
-    c->capturing = true;
-    r = record_step(c, scheme, dt);
-    c->capturing = false;
-    cudaError_t e = cudaStreamEndCapture(c->st, &g);
-    if (r) return r;
-    if (e != cudaSuccess) return fail(c, PGPU_ECUDA, "stream capture failed: %s", cudaGetErrorString(e));
-    c->launches = before;  // counted at replay
-    cudaGraphExec_t ex;
-    CK(cudaGraphInstantiate(&ex, g, 0));
-    c->graph_defs.push_back(g);
-    it = c->graphs.emplace(key, ex).first;
-  }
+  // With timing on, the steps of a call alternate between two graphs with
+  // their own event slots, so that a step's times are read while the next one
+  // runs (5000 particles: the device would idle 15 us between steps).
+  auto graph = [&](int base, cudaGraphExec_t *out) -> int {
+    auto key = std::make_tuple(scheme, dt, launch_layout(c), c->nch, c->timing, base);
+    auto it = c->graphs.find(key);
+    if (it == c->graphs.end()) {
+      cudaGraph_t g;
+      CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
+      const int64_t before = c->launches;
+      c->capturing = true;
+      const int rr = record_step(c, scheme, dt, base);
+      c->capturing = false;
+      cudaError_t e = cudaStreamEndCapture(c->st, &g);
+      if (rr) return rr;
+      if (e != cudaSuccess) return fail(c, PGPU_ECUDA, "stream capture failed: %s", cudaGetErrorString(e));
+      c->launches = before;  // counted at replay
+      cudaGraphExec_t ex;
+      CK(cudaGraphInstantiate(&ex, g, 0));
+      c->graph_defs.push_back(g);
+      it = c->graphs.emplace(key, ex).first;
+    }
+    *out = it->second;
+    return PGPU_OK;
+  };
   for (int i = 0; i < nsteps; ++i) {
-    CK(cudaGraphLaunch(it->second, c->st));
+    cudaGraphExec_t ex;
+    const int base = c->timing && (i & 1) ? 4 : 0;
+    if ((r = graph(base, &ex))) return r;
+    CK(cudaGraphLaunch(ex, c->st));
     c->launches += (1 + eval_launches(c)) * ns;
     account_pairs(c, ns);
-    if ((r = collect_timing(c, ns))) return r;
+    if (i > 0 && (r = collect_timing(c, ns, 4 - base))) return r;
   }
-  return PGPU_OK;
+  return nsteps > 0 ? collect_timing(c, ns, c->timing && ((nsteps - 1) & 1) ? 4 : 0) : PGPU_OK;
 }
 
 int pgpu_diagnose_partial(pgpu_ctx *c, int32_t system, double *fields) {
@@ -1086,8 +1196,7 @@ int pgpu_diagnose_partial(pgpu_ctx *c, int32_t system, double *fields) {
   // unordered pair is summed from its lower index, so the ranks' row ranges
   // together cover every pair once
   std::vector<PlanEntry> plan = build_plan(c, {system}, shape, nch);
-  CK(cudaMemcpyAsync(c->d_plan_diag, plan.data(), plan.size() * sizeof(PlanEntry), cudaMemcpyHostToDevice, c->st));
-  CK(cudaStreamSynchronize(c->st));
+  CK(put_data(c, c->d_plan_diag, plan.data(), plan.size() * sizeof(PlanEntry)));
   const bool quad = plan.size() > 1;
   if (quad) {
     int grid = 0;
@@ -1108,7 +1217,6 @@ int pgpu_diagnose_partial(pgpu_ctx *c, int32_t system, double *fields) {
     CK(cudaGetLastError());
     c->launches++;
   }
-  std::vector<double> h((size_t)c->diag_blocks * kDiagFields);
   const std::vector<int> &ws = c->sys[system].wakes;
   for (size_t k = 0; k < ws.size(); ++k) {
     const WakeRec &W = c->wakes[ws[k]];
@@ -1117,11 +1225,14 @@ int pgpu_diagnose_partial(pgpu_ctx *c, int32_t system, double *fields) {
     const int64_t lo = std::max(W.off, row_lo), hi = std::min(W.off + W.n, row_hi);
     if (hi <= lo) continue;
     const int grid = (int)std::min<int64_t>(ceil_div(hi - lo, 256), c->diag_blocks);
+    // the CTAs' sums go straight to the pinned ring (at most 296 x 23 values)
+    const size_t bytes = (size_t)grid * kDiagFields * sizeof(double);
+    double *h = reinterpret_cast<double *>(io_take(c, bytes));
+    if (!h) return fail(c, PGPU_ECUDA, "no pinned memory for the diagnostic sums");
     diag_wake_kernel<<<grid, 256, 0, c->st>>>(c->x0, c->sig, c->partial, nch, c->cap, lo, hi, quad ? 1 : 0,
-                                              c->cfg.kernel, c->d_diag);
+                                              c->cfg.kernel, h);
     CK(cudaGetLastError());
     c->launches++;
-    CK(cudaMemcpyAsync(h.data(), c->d_diag, (size_t)grid * kDiagFields * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     // per-CTA partials summed in CTA order: deterministic
     for (int b = 0; b < grid; ++b)
@@ -1199,7 +1310,10 @@ int pgpu_probe(pgpu_ctx *c, int32_t system, int64_t npts, const double *pts, dou
   double *d = c->stage;
   if (own) CK(cudaMallocAsync((void **)&d, need * sizeof(double), c->st));
   double *d_vel = d + 3 * npts, *d_part = d + 6 * npts;
-  CK(cudaMemcpyAsync(d, pts, 3 * npts * sizeof(double), cudaMemcpyHostToDevice, c->st));
+  CK(put_data(c, d, pts, 3 * npts * sizeof(double)));
+  // the velocities come back through the ring where they fit
+  double *h_vel = reinterpret_cast<double *>(io_take(c, 3 * npts * sizeof(double)));
+  if (h_vel) d_vel = h_vel;
   if (hi > lo) {
     auto fn = c->cfg.kernel == PGPU_KERNEL_HIGHORDER ? probe_kernel<kHighOrder> : probe_kernel<kGaussian>;
     fn<<<dim3((unsigned)tiles, (unsigned)chunks), kProbeBlock, 0, c->st>>>(c->x0, c->sig, c->cap, lo, hi, per, d, npts,
@@ -1212,9 +1326,11 @@ int pgpu_probe(pgpu_ctx *c, int32_t system, int64_t npts, const double *pts, dou
   } else {
     CK(cudaMemsetAsync(d_vel, 0, 3 * npts * sizeof(double), c->st));
   }
-  CK(cudaMemcpyAsync(vel, d_vel, 3 * npts * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  if (!h_vel) CK(cudaMemcpyAsync(vel, d_vel, 3 * npts * sizeof(double), cudaMemcpyDeviceToHost, c->st));
   if (own) CK(cudaFreeAsync(d, c->st));
   CK(cudaStreamSynchronize(c->st));
+  if (h_vel) memcpy(vel, h_vel, 3 * npts * sizeof(double));
+  c->io_pos = 0;  // the stream is idle
   return PGPU_OK;
 }
 
@@ -1223,10 +1339,8 @@ int pgpu_sync(pgpu_ctx *c) {
   DeviceScope device_scope(c->cfg.device);
   CK(cudaStreamSynchronize(c->st));
   if (c->frozen) {
-    int flag = 0;
-    CK(cudaMemcpy(&flag, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost));
-    if (flag) {
-      CK(cudaMemset(c->d_flag, 0, sizeof(int)));
+    if (*static_cast<volatile int *>(c->h_flag)) {
+      *c->h_flag = 0;
       return fail(c, PGPU_ENUMERIC, "a time step produced a non-finite particle state");
     }
   }
@@ -1260,8 +1374,7 @@ int pgpu_influence(pgpu_ctx *c) {
   const int grid = std::max(1, nb) * c->sms;
   const SlicesPlan p = build_slices_plan(c, v, grid, false);
   const int nch = p.nch;
-  CK(cudaMemcpyAsync(c->d_plan_field, p.plan.data(), p.plan.size() * sizeof(PlanEntry), cudaMemcpyHostToDevice, c->st));
-  CK(cudaStreamSynchronize(c->st));  // the plan vector is pageable host memory
+  CK(put_data(c, c->d_plan_field, p.plan.data(), p.plan.size() * sizeof(PlanEntry)));
   if (p.rows > 0) {
     FieldArgs a{c->x0, c->sig, c->partial, c->d_plan_field, (int)c->sys.size(), nch, c->cap};
     fn<<<grid, 32 * kSliceWarps, 0, c->st>>>(a);
@@ -1348,8 +1461,8 @@ int pgpu_snapshot_begin(pgpu_ctx *c, int32_t slot) {
     offs[w] = total;
     ns[w] = W.n;
     if (W.n > 0) {
-      const int grid = (int)std::min<int64_t>(ceil_div(W.n, 256), 16LL * c->sms);
-      gather_kernel<<<grid, 256, 0, c->st>>>(c->x0, W.n, W.off, c->cap, c->d_snap[slot] + 6 * total);
+      const int grid = (int)std::min<int64_t>(ceil_div(W.n, kIoRows), 8LL * c->sms);
+      gather_kernel<<<grid, kIoRows, 0, c->st>>>(c->x0, W.n, W.off, c->cap, c->d_snap[slot] + 6 * total);
       CK(cudaGetLastError());
       c->launches++;
     }

@@ -168,3 +168,35 @@ def test_field_keeps_non_finite_strengths(gpu):
     w.alpha[17, 1] = np.inf
     c, ids = context([w], capi.FP32C)
     assert np.isnan(c.vorticity_field(ids[0])[1600, 1])
+
+
+@pytest.mark.parametrize("prec", [capi.FP64, capi.FP32C])
+@pytest.mark.parametrize("n", [1, 255, 257, 512, 513, 4096, 4097, 8191, 24676, 65536, 65537])
+def test_transfers_in_pieces(gpu, n, prec):
+    """Uploads and downloads bit for bit, through the pinned ring in pieces and past its largest size; a second upload and
+    an append reuse the ring, and the plan follows the sizes."""
+    rng = np.random.default_rng(n)
+    big = n + 300
+    def wake(m):
+        return cases.Wake(rng.normal(size=(m, 3)), rng.normal(size=(m, 3)), rng.uniform(0.1, 0.2, m), rng.uniform(1, 2, m))
+    c = capi.Context(precision=prec, nu=NU)
+    k = c.add_wake(big)
+    w = wake(n)
+    for _ in range(2):
+        c.set_particles(k, w)
+        c.set_particles(k, w2 := wake(n))
+        more = wake(300)
+        c.append_particles(k, more)
+        x, a, s, v = c.particles(k)
+        for got, ref in ((x, "pos"), (a, "alpha"), (s, "sigma"), (v, "vol")):
+            assert np.array_equal(got, np.concatenate([getattr(w2, ref), getattr(more, ref)]))
+    c.set_particles(k, w)
+    y, b = c.state(k)
+    assert np.array_equal(y, w.pos) and np.array_equal(b, w.alpha)
+    if n <= 8191:
+        c.solve()
+        r, d = c.rates(k)
+        one, ids = context([w], prec)
+        one.solve()
+        for got, ref in zip((r, d), one.rates(ids[0])):
+            assert np.array_equal(got, ref)
