@@ -1279,10 +1279,11 @@ static __global__ void merge_grid_kernel(MergeArgs a) {
 // order.  Gaussian pairs at u >= kFarU64 take the far limit q = 1/rho^3, which
 // equals the closed form to double rounding; the closed form runs under a
 // warp vote.
-// 400 points of 100,000 particles, whole call: 0.31 ms, against 51.6 ms for one thread per
+// 400 points of 100,000 particles, whole call: 0.19 ms with 4 points per CTA (118
+// registers, two CTAs per SM), 0.30 with 8 (158), 0.24 with 2; 51.6 ms for one thread per
 // point over all particles (4 CTAs) with the closed form for every pair.
 constexpr int kProbeBlock = 256;
-constexpr int kProbePoints = 8;
+constexpr int kProbePoints = 4;
 
 template <int KER = kGaussian>
 __global__ void __launch_bounds__(kProbeBlock) probe_kernel(const double *x0, const double *sig, int64_t cap, int64_t lo,

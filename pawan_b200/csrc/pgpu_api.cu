@@ -1297,7 +1297,7 @@ int pgpu_probe(pgpu_ctx *c, int32_t system, int64_t npts, const double *pts, dou
   const int64_t lo = c->sys[system].off, hi = lo + sys_n(c, system);
   // Particle chunks: about eight CTAs per SM in all, of at least one particle
   // per thread, and at most 512 chunks, so that the reduction stays a small
-  // part (400 points: 24 chunks of 50 point tiles).
+  // part (400 points: 11 chunks of 100 point tiles).
   const int64_t tiles = ceil_div(npts, kProbePoints);
   int64_t chunks = std::min<int64_t>(std::max<int64_t>(1, 8LL * c->sms / tiles), 512);
   chunks = std::max<int64_t>(1, std::min(chunks, ceil_div(hi - lo, kProbeBlock)));
