@@ -9,7 +9,10 @@
 //      `leaf` particles is split into its non-empty octants, found by binary
 //      search of the sorted codes (split_count_kernel / split_write_kernel;
 //      child offsets from an exclusive scan, so the layout is deterministic)
-//   5. per-cell moments about the particle centroid (moments_kernel)
+//   5. per-cell moments about the particle centroid, FP64: the leaves from their
+//      particles (leaf_moments_kernel), the other cells from their children's,
+//      level by level (parent_moments_kernel); each leaf raises the spread radii
+//      of its ancestors (spread_kernel), and cell_data_kernel stores the cells
 //   6. per target leaf, the interaction lists (lists_kernel): a source cell
 //      whose centroid is at least `near_widths` cube widths beyond the target
 //      leaf's bounding sphere, and whose particles are all at least 4 sigma_ij
@@ -37,7 +40,7 @@ struct TreeCell {
   int first_child;      // index of the first child cell (children are contiguous), -1 for leaves
   int nchild;
   int level;
-  int pad;
+  int parent;           // -1 for the root
   unsigned long long prefix;  // Morton prefix of the cell (3 * level bits)
 };
 
@@ -136,206 +139,357 @@ __device__ __forceinline__ bool splittable(const TreeCell &c, int leaf) {
   return c.end - c.start > leaf && c.level < kTreeLevels;
 }
 
-// Number of non-empty octants of every cell of the frontier [f0, f1).
-__global__ void split_count_kernel(TreeCell *cells, int f0, int f1, const unsigned long long *code, int leaf,
+// The octants of every cell of the frontier [f0, f1), eight threads per cell:
+// thread o finds where octant o ends, so the searches of a cell run side by
+// side (the first levels are a handful of cells, and eight searches one after
+// another took 60 us of latency per level).  Returns the octant's particle
+// range, and in `mask` the non-empty octants of the cell.
+__device__ __forceinline__ int2 octant_range(const TreeCell &c, int o, int leaf, const unsigned long long *code,
+                                             unsigned &mask) {
+  int lo = c.start, hi = c.start;
+  const bool split = splittable(c, leaf);
+  if (split)
+    hi = lower_bound_prefix(code, c.start, c.end, 3 * (kTreeLevels - c.level - 1),
+                            (c.prefix << 3) + (unsigned long long)(o + 1));
+  const int prev = __shfl_up_sync(0xffffffffu, hi, 1, 8);
+  if (split && o > 0) lo = prev;
+  mask = (__ballot_sync(0xffffffffu, hi > lo) >> (threadIdx.x & 24)) & 0xffu;
+  return make_int2(lo, hi);
+}
+
+__global__ void split_count_kernel(const TreeCell *cells, int f0, int f1, const unsigned long long *code, int leaf,
                                    int *nchild) {
-  const int i = f0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= f1) return;
-  const TreeCell c = cells[i];
-  int k = 0;
-  if (splittable(c, leaf)) {
-    const int shift = 3 * (kTreeLevels - c.level - 1);
-    int lo = c.start;
-    for (int o = 0; o < 8; ++o) {
-      const int hi = lower_bound_prefix(code, lo, c.end, shift, (c.prefix << 3) + (unsigned long long)(o + 1));
-      k += hi > lo;
-      lo = hi;
-    }
-  }
-  nchild[i - f0] = k;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, i = f0 + (t >> 3), o = t & 7;
+  const TreeCell c = cells[min(i, f1 - 1)];
+  unsigned mask;
+  octant_range(c, o, leaf, code, mask);
+  if (i < f1 && o == 0) nchild[i - f0] = __popc(mask);
 }
 
 // Writes the children of every frontier cell at base + offs[i] (exclusive scan of nchild).
 __global__ void split_write_kernel(TreeCell *cells, int f0, int f1, const unsigned long long *code, int leaf,
                                    const int *offs, int base) {
-  const int i = f0 + blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, i = f0 + (t >> 3), o = t & 7;
+  const TreeCell c = cells[min(i, f1 - 1)];
+  unsigned mask;
+  const int2 r = octant_range(c, o, leaf, code, mask);
   if (i >= f1) return;
-  TreeCell c = cells[i];
-  if (!splittable(c, leaf)) {
-    cells[i].first_child = -1;
-    cells[i].nchild = 0;
-    return;
+  const int w = base + offs[i - f0];
+  if (r.y > r.x) {
+    TreeCell ch;
+    ch.start = r.x; ch.end = r.y; ch.first_child = -1; ch.nchild = 0; ch.level = c.level + 1; ch.parent = i;
+    ch.prefix = (c.prefix << 3) | (unsigned long long)o;
+    cells[w + __popc(mask & ((1u << o) - 1u))] = ch;
   }
-  const int shift = 3 * (kTreeLevels - c.level - 1);
-  int lo = c.start, w = base + offs[i - f0], k = 0;
-  for (int o = 0; o < 8; ++o) {
-    const int hi = lower_bound_prefix(code, lo, c.end, shift, (c.prefix << 3) + (unsigned long long)(o + 1));
-    if (hi > lo) {
-      TreeCell ch;
-      ch.start = lo; ch.end = hi; ch.first_child = -1; ch.nchild = 0; ch.level = c.level + 1; ch.pad = 0;
-      ch.prefix = (c.prefix << 3) | (unsigned long long)o;
-      cells[w + k] = ch;
-      ++k;
-    }
-    lo = hi;
+  if (o == 0) {
+    cells[i].first_child = mask ? w : -1;
+    cells[i].nchild = __popc(mask);
   }
-  cells[i].first_child = k ? w : -1;
-  cells[i].nchild = k;
 }
 
-__device__ __forceinline__ double block_sum_d(double v, double *red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double r = 0.0;
-  for (int k = 0; k < (int)(blockDim.x >> 5); ++k) r += red[k];
-  return r;
-}
-__device__ __forceinline__ float block_max_f(float v, float *red) {
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_down_sync(0xffffffffu, v, o));
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float r = 0.f;
-  for (int k = 0; k < (int)(blockDim.x >> 5); ++k) r = fmaxf(r, red[k]);
-  return r;
+// FP64 sums of a cell: particle positions, strength and sigma^2/2, the
+// moments about the centroid in the order of CellData (M 9, Q 18, T 30), the
+// spread radius (bits of a float, for atomicMax) and the largest sigma^2/2.
+// T only for expansions of order 3 (nm = kMoments), else nm = kMoments2.
+constexpr int kMoments = 57, kMoments2 = 27;
+struct CellSums {
+  double x[3], a[3], h;
+  double m[kMoments];
+  unsigned spread;
+  float hmax;
+};
+
+// What the interaction lists read of a cell, in one place.
+struct TreeNode {
+  float c[3], R;  // centroid, spread radius
+  float w, H;     // cube width, largest sigma^2/2
+  int start, end;
+  int first_child, nchild;
+  int pad[2];
+};
+
+__device__ __forceinline__ double warp_sum_d(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
-// One CTA per cell: centroid, total strength, first and second moments of
-// the strength about the centroid (FP64 sums, stored FP32).
-__global__ void moments_kernel(const TreeCell *cells, int ncells, const float4 *Ps, const float4 *Qs, const float *geo,
-                               CellData *out) {
-  __shared__ double red[32];
-  __shared__ float redf[32];
-  for (int ci = blockIdx.x; ci < ncells; ci += gridDim.x) {
-    const TreeCell c = cells[ci];
-    double s[7] = {0, 0, 0, 0, 0, 0, 0};
-    for (int i = c.start + threadIdx.x; i < c.end; i += blockDim.x) {
-      const float4 p = Ps[i], q = Qs[i];
-      s[0] += p.x; s[1] += p.y; s[2] += p.z; s[3] += q.x; s[4] += q.y; s[5] += q.z; s[6] += p.w;
-    }
-    double t[7];
-    for (int k = 0; k < 7; ++k) t[k] = block_sum_d(s[k], red);
-    const double cnt = (double)(c.end - c.start);
-    const double cx = t[0] / cnt, cy = t[1] / cnt, cz = t[2] / cnt;
-    double m[57];
-    for (int k = 0; k < 57; ++k) m[k] = 0.0;
-    float R = 0.f, H = 0.f;
-    for (int i = c.start + threadIdx.x; i < c.end; i += blockDim.x) {
-      const float4 p = Ps[i], q = Qs[i];
-      H = fmaxf(H, p.w);
-      const double y[3] = {p.x - cx, p.y - cy, p.z - cz};
-      const double a[3] = {q.x, q.y, q.z};
-      R = fmaxf(R, (float)sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]));
-      for (int aa = 0; aa < 3; ++aa) {
-        for (int b = 0; b < 3; ++b) m[3 * aa + b] += a[aa] * y[b];
-        m[9 + 6 * aa + 0] += a[aa] * y[0] * y[0];
-        m[9 + 6 * aa + 1] += a[aa] * y[0] * y[1];
-        m[9 + 6 * aa + 2] += a[aa] * y[0] * y[2];
-        m[9 + 6 * aa + 3] += a[aa] * y[1] * y[1];
-        m[9 + 6 * aa + 4] += a[aa] * y[1] * y[2];
-        m[9 + 6 * aa + 5] += a[aa] * y[2] * y[2];
-        double *o = m + 27 + 10 * aa;
-        o[0] += a[aa] * y[0] * y[0] * y[0];
-        o[1] += a[aa] * y[0] * y[0] * y[1];
-        o[2] += a[aa] * y[0] * y[0] * y[2];
-        o[3] += a[aa] * y[0] * y[1] * y[1];
-        o[4] += a[aa] * y[0] * y[1] * y[2];
-        o[5] += a[aa] * y[0] * y[2] * y[2];
-        o[6] += a[aa] * y[1] * y[1] * y[1];
-        o[7] += a[aa] * y[1] * y[1] * y[2];
-        o[8] += a[aa] * y[1] * y[2] * y[2];
-        o[9] += a[aa] * y[2] * y[2] * y[2];
+// One warp per leaf.
+template <int NM>
+__global__ void __launch_bounds__(128) leaf_moments_kernel(const TreeCell *cells, const int *leaves, int nleaves,
+                                                           const float4 *Ps, const float4 *Qs, CellSums *out) {
+  const int lane = threadIdx.x & 31;
+  const int li = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (li >= nleaves) return;
+  const int ci = leaves[li];
+  const int start = cells[ci].start, end = cells[ci].end;
+  double s[7] = {0, 0, 0, 0, 0, 0, 0};
+  float H = 0.f;
+  for (int i = start + lane; i < end; i += 32) {
+    const float4 p = Ps[i], q = Qs[i];
+    s[0] += p.x; s[1] += p.y; s[2] += p.z; s[3] += q.x; s[4] += q.y; s[5] += q.z; s[6] += p.w;
+    H = fmaxf(H, p.w);
+  }
+#pragma unroll
+  for (int k = 0; k < 7; ++k) s[k] = warp_sum_d(s[k]);
+  const double cnt = (double)(end - start);
+  const double cx = s[0] / cnt, cy = s[1] / cnt, cz = s[2] / cnt;
+  double m[NM];
+#pragma unroll
+  for (int k = 0; k < NM; ++k) m[k] = 0.0;
+  float R = 0.f;
+  for (int i = start + lane; i < end; i += 32) {
+    const float4 p = Ps[i], q = Qs[i];
+    const double y[3] = {p.x - cx, p.y - cy, p.z - cz};
+    const double a[3] = {q.x, q.y, q.z};
+    R = fmaxf(R, (float)sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]));
+#pragma unroll
+    for (int aa = 0; aa < 3; ++aa) {
+      int k2 = 9 + 6 * aa, k3 = 27 + 10 * aa;
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        const double ab = a[aa] * y[b];
+        m[3 * aa + b] += ab;
+#pragma unroll
+        for (int c = b; c < 3; ++c) {
+          const double abc = ab * y[c];
+          m[k2++] += abc;
+          if constexpr (NM > kMoments2) {
+#pragma unroll
+            for (int d = c; d < 3; ++d) m[k3++] += abc * y[d];
+          }
+        }
       }
     }
-    double mt[57];
-    for (int k = 0; k < 57; ++k) mt[k] = block_sum_d(m[k], red);
-    const float Rm = block_max_f(R, redf);
-    const float Hm = block_max_f(H, redf);
-    if (threadIdx.x == 0) {
-      CellData d;
-      d.v[0] = (float)cx; d.v[1] = (float)cy; d.v[2] = (float)cz;
-      d.v[3] = (float)t[3]; d.v[4] = (float)t[4]; d.v[5] = (float)t[5];
-      for (int k = 0; k < 27; ++k) d.v[6 + k] = (float)mt[k];
-      d.v[33] = Rm;
-      const float w = geo[3] / (float)(1u << c.level);
-      d.v[34] = w;
-      const unsigned long long pre = c.prefix;
-      const unsigned ix = compact21(pre), iy = compact21(pre >> 1), iz = compact21(pre >> 2);
-      d.v[35] = geo[0] + (ix + 0.5f) * w;
-      d.v[36] = geo[1] + (iy + 0.5f) * w;
-      d.v[37] = geo[2] + (iz + 0.5f) * w;
-      d.v[38] = (float)(t[6] / cnt);
-      d.v[39] = Hm;
-      for (int k = 0; k < 30; ++k) d.v[40 + k] = (float)mt[27 + k];
-      d.v[70] = 0.f;
-      d.v[71] = 0.f;
-      out[ci] = d;
-    }
-    __syncthreads();
+  }
+#pragma unroll
+  for (int k = 0; k < NM; ++k) m[k] = warp_sum_d(m[k]);
+  for (int o = 16; o > 0; o >>= 1) {
+    R = fmaxf(R, __shfl_xor_sync(0xffffffffu, R, o));
+    H = fmaxf(H, __shfl_xor_sync(0xffffffffu, H, o));
+  }
+  if (lane == 0) {
+    CellSums &c = out[ci];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { c.x[k] = s[k]; c.a[k] = s[3 + k]; }
+    c.h = s[6];
+#pragma unroll
+    for (int k = 0; k < NM; ++k) c.m[k] = m[k];
+    c.spread = __float_as_uint(R);
+    c.hmax = H;
   }
 }
 
-// Interaction lists of every leaf (one thread per leaf).  pass 0 counts,
-// pass 1 writes at the offsets of an exclusive scan of the counts.  Near
-// leaves are emitted as runs of the sorted particle order: consecutive near
-// leaves whose ranges touch are merged (siblings are visited in octant order,
-// which is sorted order, so runs are long).  The stack is bounded
-// (kListStack); overflow sets *err, and the caller treats a non-zero *err as a
-// failed build.
-__global__ void lists_kernel(const TreeCell *cells, const CellData *cd, const int *leaves, int nleaves,
-                             float near_widths, float far_u, int pass, int *far_cnt, int *near_cnt, const int *far_off,
-                             const int *near_off, int *far_list, int2 *near_runs, int *err) {
-  const int li = blockIdx.x * blockDim.x + threadIdx.x;
-  if (li >= nleaves) return;
-  const int T = leaves[li];
-  const TreeCell tc = cells[T];
-  const float tx = cd[T].v[0], ty = cd[T].v[1], tz = cd[T].v[2], tR = cd[T].v[33], tH = cd[T].v[39];
-  int stack[kListStack];
-  int sp = 0;
-  stack[sp++] = 0;
-  int nf = 0, nn = 0, run_s = -1, run_e = -1;
-  const int fo = pass ? far_off[li] : 0, no = pass ? near_off[li] : 0;
-  while (sp > 0) {
-    const int ci = stack[--sp];
-    const TreeCell c = cells[ci];
-    const bool contains = c.start <= tc.start && tc.end <= c.end;
-    const float dx = cd[ci].v[0] - tx, dy = cd[ci].v[1] - ty, dz = cd[ci].v[2] - tz;
-    const float d = sqrtf(dx * dx + dy * dy + dz * dz) - tR;
-    // far: beyond near_widths cube widths, and every pair of the two cells at
-    // u = rho^2 / sigma_ij^2 >= far_u, so that the Gaussian regularisation
-    // the singular-kernel expansion leaves out stays small
-    const float gap = d - cd[ci].v[33];
-    if (!contains && d >= near_widths * cd[ci].v[34] && gap > 0.f &&
-        gap * gap >= far_u * (tH + cd[ci].v[39])) {
-      if (pass) far_list[fo + nf] = ci;
-      ++nf;
-    } else if (c.nchild == 0) {
-      if (c.start == run_e) {
-        run_e = c.end;
+// Packed index of a symmetric pair (b <= c) and triple.
+__device__ __forceinline__ int sym2(int b, int c) {
+  if (b > c) { const int t = b; b = c; c = t; }
+  return b == 0 ? c : b == 1 ? 2 + c : 5;
+}
+
+// The split cells of [f0, f1) from their children, one warp per cell: with
+// s = c_child - c and y = y_child + s,
+//   M += A s;  Q_bc += M_b s_c + M_c s_b + A s_b s_c;
+//   T_bcd += Q_bc s_d + Q_bd s_c + Q_cd s_b + M_b s_c s_d + M_c s_b s_d + M_d s_b s_c + A s_b s_c s_d
+// (one strength component at a time).  Lane e forms moments e and 32 + e.
+__global__ void __launch_bounds__(128) parent_moments_kernel(const TreeCell *cells, int f0, int f1, int nm,
+                                                             CellSums *sums) {
+  const int lane = threadIdx.x & 31;
+  const int ci = f0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (ci >= f1) return;
+  const TreeCell c = cells[ci];
+  if (c.nchild == 0) return;
+  double x[3] = {0, 0, 0}, a[3] = {0, 0, 0}, h = 0;
+  float H = 0.f;
+  for (int k = 0; k < c.nchild; ++k) {
+    const CellSums &ch = sums[c.first_child + k];
+    for (int m = 0; m < 3; ++m) { x[m] += ch.x[m]; a[m] += ch.a[m]; }
+    h += ch.h;
+    H = fmaxf(H, ch.hmax);
+  }
+  const double cnt = (double)(c.end - c.start);
+  for (int e = lane; e < nm; e += 32) {
+    // strength component and indices of moment e
+    int aa, b, cc = -1, d = -1;
+    if (e < 9) {
+      aa = e / 3; b = e % 3;
+    } else if (e < 27) {
+      aa = (e - 9) / 6;
+      const int k = (e - 9) % 6;
+      b = k < 3 ? 0 : k < 5 ? 1 : 2;
+      cc = k < 3 ? k : k < 5 ? k - 2 : 2;
+    } else {
+      aa = (e - 27) / 10;
+      const int k = (e - 27) % 10;
+      b = k < 6 ? 0 : k < 9 ? 1 : 2;
+      cc = k < 3 ? 0 : k < 5 ? 1 : k < 6 ? 2 : k < 8 ? 1 : 2;
+      d = k < 3 ? k : k < 5 ? k - 2 : k < 6 ? 2 : k < 8 ? k - 5 : 2;
+    }
+    double v = 0.0;
+    for (int k = 0; k < c.nchild; ++k) {
+      const int chi = c.first_child + k;
+      const CellSums &ch = sums[chi];
+      const double n = (double)(cells[chi].end - cells[chi].start);
+      const double sb = ch.x[b] / n - x[b] / cnt;
+      const double A = ch.a[aa];
+      if (cc < 0) {
+        v += ch.m[e] + A * sb;
       } else {
+        const double sc = ch.x[cc] / n - x[cc] / cnt;
+        const double Mb = ch.m[3 * aa + b], Mc = ch.m[3 * aa + cc];
+        if (d < 0) {
+          v += ch.m[e] + Mb * sc + Mc * sb + A * sb * sc;
+        } else {
+          const double sd = ch.x[d] / n - x[d] / cnt;
+          const double *Q = ch.m + 9 + 6 * aa;
+          v += ch.m[e] + Q[sym2(b, cc)] * sd + Q[sym2(b, d)] * sc + Q[sym2(cc, d)] * sb + Mb * sc * sd +
+               Mc * sb * sd + ch.m[3 * aa + d] * sb * sc + A * sb * sc * sd;
+        }
+      }
+    }
+    sums[ci].m[e] = v;
+  }
+  if (lane == 0) {
+    CellSums &o = sums[ci];
+    for (int m = 0; m < 3; ++m) { o.x[m] = x[m]; o.a[m] = a[m]; }
+    o.h = h;
+    o.hmax = H;
+    o.spread = 0u;
+  }
+}
+
+// Spread radii of the split cells: one warp per leaf takes its particles'
+// largest distance from every ancestor's centroid.
+__global__ void __launch_bounds__(128) spread_kernel(const TreeCell *cells, const int *leaves, int nleaves,
+                                                     const float4 *Ps, CellSums *sums) {
+  const int lane = threadIdx.x & 31;
+  const int li = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (li >= nleaves) return;
+  const TreeCell l = cells[leaves[li]];
+  for (int ci = l.parent; ci >= 0; ci = cells[ci].parent) {
+    const double cnt = (double)(cells[ci].end - cells[ci].start);
+    const double cx = sums[ci].x[0] / cnt, cy = sums[ci].x[1] / cnt, cz = sums[ci].x[2] / cnt;
+    float R = 0.f;
+    for (int i = l.start + lane; i < l.end; i += 32) {
+      const float4 p = Ps[i];
+      const double y[3] = {p.x - cx, p.y - cy, p.z - cz};
+      R = fmaxf(R, (float)sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]));
+    }
+    for (int o = 16; o > 0; o >>= 1) R = fmaxf(R, __shfl_xor_sync(0xffffffffu, R, o));
+    // non-negative floats order as their bits
+    if (lane == 0) atomicMax(&sums[ci].spread, __float_as_uint(R));
+  }
+}
+
+__global__ void cell_data_kernel(const TreeCell *cells, int ncells, int nm, const CellSums *sums, const float *geo,
+                                 CellData *out, TreeNode *nodes) {
+  const int ci = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ci >= ncells) return;
+  const TreeCell c = cells[ci];
+  const CellSums &s = sums[ci];
+  const double cnt = (double)(c.end - c.start);
+  CellData &d = out[ci];
+  TreeNode n;
+  for (int m = 0; m < 3; ++m) {
+    d.v[m] = n.c[m] = (float)(s.x[m] / cnt);
+    d.v[3 + m] = (float)s.a[m];
+  }
+  for (int k = 0; k < 27; ++k) d.v[6 + k] = (float)s.m[k];
+  d.v[33] = n.R = __uint_as_float(s.spread);
+  const float w = geo[3] / (float)(1u << c.level);
+  d.v[34] = n.w = w;
+  const unsigned long long pre = c.prefix;
+  const unsigned ix = compact21(pre), iy = compact21(pre >> 1), iz = compact21(pre >> 2);
+  d.v[35] = geo[0] + (ix + 0.5f) * w;
+  d.v[36] = geo[1] + (iy + 0.5f) * w;
+  d.v[37] = geo[2] + (iz + 0.5f) * w;
+  d.v[38] = (float)(s.h / cnt);
+  d.v[39] = n.H = s.hmax;
+  if (nm > kMoments2)
+    for (int k = 0; k < 30; ++k) d.v[40 + k] = (float)s.m[27 + k];
+  d.v[70] = 0.f;
+  d.v[71] = 0.f;
+  n.start = c.start; n.end = c.end; n.first_child = c.first_child; n.nchild = c.nchild;
+  n.pad[0] = n.pad[1] = 0;
+  nodes[ci] = n;
+}
+
+// Interaction lists of every leaf, one warp per leaf.  pass 0 counts, pass 1
+// writes at the offsets of an exclusive scan of the counts.  A cell that is not
+// far is opened by testing its children side by side (one dependent load per
+// opened cell instead of one per visited cell); the far ones go to the list at
+// once, the others to the warp's stack, first child on top, so that near leaves
+// come up in sorted order.  Near leaves are emitted as runs of the sorted
+// particle order: consecutive near leaves whose ranges touch are merged (children
+// are in octant order, which is sorted order, so runs are long).  The stack is
+// bounded (kListStack); overflow sets *err, and the caller treats a non-zero
+// *err as a failed build.
+constexpr int kListWarps = 4;
+
+__global__ void __launch_bounds__(32 * kListWarps) lists_kernel(const TreeNode *nodes, const int *leaves, int nleaves,
+                                                                float near_widths, float far_u, int pass, int *far_cnt,
+                                                                int *near_cnt, const int *far_off, const int *near_off,
+                                                                int *far_list, int2 *near_runs, int *err) {
+  // entries: (first child, number of children), or of a near leaf (start, -end)
+  __shared__ int2 stacks[kListWarps][kListStack];
+  const int lane = threadIdx.x & 31;
+  const int li = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (li >= nleaves) return;
+  int2 *stack = stacks[threadIdx.x >> 5];
+  const TreeNode t = nodes[leaves[li]];
+  int sp = 0, nf = 0, nn = 0, run_s = -1, run_e = -1;
+  const int fo = pass ? far_off[li] : 0, no = pass ? near_off[li] : 0;
+  const TreeNode root = nodes[0];  // holds every leaf: never far
+  if (lane == 0) stack[0] = root.nchild ? make_int2(root.first_child, root.nchild) : make_int2(root.start, -root.end);
+  sp = 1;
+  __syncwarp();
+  while (sp > 0) {
+    const int2 e = stack[--sp];
+    __syncwarp();
+    if (e.y < 0) {  // a near leaf
+      if (e.x != run_e) {
         if (run_s >= 0) {
-          if (pass) near_runs[no + nn] = make_int2(run_s, run_e);
+          if (pass && lane == 0) near_runs[no + nn] = make_int2(run_s, run_e);
           ++nn;
         }
-        run_s = c.start;
-        run_e = c.end;
+        run_s = e.x;
       }
-    } else {
-      if (sp + c.nchild > kListStack) {
-        atomicExch(err, 1);
-        break;
-      }
-      // push in reverse so the children are visited in octant (sorted) order
-      for (int k = c.nchild - 1; k >= 0; --k) stack[sp++] = c.first_child + k;
+      run_e = -e.y;
+      continue;
     }
+    TreeNode c;
+    bool far = false;
+    const int ci = e.x + lane;
+    if (lane < e.y) {
+      c = nodes[ci];
+      const bool contains = c.start <= t.start && t.end <= c.end;
+      const float dx = c.c[0] - t.c[0], dy = c.c[1] - t.c[1], dz = c.c[2] - t.c[2];
+      const float d = sqrtf(dx * dx + dy * dy + dz * dz) - t.R;
+      // far: beyond near_widths cube widths, and every pair of the two cells at
+      // u = rho^2 / sigma_ij^2 >= far_u, so that the Gaussian regularisation
+      // the singular-kernel expansion leaves out stays small
+      const float gap = d - c.R;
+      far = !contains && d >= near_widths * c.w && gap > 0.f && gap * gap >= far_u * (t.H + c.H);
+    }
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned fm = __ballot_sync(0xffffffffu, far);
+    const unsigned nm = __ballot_sync(0xffffffffu, lane < e.y && !far);
+    if (far && pass) far_list[fo + nf + __popc(fm & below)] = ci;
+    nf += __popc(fm);
+    if (sp + __popc(nm) > kListStack) {
+      if (lane == 0) atomicExch(err, 1);
+      break;
+    }
+    if (lane < e.y && !far)
+      stack[sp + __popc(nm) - 1 - __popc(nm & below)] =
+          c.nchild ? make_int2(c.first_child, c.nchild) : make_int2(c.start, -c.end);
+    sp += __popc(nm);
+    __syncwarp();
   }
   if (run_s >= 0) {
-    if (pass) near_runs[no + nn] = make_int2(run_s, run_e);
+    if (pass && lane == 0) near_runs[no + nn] = make_int2(run_s, run_e);
     ++nn;
   }
-  if (!pass) {
+  if (!pass && lane == 0) {
     far_cnt[li] = nf;
     near_cnt[li] = nn;
   }

@@ -200,3 +200,26 @@ def test_transfers_in_pieces(gpu, n, prec):
         one.solve()
         for got, ref in zip((r, d), one.rates(ids[0])):
             assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("order", [2, 3])
+@pytest.mark.parametrize("n,leaf", [(1, 256), (2, 1), (300, 1), (300, 16), (5000, 7), (5000, 256), (20011, 33)])
+def test_surrogate_tree_sizes(gpu, n, leaf, order):
+    """Trees of one leaf up to leaves of single particles.  A far cell's particles lie within 0.87 widths of its centroid,
+    which is at least five widths off: the quadrupole drops (0.17)^3 = 5e-3 of a far cell's part, which is less than
+    half of the field."""
+    w = ring(n, sigma=0.02)
+    if n > 100:
+        w.pos[5] = w.pos[6]  # two particles that no cube separates
+    c, ids = context([w], capi.FP32C)
+    c.solve()
+    ref = c.rates(ids[0])
+    c.surrogate_enable(0, leaf_size=leaf, order=order, check_targets=0)
+    c.solve()
+    t = c.surrogate_tree()
+    cells = t["cells"][t["leaves"]]
+    order_ = np.argsort(cells[:, 0])
+    assert cells[order_][0, 0] == 0 and cells[order_][-1, 1] == n
+    assert np.array_equal(cells[order_][1:, 0], cells[order_][:-1, 1])
+    for got, want in zip(c.rates(ids[0]), ref):
+        assert np.abs(got - want).max() <= 2.5e-3 * np.abs(want).max()
