@@ -269,6 +269,7 @@ __device__ __forceinline__ PairTerms<double> pair_terms_ho(double r2, double s2)
 // Compile-time flags for generic lambdas.
 struct TrueType { static constexpr bool value = true; };
 struct FalseType { static constexpr bool value = false; };
+template <int N> struct IntType { static constexpr int value = N; };
 
 // Kernel selection (PGPU_KERNEL_GAUSSIAN = 0, PGPU_KERNEL_HIGHORDER = 1).
 constexpr int kGaussian = 0;

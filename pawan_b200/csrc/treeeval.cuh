@@ -195,6 +195,91 @@ __device__ __forceinline__ void far_expand(const float *v, const float *x, const
   }
 }
 
+// The expansion to order ORD <= 2 of two far cells at once (lane .x the even
+// cell, .y the odd one), added to u and s.  The terms are those of far_expand,
+// arranged by strength component: with Phi_a = sum alpha_a phi,
+//   u = -curl-like  -eps_kab d_b Phi_a,   s_i = d_i (alpha_t . u) = sum_a (H^a V_a)_i,
+// H^a the Hessian of Phi_a and V_a the (negated) rows of alpha_t's cross matrix,
+// two components each.  Per a, with m = M_a, Q = Q_a:
+//   grad = c2 r + ir^3 m + 3 ir^5 Q r
+//   H V  = r (c1 r.V + w.V) + w (r.V) + c2 V + 3 ir^5 Q V
+//   c2 = -A ir^3 - 3 ir^5 m.r - 7.5 ir^7 r.Q r + 1.5 ir^5 tr Q
+//   c1 = 3 A ir^5 + 15 ir^7 m.r + 52.5 ir^9 r.Q r - 7.5 ir^7 tr Q
+//   w  = -3 ir^5 m - 15 ir^7 Q r
+// About 190 packed operations at order 2; far_expand forms alpha_t x A, M and Q
+// per target, about 310 (1M coaxial rings, 1250 far cells per target:
+// evaluation 97 ms instead of 105 ms).
+template <int ORD>
+__device__ __forceinline__ void far_expand2(const float2 *v, const float2 *x, const float2 *at, const float2 *nat,
+                                            float2 *u, float2 *s) {
+  const float2 M1 = dup2(-1.f);
+  const float2 r[3] = {__ffma2_rn(v[0], M1, x[0]), __ffma2_rn(v[1], M1, x[1]), __ffma2_rn(v[2], M1, x[2])};
+  const float2 r2 = __ffma2_rn(r[2], r[2], __ffma2_rn(r[1], r[1], __fmul2_rn(r[0], r[0])));
+  const float2 ir = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
+  const float2 ir2 = __fmul2_rn(ir, ir), ir3 = __fmul2_rn(ir2, ir);
+  const float2 nir3 = __fmul2_rn(ir3, M1);
+  const float2 k3 = __fmul2_rn(__fmul2_rn(ir3, ir2), dup2(3.f));  // 3 ir^5
+  const float2 nk3 = __fmul2_rn(k3, M1);
+  const float2 k15 = __fmul2_rn(__fmul2_rn(k3, ir2), dup2(5.f));  // 15 ir^7
+  const float2 nk15 = __fmul2_rn(k15, M1), nk75 = __fmul2_rn(k15, dup2(-0.5f));
+  const float2 k525 = __fmul2_rn(__fmul2_rn(k15, ir2), dup2(3.5f));  // 52.5 ir^9
+  const float2 hk3 = __fmul2_rn(k3, dup2(0.5f));
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int p = (a + 1) % 3, q = (a + 2) % 3;
+    // -V_a: component p is -alpha_t[q], component q is +alpha_t[p]
+    const float2 Vp = nat[q], Vq = at[p];
+    float2 c2 = __fmul2_rn(v[3 + a], nir3), c1 = __fmul2_rn(v[3 + a], k3);
+    float2 w[3], Qr[3];
+    const float2 *m = v + 6 + 3 * a, *Q = v + 15 + 6 * a;  // Q packed (00,01,02,11,12,22)
+    if constexpr (ORD >= 1) {
+      const float2 mr = __ffma2_rn(m[2], r[2], __ffma2_rn(m[1], r[1], __fmul2_rn(m[0], r[0])));
+      c2 = __ffma2_rn(nk3, mr, c2);
+      c1 = __ffma2_rn(k15, mr, c1);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) w[i] = __fmul2_rn(nk3, m[i]);
+    }
+    if constexpr (ORD >= 2) {
+      Qr[0] = __ffma2_rn(Q[2], r[2], __ffma2_rn(Q[1], r[1], __fmul2_rn(Q[0], r[0])));
+      Qr[1] = __ffma2_rn(Q[4], r[2], __ffma2_rn(Q[3], r[1], __fmul2_rn(Q[1], r[0])));
+      Qr[2] = __ffma2_rn(Q[5], r[2], __ffma2_rn(Q[4], r[1], __fmul2_rn(Q[2], r[0])));
+      const float2 rQr = __ffma2_rn(Qr[2], r[2], __ffma2_rn(Qr[1], r[1], __fmul2_rn(Qr[0], r[0])));
+      const float2 tr = __fadd2_rn(__fadd2_rn(Q[0], Q[3]), Q[5]);
+      c2 = __ffma2_rn(hk3, tr, __ffma2_rn(nk75, rQr, c2));
+      c1 = __ffma2_rn(nk75, tr, __ffma2_rn(k525, rQr, c1));
+#pragma unroll
+      for (int i = 0; i < 3; ++i) w[i] = __ffma2_rn(nk15, Qr[i], w[i]);
+    }
+    // gradient components p and q: u[q] -= g_p, u[p] += g_q
+    float2 gp = __fmul2_rn(c2, r[p]), gq = __fmul2_rn(c2, r[q]);
+    if constexpr (ORD >= 1) {
+      gp = __ffma2_rn(ir3, m[p], gp);
+      gq = __ffma2_rn(ir3, m[q], gq);
+    }
+    if constexpr (ORD >= 2) {
+      gp = __ffma2_rn(k3, Qr[p], gp);
+      gq = __ffma2_rn(k3, Qr[q], gq);
+    }
+    u[q] = __ffma2_rn(gp, M1, u[q]);
+    u[p] = __fadd2_rn(u[p], gq);
+    const float2 rv = __ffma2_rn(r[q], Vq, __fmul2_rn(r[p], Vp));
+    float2 t = __fmul2_rn(c1, rv);
+    if constexpr (ORD >= 1) t = __ffma2_rn(w[q], Vq, __ffma2_rn(w[p], Vp, t));
+    s[p] = __ffma2_rn(c2, Vp, s[p]);
+    s[q] = __ffma2_rn(c2, Vq, s[q]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      s[i] = __ffma2_rn(r[i], t, s[i]);
+      if constexpr (ORD >= 1) s[i] = __ffma2_rn(w[i], rv, s[i]);
+      if constexpr (ORD >= 2) {
+        constexpr int S[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+        const float2 qv = __ffma2_rn(Q[S[i][q]], Vq, __fmul2_rn(Q[S[i][p]], Vp));
+        s[i] = __ffma2_rn(k3, qv, s[i]);
+      }
+    }
+  }
+}
+
 // Input features of the far-field correction network for one (target, far
 // cell) pair, and the scales of its outputs.  With r = x_t - c (c the cell's
 // particle centroid, the expansion origin), rho = |r|, rh = r/rho, w the cube
@@ -288,9 +373,11 @@ constexpr int kWarpsPerCta = 4;
 
 // Per-warp shared buffers (all carved from dynamic shared memory, after the
 // packed network when the correction is on).
+constexpr int kPairFloats = 33;  // centroid, A, M, Q: what the order-2 expansion reads
 struct WarpSmem {
   union {
     float sc[kWarpCells][kCellFloats];
+    float2 sc2[kWarpCells / 2][kPairFloats];  // cell pairs, interleaved
     SliceStage<kWarpTile / 32, false> near;
   };
 };
@@ -339,7 +426,39 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
     const float hst = pt.w, vt = qt.w;
     float vh[3] = {0, 0, 0}, vl[3] = {0, 0, 0}, dh[3] = {0, 0, 0}, dl[3] = {0, 0, 0};
     const int fo = a.far_off[li], fn = a.far_cnt[li];
-    for (int c0 = 0; c0 < fn; c0 += kWarpCells) {
+    // far cells, orders up to 2 without the network: two cells per packed
+    // instruction, one compensated addition per kWarpCells cells
+    auto far2 = [&](auto ord) {
+      constexpr int ORD = decltype(ord)::value;
+      const float2 x2[3] = {dup2(xt[0]), dup2(xt[1]), dup2(xt[2])};
+      const float2 at2[3] = {dup2(at[0]), dup2(at[1]), dup2(at[2])};
+      const float2 nat2[3] = {dup2(-at[0]), dup2(-at[1]), dup2(-at[2])};
+      constexpr int nf = ORD == 0 ? 6 : ORD == 1 ? 15 : kPairFloats;
+      for (int c0 = 0; c0 < fn; c0 += kWarpCells) {
+        const int cn = min(kWarpCells, fn - c0), cp = (cn + 1) & ~1;
+        __syncwarp();
+        for (int k = lane; k < cp * nf; k += 32) {
+          const int cc = k / nf, e = k - cc * nf;
+          // an odd last cell pairs with itself without strength
+          const float val = a.cd[a.far_list[fo + c0 + min(cc, cn - 1)]].v[e];
+          reinterpret_cast<float *>(&ws.sc2[cc >> 1][e])[cc & 1] = cc < cn || e < 3 ? val : 0.f;
+        }
+        __syncwarp();
+        float2 u2[3] = {dup2(0.f), dup2(0.f), dup2(0.f)}, s2[3] = {dup2(0.f), dup2(0.f), dup2(0.f)};
+        for (int j = 0; j < cp / 2; ++j) far_expand2<ORD>(ws.sc2[j], x2, at2, nat2, u2, s2);
+        for (int m = 0; m < 3; ++m) {
+          two_sum_acc(vh[m], vl[m], u2[m].x + u2[m].y);
+          two_sum_acc(dh[m], dl[m], s2[m].x + s2[m].y);
+        }
+      }
+    };
+    const bool packed = !MLP && a.order <= 2;
+    if constexpr (!MLP) {
+      if (a.order == 2) far2(IntType<2>{});
+      else if (a.order == 1) far2(IntType<1>{});
+      else if (a.order == 0) far2(IntType<0>{});
+    }
+    for (int c0 = packed ? fn : 0; c0 < fn; c0 += kWarpCells) {
       const int cn = min(kWarpCells, fn - c0);
       __syncwarp();
       // the cell data the expansion reads: the third moments only at order 3
