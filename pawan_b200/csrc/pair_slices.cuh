@@ -114,15 +114,18 @@ __device__ __forceinline__ void stage_source(SliceStage<SL, SPLIT> &st, int k, f
   dn[4] = px * q.y - py * q.x;
 }
 
-// The Gaussian sums of one target over npr source pairs of a staged slice:
-// the far limit, or the closed form (its diffusion into sdv).
+// The Gaussian sums of one target over source pairs r0, r0 + step, ... (n of
+// them) of a staged slice: the far limit, or the closed form (its diffusion
+// into sdv).
 template <int SL, bool SPLIT>
-__device__ __forceinline__ void far_slice(const SliceStage<SL, SPLIT> &st, int npr, const float2 *X, const float2 *AT,
-                                          float xr0, float xr1, float xr2, float2 *sv, float2 *sd, float2 *sp) {
+__device__ __forceinline__ void far_slice(const SliceStage<SL, SPLIT> &st, int n, int r0, int step, const float2 *X,
+                                          const float2 *AT, float xr0, float xr1, float xr2, float2 *sv, float2 *sd,
+                                          float2 *sp) {
   float2 B3[3];
   far_b3(xr0, xr1, xr2, AT, B3);
 #pragma unroll 2
-  for (int r = 0; r < npr; ++r) {
+  for (int k = 0; k < n; ++k) {
+    const int r = r0 + k * step;
     const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1], na = st.N[2 * r],
                  nb = st.N[2 * r + 1];
     far_pair2(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y), make_float2(qa.x, qa.y),
@@ -131,12 +134,13 @@ __device__ __forceinline__ void far_slice(const SliceStage<SL, SPLIT> &st, int n
   }
 }
 template <bool SPLIT, bool CROSS, int SL>
-__device__ __forceinline__ void mid_slice(const SliceStage<SL, SPLIT> &st, int npr, const float2 *X, const float *xl,
-                                          const float *at, float hst, float vt, const MidSigma2 *uni, float2 *sv,
+__device__ __forceinline__ void mid_slice(const SliceStage<SL, SPLIT> &st, int n, int r0, int step, const float2 *X,
+                                          const float *xl, const float *at, float hst, float vt, const MidSigma2 *uni, float2 *sv,
                                           float2 *sd, float2 *sp, float *sdv, unsigned &nfull) {
   float2 sdv2[3] = {dup2(0.f), dup2(0.f), dup2(0.f)};
 #pragma unroll 2
-  for (int r = 0; r < npr; ++r) {
+  for (int k = 0; k < n; ++k) {
+    const int r = r0 + k * step;
     const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1];
     float2 lx = dup2(0.f), ly = lx, lz = lx;
     if constexpr (SPLIT) {
@@ -275,15 +279,15 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
           sd[m] = __fmul2_rn(sd[m], dup2(-3.f));
         }
       } else if (far) {
-        far_slice(st, npr, X, AT, pt.x - rx, pt.y - ry, pt.z - rz, sv, sd, sp);
+        far_slice(st, npr, 0, 1, X, AT, pt.x - rx, pt.y - ry, pt.z - rz, sv, sd, sp);
       } else if (warp_min(hmin) == sbox.hs && thmin == tb.hs) {
         // one sigma for all of the slice's pairs, as in every wake shed with
         // one radius: its factors leave the loop (an odd tail's padding
         // source carries no strength, so its sigma does not matter)
         const MidSigma2 g = mid_sigma2(dup2(tb.hs + sbox.hs));
-        mid_slice<SPLIT, true>(st, npr, X, xl, at, pt.w, qt.w, &g, sv, sd, sp, sdv, nfull);
+        mid_slice<SPLIT, true>(st, npr, 0, 1, X, xl, at, pt.w, qt.w, &g, sv, sd, sp, sdv, nfull);
       } else {
-        mid_slice<SPLIT, true>(st, npr, X, xl, at, pt.w, qt.w, nullptr, sv, sd, sp, sdv, nfull);
+        mid_slice<SPLIT, true>(st, npr, 0, 1, X, xl, at, pt.w, qt.w, nullptr, sv, sd, sp, sdv, nfull);
       }
       fold_group_f32(far, pt.x - rx, pt.y - ry, pt.z - rz, at, a.nu2, sv, sd, sp, sdv, vh, vl, dh, dl);
     }

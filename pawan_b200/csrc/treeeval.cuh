@@ -416,7 +416,14 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
     const int2 it = items[item];
     const int li = it.x;
     const TreeCell tc = a.cells[a.leaves[li]];
-    const int t0 = tc.start + it.y * 32 + lane;
+    // A slice of at most 16 targets (half of the leaves' last slices) gives
+    // each of them two lanes, h = 0 and 1, which take every other pair of the
+    // far cells and near sources and add their sums at the end (1M coaxial
+    // rings: 90 ms instead of 97 ms).
+    const int left = tc.end - (tc.start + it.y * 32);
+    const bool half = !MLP && a.order <= 2 && left <= 16;
+    const int h = half ? lane >> 4 : 0, step = half ? 2 : 1;
+    const int t0 = tc.start + it.y * 32 + (half ? lane & 15 : lane);
     const int t = min(t0, tc.end - 1);
     const int ti = a.idx[t];
     const bool mine = t0 < tc.end && ti >= a.own_lo && ti < a.own_hi;
@@ -435,17 +442,17 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
       const float2 nat2[3] = {dup2(-at[0]), dup2(-at[1]), dup2(-at[2])};
       constexpr int nf = ORD == 0 ? 6 : ORD == 1 ? 15 : kPairFloats;
       for (int c0 = 0; c0 < fn; c0 += kWarpCells) {
-        const int cn = min(kWarpCells, fn - c0), cp = (cn + 1) & ~1;
+        const int cn = min(kWarpCells, fn - c0), cp = (cn + 2 * step - 1) & ~(2 * step - 1);
         __syncwarp();
         for (int k = lane; k < cp * nf; k += 32) {
           const int cc = k / nf, e = k - cc * nf;
-          // an odd last cell pairs with itself without strength
+          // the last pairs are filled up with the last cell, without strength
           const float val = a.cd[a.far_list[fo + c0 + min(cc, cn - 1)]].v[e];
           reinterpret_cast<float *>(&ws.sc2[cc >> 1][e])[cc & 1] = cc < cn || e < 3 ? val : 0.f;
         }
         __syncwarp();
         float2 u2[3] = {dup2(0.f), dup2(0.f), dup2(0.f)}, s2[3] = {dup2(0.f), dup2(0.f), dup2(0.f)};
-        for (int j = 0; j < cp / 2; ++j) far_expand2<ORD>(ws.sc2[j], x2, at2, nat2, u2, s2);
+        for (int j = h; j < cp / 2; j += step) far_expand2<ORD>(ws.sc2[j], x2, at2, nat2, u2, s2);
         for (int m = 0; m < 3; ++m) {
           two_sum_acc(vh[m], vl[m], u2[m].x + u2[m].y);
           two_sum_acc(dh[m], dl[m], s2[m].x + s2[m].y);
@@ -538,27 +545,32 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
         __syncwarp();
         // source pairs; an odd tail pairs with a padding source (zero strength, far away)
         const int npr = (min(kWarpTile, run.y - sb) + 1) >> 1;
+        const int n = half ? (npr + 1) >> 1 : npr;  // an odd pair pairs with padding sources (every slot is staged)
         float2 sv[3], sd[3], sp[3];
         float sdv[3] = {0.f, 0.f, 0.f};
 #pragma unroll
         for (int m = 0; m < 3; ++m) sv[m] = sd[m] = sp[m] = dup2(0.f);
         if (far_tile) {
-          far_slice(st, npr, X2, AT3, xt[0] - rx, xt[1] - ry, xt[2] - rz, sv, sd, sp);
+          far_slice(st, n, h, step, X2, AT3, xt[0] - rx, xt[1] - ry, xt[2] - rz, sv, sd, sp);
         } else if (warp_min(hmin) == sbx.hs && thmin == tb.hs) {
           const MidSigma2 g = mid_sigma2(dup2(tb.hs + sbx.hs));
-          mid_slice<false, false>(st, npr, X2, xt, at, hst, vt, &g, sv, sd, sp, sdv, nfull);
+          mid_slice<false, false>(st, n, h, step, X2, xt, at, hst, vt, &g, sv, sd, sp, sdv, nfull);
         } else {
-          mid_slice<false, false>(st, npr, X2, xt, at, hst, vt, nullptr, sv, sd, sp, sdv, nfull);
+          mid_slice<false, false>(st, n, h, step, X2, xt, at, hst, vt, nullptr, sv, sd, sp, sdv, nfull);
         }
         fold_group_f32<false>(far_tile, xt[0] - rx, xt[1] - ry, xt[2] - rz, at, a.nu2, sv, sd, sp, sdv, vh, vl, dh, dl);
       }
     }
-    if (mine) {
+    double out[6];
+    for (int m = 0; m < 3; ++m) {
+      out[m] = (double)vh[m] + (double)vl[m];
+      out[3 + m] = (double)dh[m] + (double)dl[m];
+    }
+    if (half)
+      for (int m = 0; m < 6; ++m) out[m] += __shfl_xor_sync(0xffffffffu, out[m], 16);
+    if (mine && h == 0) {
       double *o = a.partial + a.off + ti;
-      for (int m = 0; m < 3; ++m) {
-        o[m * a.cap] = ((double)vh[m] + (double)vl[m]) * kInv4Pi;
-        o[(3 + m) * a.cap] = ((double)dh[m] + (double)dl[m]) * kInv4Pi;
-      }
+      for (int m = 0; m < 6; ++m) o[m * a.cap] = out[m] * kInv4Pi;
     }
   }
 }
