@@ -197,9 +197,10 @@ __device__ __forceinline__ bool all_far(const WarpBox &t, const WarpBox &s, floa
 // (TILE == BLOCK: each thread stages one record), CG sources per compensation
 // group (plain FP32 partial sums over CG sources, then an error-free two-sum
 // into the per-target (hi, lo) accumulators).
-// This generic body serves the FP64 mode of the Gaussian kernel and both modes
-// of the high-order kernel (KER = kHighOrder: every pair takes pair_terms_ho,
-// which has no far regime to skip); the FP32 Gaussian mode uses
+// This generic body serves the asked-for and tuned shapes of the FP64 mode and
+// of both modes of the high-order kernel (KER = kHighOrder: every pair takes
+// pair_terms_ho, which has no far regime to skip), whose default is the row list
+// (pair_slices.cuh, pair_slices64.cuh); the FP32 Gaussian mode uses
 // pair_body_f32 (pair_f32.cuh), the same decomposition with packed FP32.
 template <typename T, int BLOCK, int TPT, int CG, int KER>
 __device__ __forceinline__ void pair_body_generic(const PairArgs<T> &a) {
@@ -509,7 +510,7 @@ namespace pgpu {
 // FP64 shapes with one target per thread are held to 128 registers (a few
 // bytes of spill), which fits two 256-thread CTAs per SM instead of one: per
 // evaluation of the 1M ring 3196 ms instead of 3632 ms (Gaussian) and
-// 4505 ms instead of 5743 ms (high-order).  With more targets per thread the
+// 4505 ms instead of 5743 ms (high-order), both with CUDA's erf and roots.  With more targets per thread the
 // same cap spills hundreds of bytes, so those shapes keep the registers they
 // need.
 template <typename T, int BLOCK, int TPT, int KER>
