@@ -733,9 +733,10 @@ __global__ void __launch_bounds__(kIoRows) upload_kernel(const double *stage, in
   }
 }
 
-// SoA [6][cap] (from slot offset `off`) -> row-major (n, 3) x 2.
+// SoA [3 parts][cap] (from slot offset `off`) -> row-major (n, 3) x parts, parts
+// 1 or 2.
 static __global__ void __launch_bounds__(kIoRows) gather_kernel(const double *src, int64_t n, int64_t off, int64_t cap,
-                                                                double *stage) {
+                                                                int parts, double *stage) {
   __shared__ double s[6 * kIoRows];
   for (int64_t b = blockIdx.x * (int64_t)kIoRows; b < n; b += (int64_t)gridDim.x * kIoRows) {
     const int rows = (int)min((int64_t)kIoRows, n - b);
@@ -743,13 +744,13 @@ static __global__ void __launch_bounds__(kIoRows) gather_kernel(const double *sr
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
         s[3 * threadIdx.x + m] = src[m * cap + off + b + threadIdx.x];
-        s[3 * kIoRows + 3 * threadIdx.x + m] = src[(3 + m) * cap + off + b + threadIdx.x];
+        if (parts > 1) s[3 * kIoRows + 3 * threadIdx.x + m] = src[(3 + m) * cap + off + b + threadIdx.x];
       }
     }
     __syncthreads();
     for (int t = threadIdx.x; t < 3 * rows; t += kIoRows) {
       stage[3 * b + t] = s[t];
-      stage[3 * n + 3 * b + t] = s[3 * kIoRows + t];
+      if (parts > 1) stage[3 * n + 3 * b + t] = s[3 * kIoRows + t];
     }
     __syncthreads();
   }
@@ -1062,15 +1063,13 @@ __global__ void __launch_bounds__(32 * kSliceWarps) field_kernel(FieldArgs a) {
   }
 }
 
-// field[m][i] = sum over chunks of partial[c][m][i], m = 0..2; components 3..5
-// of field are zero (the [6][cap] layout the row gather expects).
+// field[m][i] = sum over chunks of partial[c][m][i], m = 0..2.
 static __global__ void field_reduce_kernel(const double *partial, int nch, int64_t cap, double *field) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < cap; i += (int64_t)gridDim.x * blockDim.x) {
     for (int m = 0; m < 3; ++m) {
       double v = 0.0;
       for (int c = 0; c < nch; ++c) v += partial[((int64_t)c * 6 + m) * cap + i];
       field[m * cap + i] = v;
-      field[(3 + m) * cap + i] = 0.0;
     }
   }
 }

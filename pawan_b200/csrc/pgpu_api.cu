@@ -117,7 +117,7 @@ struct pgpu_ctx {
   void *P = nullptr, *Q = nullptr;
   int64_t *d_sysoff = nullptr, *d_sysn = nullptr, *d_syst = nullptr;
   PlanEntry *d_plan = nullptr, *d_plan_diag = nullptr, *d_plan_field = nullptr;
-  double *d_field = nullptr;  // [6][cap] vorticity field (components 0..2), allocated by pgpu_influence
+  double *d_field = nullptr;  // [3][cap] vorticity field, allocated by pgpu_influence
   unsigned long long *d_merge = nullptr;  // merge candidate keys (pgpu_merge): d_merge_cap, a counter, d_merge_cap sorted
   int64_t d_merge_cap = 0;
   void *d_merge_tmp = nullptr;  // radix-sort space of the candidate keys
@@ -990,11 +990,13 @@ int pgpu_get_num_particles(pgpu_ctx *c, int32_t wake, int64_t *n) {
   return PGPU_OK;
 }
 
+// Components 0..2 of the wake's rows to a and, unless b is null, 3..5 to b.
 static int download_rows(pgpu_ctx *c, const double *src, const WakeRec &W, double *a, double *b) {
   if (W.n == 0) return PGPU_OK;
+  const int parts = b ? 2 : 1;
   auto launch = [&](int64_t at, int64_t k, double *dst) -> int {
     const int grid = (int)std::min<int64_t>(ceil_div(k, kIoRows), 8LL * c->sms);
-    gather_kernel<<<grid, kIoRows, 0, c->st>>>(src, k, W.off + at, c->cap, dst);
+    gather_kernel<<<grid, kIoRows, 0, c->st>>>(src, k, W.off + at, c->cap, parts, dst);
     CK(cudaGetLastError());
     c->launches++;
     return PGPU_OK;
@@ -1002,7 +1004,7 @@ static int download_rows(pgpu_ctx *c, const double *src, const WakeRec &W, doubl
   if (W.n > kIoRowsMax) {
     if (int r = launch(0, W.n, c->stage)) return r;
     CK(cudaMemcpyAsync(a, c->stage, 3 * W.n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(b, c->stage + 3 * W.n, 3 * W.n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    if (b) CK(cudaMemcpyAsync(b, c->stage + 3 * W.n, 3 * W.n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     return PGPU_OK;
   }
@@ -1013,11 +1015,11 @@ static int download_rows(pgpu_ctx *c, const double *src, const WakeRec &W, doubl
     for (int q = 0; q < 2; ++q) {
       const int64_t lo = at + q * piece, k = std::min(piece, W.n - lo);
       if (k <= 0) break;
-      h[q] = reinterpret_cast<double *>(io_take(c, 6 * k * sizeof(double)));
+      h[q] = reinterpret_cast<double *>(io_take(c, 3 * parts * k * sizeof(double)));
       if (!h[q]) return fail(c, PGPU_ECUDA, "waiting for the pinned transfer buffer failed");
       if (q == 1 && h[1] <= h[0]) {  // the ring started over and the first piece has landed: take it out first
         memcpy(a + 3 * at, h[0], 3 * piece * sizeof(double));
-        memcpy(b + 3 * at, h[0] + 3 * piece, 3 * piece * sizeof(double));
+        if (b) memcpy(b + 3 * at, h[0] + 3 * piece, 3 * piece * sizeof(double));
         h[0] = nullptr;
       }
       if (int r = launch(lo, k, h[q])) return r;
@@ -1027,7 +1029,7 @@ static int download_rows(pgpu_ctx *c, const double *src, const WakeRec &W, doubl
       const int64_t lo = at + q * piece, k = std::min(piece, W.n - lo);
       if (!h[q]) continue;
       memcpy(a + 3 * lo, h[q], 3 * k * sizeof(double));
-      memcpy(b + 3 * lo, h[q] + 3 * k, 3 * k * sizeof(double));
+      if (b) memcpy(b + 3 * lo, h[q] + 3 * k, 3 * k * sizeof(double));
     }
     c->io_pos = 0;  // the stream is idle: nothing needs the ring any more
   }
@@ -1392,7 +1394,7 @@ int pgpu_influence(pgpu_ctx *c) {
   int r = check_contiguous(c);
   if (r) return r;
   if (!c->d_field) {
-    const cudaError_t e = cudaMalloc((void **)&c->d_field, 6 * (size_t)c->cap * sizeof(double));
+    const cudaError_t e = cudaMalloc((void **)&c->d_field, 3 * (size_t)c->cap * sizeof(double));
     if (e != cudaSuccess) {
       cudaGetLastError();
       c->d_field = nullptr;
@@ -1432,8 +1434,7 @@ int pgpu_get_vorticity_field(pgpu_ctx *c, int32_t wake, double *field) {
   if (!field) return fail(c, PGPU_EINVAL, "null output array");
   if (!c->d_field) return fail(c, PGPU_EINVAL, "no vorticity field was computed (pgpu_influence)");
   const WakeRec &W = c->wakes[wake];
-  std::vector<double> zeros(3 * (size_t)W.n);
-  return download_rows(c, c->d_field, W, field, zeros.data());
+  return download_rows(c, c->d_field, W, field, nullptr);
 }
 
 int pgpu_set_timing(pgpu_ctx *c, int on) {
@@ -1499,7 +1500,7 @@ int pgpu_snapshot_begin(pgpu_ctx *c, int32_t slot) {
     ns[w] = W.n;
     if (W.n > 0) {
       const int grid = (int)std::min<int64_t>(ceil_div(W.n, kIoRows), 8LL * c->sms);
-      gather_kernel<<<grid, kIoRows, 0, c->st>>>(c->x0, W.n, W.off, c->cap, c->d_snap[slot] + 6 * total);
+      gather_kernel<<<grid, kIoRows, 0, c->st>>>(c->x0, W.n, W.off, c->cap, 2, c->d_snap[slot] + 6 * total);
       CK(cudaGetLastError());
       c->launches++;
     }
