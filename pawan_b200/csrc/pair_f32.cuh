@@ -85,11 +85,18 @@ __device__ __forceinline__ void far_pair2(float2 px, float2 py, float2 pz, float
 // Two pairs at once of the high-order kernel (pair_terms_ho): with R =
 // rho^2 + sigma^2, q' = (R + 1.5 sigma^2) R^-2.5, F'/-3 = (R + 2.5 sigma^2)
 // R^-3.5 and zd'/52.5 = sigma^4 R^-4.5.  zx, zy: lanes at rho = 0, whose terms
-// are all zero.
+// are all zero.  uni: the powers of sigma where one sigma serves every pair, or
+// null (two operations less, and two sums of two operands instead of three).
 struct HoTerms2 {
   float2 q, F3, zd;
 };
-__device__ __forceinline__ HoTerms2 ho_terms2(float2 R, float2 s2, bool zx, bool zy) {
+struct HoSigma2 {
+  float2 s2, s15, s25, s4;  // sigma^2, 1.5 sigma^2, 2.5 sigma^2, sigma^4
+};
+__device__ __forceinline__ HoSigma2 ho_sigma2(float2 s2) {
+  return {s2, __fmul2_rn(s2, dup2(1.5f)), __fmul2_rn(s2, dup2(2.5f)), __fmul2_rn(s2, s2)};
+}
+__device__ __forceinline__ HoTerms2 ho_terms2(float2 R, float2 s2, bool zx, bool zy, const HoSigma2 *uni) {
   float2 iR = make_float2(fast_rsqrt(R.x), fast_rsqrt(R.y));
   const float2 h = __fmul2_rn(__fmul2_rn(R, dup2(-0.5f)), iR);
   iR = __fmul2_rn(iR, __ffma2_rn(h, iR, dup2(1.5f)));  // one Newton step, as rsqrt_nr
@@ -99,9 +106,9 @@ __device__ __forceinline__ HoTerms2 ho_terms2(float2 R, float2 s2, bool zx, bool
   const float2 iR5 = __fmul2_rn(__fmul2_rn(iR2, iR2), iR);
   const float2 iR7 = __fmul2_rn(iR5, iR2);
   HoTerms2 o;
-  o.q = __fmul2_rn(__ffma2_rn(s2, dup2(1.5f), R), iR5);
-  o.F3 = __fmul2_rn(__ffma2_rn(s2, dup2(2.5f), R), iR7);
-  o.zd = __fmul2_rn(__fmul2_rn(s2, s2), __fmul2_rn(iR7, iR2));
+  o.q = __fmul2_rn(uni ? __fadd2_rn(R, uni->s15) : __ffma2_rn(s2, dup2(1.5f), R), iR5);
+  o.F3 = __fmul2_rn(uni ? __fadd2_rn(R, uni->s25) : __ffma2_rn(s2, dup2(2.5f), R), iR7);
+  o.zd = __fmul2_rn(uni ? uni->s4 : __fmul2_rn(s2, s2), __fmul2_rn(iR7, iR2));
   return o;
 }
 
@@ -112,17 +119,17 @@ __device__ __forceinline__ HoTerms2 ho_terms2(float2 R, float2 s2, bool zx, bool
 // q alpha_s, sv q n, sd (F/-3) dot d, sz zd alpha_s, sw zd v_s.
 __device__ __forceinline__ void ho_far_pair2(float2 px, float2 py, float2 pz, float2 ph, float2 ax, float2 ay,
                                              float2 az, float2 av, float2 nx, float2 ny, float2 nz, const float2 *X,
-                                             float hst, const float2 *AT, const float2 *B, float2 *sv, float2 *sd,
-                                             float2 *sp, float2 *sz, float2 &sw) {
+                                             float hst, const HoSigma2 *uni, const float2 *AT, const float2 *B,
+                                             float2 *sv, float2 *sd, float2 *sp, float2 *sz, float2 &sw) {
   const float2 M1 = make_float2(-1.f, -1.f);
   const float2 dx = __ffma2_rn(px, M1, X[0]);
   const float2 dy = __ffma2_rn(py, M1, X[1]);
   const float2 dz = __ffma2_rn(pz, M1, X[2]);
-  const float2 s2 = __fadd2_rn(dup2(hst), ph);
+  const float2 s2 = uni ? uni->s2 : __fadd2_rn(dup2(hst), ph);
   float2 R = __ffma2_rn(dx, dx, s2);
   R = __ffma2_rn(dy, dy, R);
   R = __ffma2_rn(dz, dz, R);
-  const HoTerms2 t = ho_terms2(R, s2, false, false);
+  const HoTerms2 t = ho_terms2(R, s2, false, false, uni);
   sp[0] = __ffma2_rn(t.q, ax, sp[0]);
   sp[1] = __ffma2_rn(t.q, ay, sp[1]);
   sp[2] = __ffma2_rn(t.q, az, sp[2]);
@@ -149,8 +156,8 @@ __device__ __forceinline__ void ho_far_pair2(float2 px, float2 py, float2 pz, fl
 // per pair, from the pair's own distance (58 operations).
 __device__ __forceinline__ void ho_near_pair2(float2 px, float2 py, float2 pz, float2 ph, float2 ax, float2 ay,
                                               float2 az, float2 av, const float2 *X, const float *at, float hst,
-                                              float vt, const float2 *AT, float2 *sv, float2 *sd, float2 *sp,
-                                              float2 *sz) {
+                                              float vt, const HoSigma2 *uni, const float2 *AT, float2 *sv,
+                                              float2 *sd, float2 *sp, float2 *sz) {
   const float2 M1 = make_float2(-1.f, -1.f);
   const float2 dx = __ffma2_rn(px, M1, X[0]);
   const float2 dy = __ffma2_rn(py, M1, X[1]);
@@ -158,8 +165,8 @@ __device__ __forceinline__ void ho_near_pair2(float2 px, float2 py, float2 pz, f
   float2 r2 = __fmul2_rn(dx, dx);
   r2 = __ffma2_rn(dy, dy, r2);
   r2 = __ffma2_rn(dz, dz, r2);
-  const float2 s2 = __fadd2_rn(dup2(hst), ph);
-  const HoTerms2 t = ho_terms2(__fadd2_rn(r2, s2), s2, !(r2.x > 0.f), !(r2.y > 0.f));
+  const float2 s2 = uni ? uni->s2 : __fadd2_rn(dup2(hst), ph);
+  const HoTerms2 t = ho_terms2(__fadd2_rn(r2, s2), s2, !(r2.x > 0.f), !(r2.y > 0.f), uni);
   const float2 wx = make_float2(ay.x * dz.x - az.x * dy.x, ay.y * dz.y - az.y * dy.y);
   const float2 wy = make_float2(az.x * dx.x - ax.x * dz.x, az.y * dx.y - ax.y * dz.y);
   const float2 wz = make_float2(ax.x * dy.x - ay.x * dx.x, ax.y * dy.y - ay.y * dx.y);

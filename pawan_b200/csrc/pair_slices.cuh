@@ -17,7 +17,7 @@
 //
 // High-order kernel (KER): every pair takes its full terms, two sources per
 // packed instruction, 42 FP32 operations in slices far from the targets and 58
-// in the others, against 68 scalar instructions in the generic body; no pair
+// in the others (two less where one sigma serves the slice), against 68 scalar instructions in the generic body; no pair
 // is cheap enough for wider tiles to pay, so it takes these slices at any size.
 #pragma once
 
@@ -248,30 +248,41 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
       for (int m = 0; m < 3; ++m) sv[m] = sd[m] = sp[m] = dup2(0.f);
       if constexpr (KER == kHighOrder) {
         float2 zs[3] = {dup2(0.f), dup2(0.f), dup2(0.f)};
-        if (far) {
-          float2 B[3], sw = dup2(0.f);
-          far_b3(pt.x - rx, pt.y - ry, pt.z - rz, AT, B);
+        auto sums = [&](const HoSigma2 *uni) {
+          if (far) {
+            float2 B[3], sw = dup2(0.f);
+            far_b3(pt.x - rx, pt.y - ry, pt.z - rz, AT, B);
 #pragma unroll 2
-          for (int r = 0; r < npr; ++r) {
-            const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1],
-                         na = st.N[2 * r], nb = st.N[2 * r + 1];
-            ho_far_pair2(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y),
-                         make_float2(pb.z, pb.w), make_float2(qa.x, qa.y), make_float2(qa.z, qa.w),
-                         make_float2(qb.x, qb.y), make_float2(qb.z, qb.w), make_float2(na.x, na.y),
-                         make_float2(na.z, na.w), make_float2(nb.x, nb.y), X, pt.w, AT, B, sv, sd, sp, zs, sw);
-          }
+            for (int r = 0; r < npr; ++r) {
+              const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1],
+                           na = st.N[2 * r], nb = st.N[2 * r + 1];
+              ho_far_pair2(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y),
+                           make_float2(pb.z, pb.w), make_float2(qa.x, qa.y), make_float2(qa.z, qa.w),
+                           make_float2(qb.x, qb.y), make_float2(qb.z, qb.w), make_float2(na.x, na.y),
+                           make_float2(na.z, na.w), make_float2(nb.x, nb.y), X, pt.w, uni, AT, B, sv, sd, sp, zs, sw);
+            }
 #pragma unroll
-          for (int m = 0; m < 3; ++m) sdv[m] = qt.w * (zs[m].x + zs[m].y) - (sw.x + sw.y) * at[m];
+            for (int m = 0; m < 3; ++m) sdv[m] = qt.w * (zs[m].x + zs[m].y) - (sw.x + sw.y) * at[m];
+          } else {
+#pragma unroll 2
+            for (int r = 0; r < npr; ++r) {
+              const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1];
+              ho_near_pair2(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y),
+                            make_float2(pb.z, pb.w), make_float2(qa.x, qa.y), make_float2(qa.z, qa.w),
+                            make_float2(qb.x, qb.y), make_float2(qb.z, qb.w), X, at, pt.w, qt.w, uni, AT, sv, sd, sp,
+                            zs);
+            }
+#pragma unroll
+            for (int m = 0; m < 3; ++m) sdv[m] = zs[m].x + zs[m].y;
+          }
+        };
+        // one sigma for all of the slice's pairs: its powers leave the loop (a
+        // padding source's terms vanish with R^-2.5 at rho ~ 1e18)
+        if (warp_min(hmin) == sbox.hs && thmin == tb.hs) {
+          const HoSigma2 g = ho_sigma2(dup2(tb.hs + sbox.hs));
+          sums(&g);
         } else {
-#pragma unroll 2
-          for (int r = 0; r < npr; ++r) {
-            const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1];
-            ho_near_pair2(make_float2(pa.x, pa.y), make_float2(pa.z, pa.w), make_float2(pb.x, pb.y),
-                          make_float2(pb.z, pb.w), make_float2(qa.x, qa.y), make_float2(qa.z, qa.w),
-                          make_float2(qb.x, qb.y), make_float2(qb.z, qb.w), X, at, pt.w, qt.w, AT, sv, sd, sp, zs);
-          }
-#pragma unroll
-          for (int m = 0; m < 3; ++m) sdv[m] = zs[m].x + zs[m].y;
+          sums(nullptr);
         }
 #pragma unroll
         for (int m = 0; m < 3; ++m) {

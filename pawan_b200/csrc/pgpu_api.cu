@@ -578,7 +578,7 @@ SlicesPlan build_slices_plan(const pgpu_ctx *c, int variant, int grid, bool own_
 // 64-source ones above 45 million pairs.  A shape or chunk count that was asked
 // for, and a tuned shape, keep the tiles.  The high-order kernel's full terms
 // for every pair take the slices at any size (1000 particles: 14 against 52 us
-// in 256 x 1 tiles; 60,000: 6.4 against 8.1 ms; 400,000: 275 against 345 ms), and
+// in 256 x 1 tiles; 60,000: 6.7 against 8.9 ms per call), and
 // so does FP64 (5000 particles: 161 against 301 us in 128 x 1 tiles; 60,001:
 // 11.0 against 12.0 ms; 200,000: 121 against 125 ms; high-order 60,001: 12.5
 // against 14.2 ms), there too with 32-source slices below 45 million pairs
