@@ -48,6 +48,8 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices64_kernel(Pair
     tb.init();
     tb.add((float)pt.x, (float)pt.y, (float)pt.z, (float)pt.w);
     reduce_box(tb);
+    const double hst0 = __shfl_sync(0xffffffffu, hst, 0);
+    const bool one_t = __all_sync(0xffffffffu, hst == hst0);
 #pragma unroll
     for (int m = 0; m < 6; ++m) hi[32 * m] = lo[32 * m] = 0.0;
     unsigned nfull = 0;
@@ -61,6 +63,8 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices64_kernel(Pair
       WarpBox sbox;
       sbox.init();
       double rx = 0, ry = 0, rz = 0;  // reference point: the slice's first source
+      double hs0 = 0;
+      bool one = one_t;  // one sigma for all of the slice's pairs
 #pragma unroll
       for (int j = 0; j < SL; ++j) {
         const int64_t i = cur + lane + 32 * j;
@@ -70,7 +74,9 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices64_kernel(Pair
           rx = __shfl_sync(0xffffffffu, p.x, 0);
           ry = __shfl_sync(0xffffffffu, p.y, 0);
           rz = __shfl_sync(0xffffffffu, p.z, 0);
+          hs0 = __shfl_sync(0xffffffffu, p.w, 0);
         }
+        one = one && (p.w == hs0 || i >= s1);
         const int e = lane + 32 * j;
         const double px = p.x - rx, py = p.y - ry, pz = p.z - rz;
         st.xy[e] = make_double2(p.x, p.y);
@@ -82,6 +88,8 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices64_kernel(Pair
         if (i < s1) sbox.add((float)p.x, (float)p.y, (float)p.z, (float)p.w);
       }
       reduce_box(sbox);
+      one = __all_sync(0xffffffffu, one);
+      const double is1 = one ? fast_rsqrt(hst0 + hs0) : 0.0;  // then 1/sigma leaves the loop
       // far by the boxes, as the tiles of pair_body_generic; positions below
       // 1e18 keep rho^2 of a far pair a positive normal number, so that its
       // root needs no test
@@ -150,7 +158,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices64_kernel(Pair
             const bool near = r2 < kFarU64 * s2;
             if (__any_sync(0xffffffffu, near)) {
               if (near) {
-                const PairTerms<double> t = pair_terms(r2, s2, ir, fast_rsqrt(s2));
+                const PairTerms<double> t = pair_terms(r2, s2, ir, one ? is1 : fast_rsqrt(s2));
                 q = t.q; F = t.F;
                 sdv[0] += t.zd * (vt * axy.x - azv.y * at[0]);
                 sdv[1] += t.zd * (vt * axy.y - azv.y * at[1]);

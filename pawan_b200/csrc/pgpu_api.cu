@@ -579,8 +579,8 @@ SlicesPlan build_slices_plan(const pgpu_ctx *c, int variant, int grid, bool own_
 // for, and a tuned shape, keep the tiles.  The high-order kernel's full terms
 // for every pair take the slices at any size (1000 particles: 14 against 52 us
 // in 256 x 1 tiles; 60,000: 6.7 against 8.9 ms per call), and
-// so does FP64 (5000 particles: 161 against 301 us in 128 x 1 tiles; 60,001:
-// 11.0 against 12.0 ms; 200,000: 121 against 125 ms; high-order 60,001: 12.5
+// so does FP64 (5000 particles: 158 against 301 us in 128 x 1 tiles; 60,001:
+// 10.7 against 12.0 ms; 200,000: 121 against 125 ms; high-order 60,001: 12.5
 // against 14.2 ms), there too with 32-source slices below 45 million pairs
 // (10,000 particles: 562 against 583 us), 64-source ones above.
 int choose_slices(const pgpu_ctx *c) {
