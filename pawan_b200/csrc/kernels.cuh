@@ -928,7 +928,8 @@ __global__ void __launch_bounds__(BLOCK) diag_pair_kernel(DiagArgs<T> a) {
 // rounding into percent-level strength errors.  Per target and source chunk,
 // row sums go to partial[c][0..2][t]; field_reduce_kernel adds the chunks.
 // e^{-u/2} is below the smallest double from u = 1491 on, so a pair at
-// u >= 1500 adds exactly zero.
+// u >= 1500 adds exactly zero.  A position, radius or strength that is not a
+// number reaches every target, as in the sum without the test.
 //
 // Bound by the FP64 pipe: about 30 operations per pair of one radius, half of
 // them the exponential.  Rows of 32 targets by eight slices (pair_slices.cuh);
@@ -978,6 +979,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps) field_kernel(FieldArgs a) {
     reduce_box(tb);
     const double hst0 = __shfl_sync(0xffffffffu, hst, 0);
     const bool one_t = __all_sync(0xffffffffu, hst == hst0);
+    const bool number_t = __all_sync(0xffffffffu, !isnan(xt + yt + zt + hst));  // the boxes pass over NaN
     double k0 = 0, k1 = 0, k2 = 0;
     for (int r = 0; r < run.nrows; ++r) {
       const int64_t cur = run.pe.off + (g * W + w) * S;
@@ -987,7 +989,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps) field_kernel(FieldArgs a) {
       __syncwarp();
       WarpBox sbox;
       sbox.init();
-      bool finite = true, one = one_t;
+      bool finite = number_t, one = one_t;
       double hs0 = 0;
 #pragma unroll
       for (int j = 0; j < SL; ++j) {
@@ -1001,11 +1003,11 @@ __global__ void __launch_bounds__(32 * kSliceWarps) field_kernel(FieldArgs a) {
         st.az[e] = az;
         sbox.add((float)x, (float)y, (float)z, (float)hs);
         if (j == 0) hs0 = __shfl_sync(0xffffffffu, hs, 0);
-        finite = finite && isfinite(ax) && isfinite(ay) && isfinite(az);
+        finite = finite && isfinite(ax) && isfinite(ay) && isfinite(az) && !isnan(x + y + z + hs);
         one = one && hs == hs0;
       }
       reduce_box(sbox);
-      // slices that add exactly zero (a strength that is not finite would not)
+      // slices that add exactly zero (a strength that is not finite, or a NaN position or radius, would not)
       if (KER == kGaussian && all_far(tb, sbox, 1510.f) && bounded(tb) && bounded(sbox) &&
           __all_sync(0xffffffffu, finite))
         continue;
@@ -1039,7 +1041,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps) field_kernel(FieldArgs a) {
               i2 = is * is;
               c = kInv2Pi15 * i2 * is;
             }
-            const double z = r2 < 1500.0 * s2 ? c * exp(-0.5 * (r2 * i2)) : 0.0;
+            const double z = r2 >= 1500.0 * s2 ? 0.0 : c * exp(-0.5 * (r2 * i2));  // NaN stays NaN
             k0 += z * axy.x;
             k1 += z * axy.y;
             k2 += z * st.az[j];
