@@ -206,7 +206,8 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
     tb.init();
     tb.add(pt.x, pt.y, pt.z, pt.w);
     reduce_box(tb);
-    const float thmin = warp_min(pt.w);
+    // one radius among the targets (equality with the largest, which no NaN passes)
+    const bool one_t = __all_sync(0xffffffffu, pt.w == tb.hs);
 
     for (int r = 0; r < run.nrows; ++r) {
       const int64_t cur = sb;
@@ -222,7 +223,6 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
                   rz = __shfl_sync(0xffffffffu, gp[0].z, 0);
       WarpBox sbox;
       sbox.init();
-      float hmin = 3.0e38f;
 #pragma unroll
       for (int j = 0; j < SL; ++j) {
         const float4 p = gp[j], q = gq[j];
@@ -231,13 +231,13 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
           float *dl_ = reinterpret_cast<float *>(st.L) + ((lane + 32 * j) >> 1) * 8 + (lane & 1);
           dl_[0] = gl[j].x; dl_[2] = gl[j].y; dl_[4] = gl[j].z;
         }
-        if (cur + lane + 32 * j < s1) {
-          sbox.add(p.x, p.y, p.z, p.w);
-          hmin = fminf(hmin, p.w);
-        }
+        if (cur + lane + 32 * j < s1) sbox.add(p.x, p.y, p.z, p.w);
       }
       reduce_box(sbox);
       const bool far = all_far(tb, sbox);
+      bool one = one_t;  // one sigma for all of the slice's pairs
+#pragma unroll
+      for (int j = 0; j < SL; ++j) one = one && (gp[j].w == sbox.hs || cur + lane + 32 * j >= s1);
       __syncwarp();
       if (r + 1 < run.nrows && sb < s1) fetch(sb);
       const int npr = (int)(min((int64_t)S, s1 - cur) + 1) >> 1;  // an odd tail pairs with a padding source
@@ -276,9 +276,9 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
             for (int m = 0; m < 3; ++m) sdv[m] = zs[m].x + zs[m].y;
           }
         };
-        // one sigma for all of the slice's pairs: its powers leave the loop (a
-        // padding source's terms vanish with R^-2.5 at rho ~ 1e18)
-        if (warp_min(hmin) == sbox.hs && thmin == tb.hs) {
+        // one sigma: its powers leave the loop (a padding source's terms
+        // vanish with R^-2.5 at rho ~ 1e18)
+        if (__all_sync(0xffffffffu, one)) {
           const HoSigma2 g = ho_sigma2(dup2(tb.hs + sbox.hs));
           sums(&g);
         } else {
@@ -291,10 +291,10 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
         }
       } else if (far) {
         far_slice(st, npr, 0, 1, X, AT, pt.x - rx, pt.y - ry, pt.z - rz, sv, sd, sp);
-      } else if (warp_min(hmin) == sbox.hs && thmin == tb.hs) {
-        // one sigma for all of the slice's pairs, as in every wake shed with
-        // one radius: its factors leave the loop (an odd tail's padding
-        // source carries no strength, so its sigma does not matter)
+      } else if (__all_sync(0xffffffffu, one)) {
+        // one sigma, as in every wake shed with one radius: its factors leave
+        // the loop (an odd tail's padding source carries no strength, so its
+        // sigma does not matter)
         const MidSigma2 g = mid_sigma2(dup2(tb.hs + sbox.hs));
         mid_slice<SPLIT, true>(st, npr, 0, 1, X, xl, at, pt.w, qt.w, &g, sv, sd, sp, sdv, nfull);
       } else {

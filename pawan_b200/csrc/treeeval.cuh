@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
     tb.init();
     tb.add(xt[0], xt[1], xt[2], hst);
     reduce_box(tb);
-    const float thmin = warp_min(hst);
+    const bool one_t = __all_sync(0xffffffffu, hst == tb.hs);  // one radius among the targets (no NaN passes)
     constexpr int SL = kWarpTile / 32;
     auto &st = ws.near;
     unsigned nfull = 0;
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
         __syncwarp();
         WarpBox sbx;
         sbx.init();
-        float hmin = 3.0e38f, rx = 0.f, ry = 0.f, rz = 0.f;
+        float hs[SL], rx = 0.f, ry = 0.f, rz = 0.f;
 #pragma unroll
         for (int j = 0; j < SL; ++j) {
           const int i = sb + lane + 32 * j;
@@ -535,12 +535,13 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
             rz = __shfl_sync(0xffffffffu, p.z, 0);
           }
           stage_source(st, lane + 32 * j, p, q, rx, ry, rz);
-          if (i < run.y) {
-            sbx.add(p.x, p.y, p.z, p.w);
-            hmin = fminf(hmin, p.w);
-          }
+          if (i < run.y) sbx.add(p.x, p.y, p.z, p.w);
+          hs[j] = p.w;
         }
         reduce_box(sbx);
+        bool one = one_t;  // one sigma for all of the slice's pairs
+#pragma unroll
+        for (int j = 0; j < SL; ++j) one = one && (hs[j] == sbx.hs || sb + lane + 32 * j >= run.y);
         const bool far_tile = all_far(tb, sbx);
         __syncwarp();
         // source pairs; an odd tail pairs with a padding source (zero strength, far away)
@@ -552,7 +553,7 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
         for (int m = 0; m < 3; ++m) sv[m] = sd[m] = sp[m] = dup2(0.f);
         if (far_tile) {
           far_slice(st, n, h, step, X2, AT3, xt[0] - rx, xt[1] - ry, xt[2] - rz, sv, sd, sp);
-        } else if (warp_min(hmin) == sbx.hs && thmin == tb.hs) {
+        } else if (__all_sync(0xffffffffu, one)) {
           const MidSigma2 g = mid_sigma2(dup2(tb.hs + sbx.hs));
           mid_slice<false, false>(st, n, h, step, X2, xt, at, hst, vt, &g, sv, sd, sp, sdv, nfull);
         } else {

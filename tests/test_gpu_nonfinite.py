@@ -29,3 +29,30 @@ def test_field_of_a_nan_particle(gpu, n, what):
     getattr(w, what)[17] = np.nan
     c, k = context(w)
     assert np.isnan(c.vorticity_field(k)).any(axis=1).all()
+
+
+@pytest.mark.parametrize("n", [40, 300, 3000, 9000])
+@pytest.mark.parametrize("kernel", ["gaussian", "highorder"])
+def test_rates_of_a_nan_radius(gpu, n, kernel):
+    """A NaN radius: the high-order kernel's terms need it for every pair, the Gaussian kernel's for the pairs near the
+    particle, itself among them; particles a whole diameter away keep finite rates there."""
+    w = ring(n)
+    w.sigma[17] = np.nan
+    c, k = context(w, kernel=kernel)
+    c.solve()
+    bad = np.isnan(np.concatenate(c.rates(k), axis=1)).any(axis=1)
+    assert bad[17]
+    if kernel == "highorder":
+        assert bad.all()
+    elif n >= 3000:
+        assert not bad[n // 2]
+
+
+def test_surrogate_rates_of_a_nan_radius(gpu):
+    w = ring(3000)
+    w.sigma[17] = np.nan
+    c, k = context(w)
+    c.surrogate_enable(0, check_targets=0)
+    c.solve()
+    v, a = c.rates(k)
+    assert np.isnan(v[17]).any() and np.isnan(a[17]).any()
