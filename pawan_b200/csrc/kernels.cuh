@@ -1321,7 +1321,7 @@ __global__ void __launch_bounds__(kProbeBlock) probe_kernel(const double *x0, co
       if constexpr (KER == kHighOrder) {
         q = pair_terms_ho(r2, s2).q;
       } else {
-        const bool near = r2 < kFarU64 * s2;
+        const bool near = !(r2 >= kFarU64 * s2);  // a NaN radius takes the closed form, which passes it on
         const double ir = fast_rsqrt(r2);
         q = ir * ir * ir;
         if (__any_sync(0xffffffffu, near)) {

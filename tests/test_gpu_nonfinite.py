@@ -56,3 +56,13 @@ def test_surrogate_rates_of_a_nan_radius(gpu):
     c.solve()
     v, a = c.rates(k)
     assert np.isnan(v[17]).any() and np.isnan(a[17]).any()
+
+
+@pytest.mark.parametrize("kernel", ["gaussian", "highorder"])
+@pytest.mark.parametrize("what", ["pos", "alpha", "sigma"])
+def test_probe_of_a_nan_particle(gpu, what, kernel):
+    """Every particle acts on every point, near or far."""
+    w = ring(1000)
+    getattr(w, what)[17] = np.nan
+    c, _ = context(w, kernel=kernel)
+    assert np.isnan(c.probe([[1.0, 0.0, 0.01], [30.0, -20.0, 5.0], [0.0, 0.0, 0.0]])).any(axis=1).all()
