@@ -166,6 +166,20 @@ struct WarpBox {
     lo[2] = fminf(lo[2], z); hi[2] = fmaxf(hi[2], z);
     hs = fmaxf(hs, h);
   }
+  // A box of FP64 points rounded to FP32, widened by more than the rounding:
+  // without it, cores next to each other far from the origin could be one FP32
+  // step (1 at a coordinate of 1e7) apart and pass for far.  Once per box:
+  // rounding keeps the order, so the smallest rounded value is that of the
+  // smallest point (widening every point cost the vorticity field of 30,000
+  // particles 5%).
+  __device__ __forceinline__ void widen() {
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      lo[m] = fmaf(fabsf(lo[m]), -0x1p-22f, lo[m]);
+      hi[m] = fmaf(fabsf(hi[m]), 0x1p-22f, hi[m]);
+    }
+    hs = fmaf(hs, 0x1p-22f, hs);
+  }
   __device__ __forceinline__ void reduce() {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -274,6 +288,7 @@ __device__ __forceinline__ void pair_body_generic(const PairArgs<T> &a) {
 #pragma unroll
       for (int k = 0; k < TPT; ++k) tb.add(xt[k][0], xt[k][1], xt[k][2], hst[k]);
       tb.reduce();
+      if constexpr (sizeof(T) == 8) tb.widen();
     }
 
     // Stage the first tile.
@@ -312,6 +327,7 @@ __device__ __forceinline__ void pair_body_generic(const PairArgs<T> &a) {
           sb_box.add(p.x, p.y, p.z, p.w);
         }
         sb_box.reduce();
+        if constexpr (sizeof(T) == 8) sb_box.widen();
         far_tile = all_far(tb, sb_box, kTileFarU);
       }
       // reference point of far tiles and n_s of the source this thread staged
@@ -977,6 +993,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps) field_kernel(FieldArgs a) {
     tb.init();
     tb.add((float)xt, (float)yt, (float)zt, (float)hst);
     reduce_box(tb);
+    tb.widen();
     const double hst0 = __shfl_sync(0xffffffffu, hst, 0);
     const bool one_t = __all_sync(0xffffffffu, hst == hst0);
     const bool number_t = __all_sync(0xffffffffu, !isnan(xt + yt + zt + hst));  // the boxes pass over NaN
@@ -1007,6 +1024,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps) field_kernel(FieldArgs a) {
         one = one && hs == hs0;
       }
       reduce_box(sbox);
+      sbox.widen();
       // slices that add exactly zero (a strength that is not finite, or a NaN position or radius, would not)
       if (KER == kGaussian && all_far(tb, sbox, 1510.f) && bounded(tb) && bounded(sbox) &&
           __all_sync(0xffffffffu, finite))

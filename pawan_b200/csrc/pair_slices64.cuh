@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices64_kernel(Pair
     tb.init();
     tb.add((float)pt.x, (float)pt.y, (float)pt.z, (float)pt.w);
     reduce_box(tb);
+    tb.widen();
     const double hst0 = __shfl_sync(0xffffffffu, hst, 0);
     const bool one_t = __all_sync(0xffffffffu, hst == hst0);
 #pragma unroll
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices64_kernel(Pair
         if (i < s1) sbox.add((float)p.x, (float)p.y, (float)p.z, (float)p.w);
       }
       reduce_box(sbox);
+      sbox.widen();
       one = __all_sync(0xffffffffu, one);
       const double is1 = one ? fast_rsqrt(hst0 + hs0) : 0.0;  // then 1/sigma leaves the loop
       // far by the boxes, as the tiles of pair_body_generic; positions below
