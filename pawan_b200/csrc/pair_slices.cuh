@@ -93,21 +93,24 @@ __device__ __forceinline__ void row_run_sums(const RowRun &r, const double *red,
   }
 }
 
-template <int SL, bool SPLIT> struct SliceStage {
-  float4 P[32 * SL], Q[32 * SL], N[32 * SL];  // pair-interleaved as in pair_f32.cuh
+// REF: with n_s, for far pairs formed from a reference point (far_slice).
+template <int SL, bool SPLIT, bool REF = true> struct SliceStage {
+  float4 P[32 * SL], Q[32 * SL];  // pair-interleaved as in pair_f32.cuh
+  float4 N[REF ? 32 * SL : 1];
   float4 L[SPLIT ? 32 * SL : 1];
 };
 
 // Source k of a slice (position p, strength and volume q), its n_s taken
 // about the slice's reference point.
-template <int SL, bool SPLIT>
-__device__ __forceinline__ void stage_source(SliceStage<SL, SPLIT> &st, int k, float4 p, float4 q, float rx, float ry,
-                                             float rz) {
+template <int SL, bool SPLIT, bool REF>
+__device__ __forceinline__ void stage_source(SliceStage<SL, SPLIT, REF> &st, int k, float4 p, float4 q, float rx,
+                                             float ry, float rz) {
   const int e = (k >> 1) * 8 + (k & 1);
   float *dp = reinterpret_cast<float *>(st.P) + e, *dq = reinterpret_cast<float *>(st.Q) + e,
         *dn = reinterpret_cast<float *>(st.N) + e;
   dp[0] = p.x; dp[2] = p.y; dp[4] = p.z; dp[6] = p.w;
   dq[0] = q.x; dq[2] = q.y; dq[4] = q.z; dq[6] = q.w;
+  if constexpr (!REF) return;
   const float px = p.x - rx, py = p.y - ry, pz = p.z - rz;
   dn[0] = py * q.z - pz * q.y;
   dn[2] = pz * q.x - px * q.z;
@@ -133,8 +136,49 @@ __device__ __forceinline__ void far_slice(const SliceStage<SL, SPLIT> &st, int n
               make_float2(nb.x, nb.y), X, AT, B3, sv, sd, sp);
   }
 }
-template <bool SPLIT, bool CROSS, int SL>
-__device__ __forceinline__ void mid_slice(const SliceStage<SL, SPLIT> &st, int n, int r0, int step, const float2 *X,
+// The far limit without a reference point: w = alpha_s x d per pair (28 packed
+// operations), for slices whose sources may lie far apart.  AT = -3 alpha_t;
+// sv sums q w, sp q alpha_s.
+template <int SL, bool SPLIT>
+__device__ __forceinline__ void far_slice_direct(const SliceStage<SL, SPLIT, false> &st, int n, int r0, int step,
+                                                 const float2 *X, const float2 *AT, float2 *sv, float2 *sd,
+                                                 float2 *sp) {
+  const float2 M1 = make_float2(-1.f, -1.f);
+#pragma unroll 2
+  for (int k = 0; k < n; ++k) {
+    const int r = r0 + k * step;
+    const float4 pa = st.P[2 * r], pb = st.P[2 * r + 1], qa = st.Q[2 * r], qb = st.Q[2 * r + 1];
+    const float2 ax = make_float2(qa.x, qa.y), ay = make_float2(qa.z, qa.w), az = make_float2(qb.x, qb.y);
+    const float2 dx = __ffma2_rn(make_float2(pa.x, pa.y), M1, X[0]);
+    const float2 dy = __ffma2_rn(make_float2(pa.z, pa.w), M1, X[1]);
+    const float2 dz = __ffma2_rn(make_float2(pb.x, pb.y), M1, X[2]);
+    float2 r2 = __fmul2_rn(dx, dx);
+    r2 = __ffma2_rn(dy, dy, r2);
+    r2 = __ffma2_rn(dz, dz, r2);
+    const float2 ir = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
+    const float2 A = __fmul2_rn(ir, ir);
+    const float2 q = __fmul2_rn(A, ir);
+    const float2 F = __fmul2_rn(q, A);
+    const float2 wx = make_float2(ay.x * dz.x - az.x * dy.x, ay.y * dz.y - az.y * dy.y);
+    const float2 wy = make_float2(az.x * dx.x - ax.x * dz.x, az.y * dx.y - ax.y * dz.y);
+    const float2 wz = make_float2(ax.x * dy.x - ay.x * dx.x, ax.y * dy.y - ay.y * dx.y);
+    sv[0] = __ffma2_rn(q, wx, sv[0]);
+    sv[1] = __ffma2_rn(q, wy, sv[1]);
+    sv[2] = __ffma2_rn(q, wz, sv[2]);
+    float2 dot = __fmul2_rn(AT[0], wx);
+    dot = __ffma2_rn(AT[1], wy, dot);
+    dot = __ffma2_rn(AT[2], wz, dot);
+    const float2 fd = __fmul2_rn(F, dot);
+    sd[0] = __ffma2_rn(fd, dx, sd[0]);
+    sd[1] = __ffma2_rn(fd, dy, sd[1]);
+    sd[2] = __ffma2_rn(fd, dz, sd[2]);
+    sp[0] = __ffma2_rn(q, ax, sp[0]);
+    sp[1] = __ffma2_rn(q, ay, sp[1]);
+    sp[2] = __ffma2_rn(q, az, sp[2]);
+  }
+}
+template <bool SPLIT, bool CROSS, int SL, bool REF>
+__device__ __forceinline__ void mid_slice(const SliceStage<SL, SPLIT, REF> &st, int n, int r0, int step, const float2 *X,
                                           const float *xl, const float *at, float hst, float vt, const MidSigma2 *uni, float2 *sv,
                                           float2 *sd, float2 *sp, float *sdv, unsigned &nfull) {
   float2 sdv2[3] = {dup2(0.f), dup2(0.f), dup2(0.f)};

@@ -369,6 +369,7 @@ struct TreeEvalArgs {
 // SM busy.  items[k] = (leaf index, slice); counter[0] must be 0 at launch.
 constexpr int kWarpTile = 64;
 constexpr int kWarpCells = 16;
+constexpr int kNearGroup = 16;  // pairs of a compensation group of the near field
 constexpr int kWarpsPerCta = 4;
 
 // Per-warp shared buffers (all carved from dynamic shared memory, after the
@@ -378,7 +379,7 @@ struct WarpSmem {
   union {
     float sc[kWarpCells][kCellFloats];
     float2 sc2[kWarpCells / 2][kPairFloats];  // cell pairs, interleaved
-    SliceStage<kWarpTile / 32, false> near;
+    SliceStage<kWarpTile / 32, false, false> near;
   };
 };
 struct WarpSmemMlp {
@@ -504,8 +505,11 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
     // the others the closed form, with sigma's factors out of the loop where
     // one radius serves the slice.  It is most of the evaluation (about 28,000
     // near particles per target on the 1M coaxial rings) and bound by the FP32
-    // pipe: the evaluation takes 105 ms, and 116 ms with 64-source slices boxed
-    // by shuffles and sigma's factors per pair.
+    // pipe.  A lane's sums are compensated every kNearGroup pairs: groups of 64
+    // sources put dalpha of a 5000-particle Gaussian ring off by 4.1e-6, 32 by
+    // 2.7e-6 (norm-wise).  The far limit takes w per pair: the sources of a run
+    // may lie anywhere between two leaves, and w costs no more than staging n_s
+    // (evaluation 91 ms; 97 ms with the direct kernel's reference points).
     const float2 X2[3] = {dup2(xt[0]), dup2(xt[1]), dup2(xt[2])};
     const float2 AT3[3] = {dup2(-3.f * at[0]), dup2(-3.f * at[1]), dup2(-3.f * at[2])};
     WarpBox tb;
@@ -523,18 +527,13 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
         __syncwarp();
         WarpBox sbx;
         sbx.init();
-        float hs[SL], rx = 0.f, ry = 0.f, rz = 0.f;
+        float hs[SL];
 #pragma unroll
         for (int j = 0; j < SL; ++j) {
           const int i = sb + lane + 32 * j;
           const float4 p = i < run.y ? a.Ps[i] : pad_P<float>();
           const float4 q = i < run.y ? a.Qs[i] : pad_Q<float>();
-          if (j == 0) {
-            rx = __shfl_sync(0xffffffffu, p.x, 0);
-            ry = __shfl_sync(0xffffffffu, p.y, 0);
-            rz = __shfl_sync(0xffffffffu, p.z, 0);
-          }
-          stage_source(st, lane + 32 * j, p, q, rx, ry, rz);
+          stage_source(st, lane + 32 * j, p, q, 0.f, 0.f, 0.f);
           if (i < run.y) sbx.add(p.x, p.y, p.z, p.w);
           hs[j] = p.w;
         }
@@ -547,19 +546,24 @@ __global__ void __launch_bounds__(32 * eval_warps<MLP>()) tree_eval_warp_kernel(
         // source pairs; an odd tail pairs with a padding source (zero strength, far away)
         const int npr = (min(kWarpTile, run.y - sb) + 1) >> 1;
         const int n = half ? (npr + 1) >> 1 : npr;  // an odd pair pairs with padding sources (every slot is staged)
-        float2 sv[3], sd[3], sp[3];
-        float sdv[3] = {0.f, 0.f, 0.f};
+        one = __all_sync(0xffffffffu, one);
+        const MidSigma2 g = mid_sigma2(dup2(tb.hs + sbx.hs));
+        // one compensation group per kNearGroup pairs of a lane
+        for (int b = 0; b < n; b += kNearGroup) {
+          const int r0 = h + b * step, nb = min(kNearGroup, n - b);
+          float2 sv[3], sd[3], sp[3];
+          float sdv[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-        for (int m = 0; m < 3; ++m) sv[m] = sd[m] = sp[m] = dup2(0.f);
-        if (far_tile) {
-          far_slice(st, n, h, step, X2, AT3, xt[0] - rx, xt[1] - ry, xt[2] - rz, sv, sd, sp);
-        } else if (__all_sync(0xffffffffu, one)) {
-          const MidSigma2 g = mid_sigma2(dup2(tb.hs + sbx.hs));
-          mid_slice<false, false>(st, n, h, step, X2, xt, at, hst, vt, &g, sv, sd, sp, sdv, nfull);
-        } else {
-          mid_slice<false, false>(st, n, h, step, X2, xt, at, hst, vt, nullptr, sv, sd, sp, sdv, nfull);
+          for (int m = 0; m < 3; ++m) sv[m] = sd[m] = sp[m] = dup2(0.f);
+          if (far_tile) {
+            far_slice_direct(st, nb, r0, step, X2, AT3, sv, sd, sp);
+          } else if (one) {
+            mid_slice<false, false>(st, nb, r0, step, X2, xt, at, hst, vt, &g, sv, sd, sp, sdv, nfull);
+          } else {
+            mid_slice<false, false>(st, nb, r0, step, X2, xt, at, hst, vt, nullptr, sv, sd, sp, sdv, nfull);
+          }
+          fold_group_f32<false>(false, 0.f, 0.f, 0.f, at, a.nu2, sv, sd, sp, sdv, vh, vl, dh, dl);
         }
-        fold_group_f32<false>(far_tile, xt[0] - rx, xt[1] - ry, xt[2] - rz, at, a.nu2, sv, sd, sp, sdv, vh, vl, dh, dl);
       }
     }
     double out[6];
