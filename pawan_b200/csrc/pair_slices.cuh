@@ -362,4 +362,54 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
   }
 }
 
+// How many pairs of a system take the closed form in slices and in CTA-wide
+// tiles (choose_slices): one CTA per sampled target position, against every
+// `stride`-th block of 128 sources of its system.  out[sample] = (32-source slices not far
+// from 32 targets, 128-source tiles not far from 160 targets, the span of a
+// warp of 128 x 2 tiles, blocks).
+struct NearSample {
+  int64_t off, n, t;  // first particle and particles of the system, first target
+};
+static __global__ void __launch_bounds__(256) near_share_kernel(const float4 *P, const NearSample *samples,
+                                                                int max_blocks, int4 *out) {
+  __shared__ int n32, n128;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const NearSample s = samples[blockIdx.x];
+  const int64_t end = s.off + s.n, blocks = (s.n + 127) / 128, stride = (blocks + max_blocks - 1) / max_blocks;
+  if (threadIdx.x == 0) n32 = n128 = 0;
+  __syncthreads();
+  WarpBox t32, t160;
+  t160.init();
+  for (int j = 0; j < 5; ++j) {
+    const float4 p = P[min(s.t + lane + 32 * j, end - 1)];
+    t160.add(p.x, p.y, p.z, p.w);
+    if (j == 0) {
+      t32 = t160;
+      reduce_box(t32);
+    }
+  }
+  reduce_box(t160);
+  for (int64_t b = w * stride; b < blocks; b += 8 * stride) {
+    WarpBox tile;
+    tile.init();
+    int near = 0;
+    for (int j = 0; j < 4; ++j) {
+      const float4 p = P[min(s.off + 128 * b + 32 * j + lane, end - 1)];
+      WarpBox slice;
+      slice.init();
+      slice.add(p.x, p.y, p.z, p.w);
+      tile.add(p.x, p.y, p.z, p.w);
+      reduce_box(slice);
+      near += !all_far(t32, slice);
+    }
+    reduce_box(tile);
+    if (lane == 0) {
+      atomicAdd(&n32, near);
+      atomicAdd(&n128, (int)!all_far(t160, tile));
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) out[blockIdx.x] = make_int4(n32, n128, (int)((blocks + stride - 1) / stride), 0);
+}
+
 }  // namespace pgpu

@@ -561,6 +561,43 @@ SlicesPlan build_slices_plan(const pgpu_ctx *c, int variant, int grid, bool own_
   return p;
 }
 
+// Whether the closed-form pairs that 32-source slices save outweigh the tiles'
+// two targets per staged source, from box tests at 128 positions spread over
+// the context's pairs.  F and f are the shares of closed-form pairs in tiles
+// and in slices; slices against tiles, in ms: F - f = 0.01 (1M ring of 1000 per
+// section) 1409 / 1083; 0.14 (rotor wake of 600,000) 491 / 516; 0.27 (of 200,000)
+// 58.6 / 74.5.  They meet at about 1/8.
+int rows_pay(pgpu_ctx *c, double pairs, bool *pay) {
+  constexpr int kSamples = 128;
+  NearSample smp[kSamples];
+  double before = 0.0;
+  int k = 0;
+  for (int s = 0; s < (int)c->sys.size(); ++s) {
+    const int64_t n = sys_n(c, s);
+    const auto t = owned(c, s);
+    const double p = (double)t.second * (double)n;
+    for (; k < kSamples && (k + 0.5) / kSamples * pairs < before + p; ++k) {
+      const int64_t i = std::min<int64_t>(t.second - 1, (int64_t)(((k + 0.5) / kSamples * pairs - before) / n));
+      smp[k] = {c->sys[s].off, n, c->sys[s].off + t.first + i};
+    }
+    before += p;
+  }
+  *pay = false;
+  if (k == 0) return PGPU_OK;
+  NearSample *in = reinterpret_cast<NearSample *>(io_take(c, sizeof(smp)));
+  int4 *out = in ? reinterpret_cast<int4 *>(io_take(c, kSamples * sizeof(int4))) : nullptr;
+  if (!out) return fail(c, PGPU_ECUDA, "waiting for the pinned transfer buffer failed");
+  memcpy(in, smp, k * sizeof(NearSample));
+  near_share_kernel<<<k, 256, 0, c->st>>>(static_cast<const float4 *>(c->P), in, 512, out);
+  CK(cudaGetLastError());
+  c->launches++;
+  CK(cudaStreamSynchronize(c->st));
+  double gain = 0.0;  // sum of F - f
+  for (int j = 0; j < k; ++j) gain += (out[j].y - 0.25 * out[j].x) / out[j].z;
+  *pay = gain > k / 8.0;
+  return PGPU_OK;
+}
+
 // Variant of the slices kernel for the context's next evaluations, -1 for the
 // CTA-wide tiles of pair_kernel.  Times per evaluation, CTA-wide 128 x 2 tiles
 // / 32-source / 64-source slices, in us:
@@ -572,10 +609,11 @@ SlicesPlan build_slices_plan(const pgpu_ctx *c, int variant, int grid, bool own_
 //     200,000: 76,306 / 58,493 / 58,840
 // The CTA-wide tiles need about 24 items per CTA to fill the device and gain
 // two targets per staged source; the slices' finer boxes find more far pairs.
-// So dense filaments (split positions) take 32-source slices at any size, and
-// the others slices while all systems together have fewer than 48,000 targets
-// (16 rings of 2000-32,000, 160,000 in all: 5.8 ms in tiles, 6.3 ms in slices),
-// 64-source ones above 45 million pairs.  A shape or chunk count that was asked
+// So all take slices while all systems together have fewer than 48,000 targets
+// (16 rings of 2000-32,000, 160,000 in all: 5.8 ms in tiles, 6.3 ms in slices):
+// 64-source ones above 45 million pairs, 32-source ones with split positions.
+// Beyond, contexts with split positions, which are meant for dense filaments,
+// keep the slices where the finer boxes pay (rows_pay).  A shape or chunk count that was asked
 // for, and a tuned shape, keep the tiles.  The high-order kernel's full terms
 // for every pair take the slices at any size (1000 particles: 14 against 52 us
 // in 256 x 1 tiles; 60,000: 6.7 against 8.9 ms per call), and
@@ -583,17 +621,23 @@ SlicesPlan build_slices_plan(const pgpu_ctx *c, int variant, int grid, bool own_
 // 10.7 against 12.0 ms; 200,000: 121 against 125 ms; high-order 60,001: 12.5
 // against 14.2 ms), there too with 32-source slices below 45 million pairs
 // (10,000 particles: 562 against 583 us), 64-source ones above.
-int choose_slices(const pgpu_ctx *c) {
-  if (!c->auto_shape || c->cfg.chunks > 0 || c->sur) return -1;
-  if (uses_split(c)) return 0;
+int choose_slices(pgpu_ctx *c, int *variant) {
+  *variant = -1;
+  if (!c->auto_shape || c->cfg.chunks > 0 || c->sur) return PGPU_OK;
   double pairs = 0.0, targets = 0.0;
   for (int s = 0; s < (int)c->sys.size(); ++s) {
     const double tn = (double)owned(c, s).second;
     pairs += tn * (double)sys_n(c, s);
     targets += tn;
   }
-  if (targets > 48000.0 && c->cfg.kernel == PGPU_KERNEL_GAUSSIAN && !fp64(c)) return -1;
-  return pairs < 4.5e7 ? 0 : 1;
+  if (targets > 48000.0 && c->cfg.kernel == PGPU_KERNEL_GAUSSIAN && !fp64(c)) {
+    bool pay = false;
+    if (uses_split(c))
+      if (int r = rows_pay(c, pairs, &pay)) return r;
+    if (!pay) return PGPU_OK;
+  }
+  *variant = uses_split(c) || pairs < 4.5e7 ? 0 : 1;
+  return PGPU_OK;
 }
 
 int upload_plan(pgpu_ctx *c) {
@@ -612,7 +656,8 @@ int upload_plan(pgpu_ctx *c) {
     }
   }
   std::vector<PlanEntry> plan;
-  c->slices = c->groups.empty() ? choose_slices(c) : -1;
+  c->slices = -1;
+  if (c->groups.empty() && (r = choose_slices(c, &c->slices))) return r;
   if (c->slices >= 0) {
     SlicesPlan p = build_slices_plan(c, c->slices, c->grid_slices[c->slices], true);
     plan = std::move(p.plan);
