@@ -45,3 +45,18 @@ def test_split_positions(gpu, wakes, rows):
         t = np.linspace(0, w.n - 1, 20).astype(np.int64)
         for got, ref in zip(c.rates(k), O.restate_rates(w, NU, targets=t)):
             assert np.abs(got[t] - ref).max() <= 1e-5 * np.abs(got).max()
+
+
+@pytest.mark.parametrize("n,most", [(4000, 2), (8192, 2), (8193, 1), (24676, 1), (65536, 1), (65537, 1)])
+def test_upload_launches(gpu, n, most):
+    """Two halves of the pinned ring at most: uploads that would turn it over (a wait for the stream each time) go through
+    the device's staging buffer in one piece."""
+    w = section_ring(-(-n // 250) * 250).subset(n)
+    c = capi.Context(precision=capi.FP32C, nu=NU)
+    k = c.add_wake(n)
+    c.set_particles(k, w)
+    before = c.launch_count()
+    c.set_particles(k, w)
+    assert c.launch_count() - before <= most
+    for got, ref in zip(c.particles(k), (w.pos, w.alpha, w.sigma, w.vol)):
+        assert np.array_equal(got, ref)
