@@ -214,31 +214,61 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
-// One warp per leaf.
-template <int NM>
-__global__ void __launch_bounds__(128) leaf_moments_kernel(const TreeCell *cells, const int *leaves, int nleaves,
-                                                           const float4 *Ps, const float4 *Qs, CellSums *out) {
-  const int lane = threadIdx.x & 31;
-  const int li = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (li >= nleaves) return;
-  const int ci = leaves[li];
-  const int start = cells[ci].start, end = cells[ci].end;
+// A leaf is one warp's work, four warps per CTA.  Only leaves at the last level
+// hold more than the leaf size (at most 512): particles that no cube separates,
+// any number of them.  Those above kWarpLeaf take a CTA of kLeafWarps warps in a
+// launch of their own, made when the tree has that level (100,000 particles in
+// one point of 300,000: tree 22.8 ms with one warp for them and their 21
+// ancestors in turn).
+constexpr int kWarpLeaf = 1024, kLeafWarps = 8, kLeafGrid = 1024;
+
+// Sum and maximum over the W warps of a leaf; all threads get the sum in the
+// same order.
+template <int W> __device__ __forceinline__ double leaf_sum_d(double v, double *red) {
+  v = warp_sum_d(v);
+  if constexpr (W > 1) {
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0.0;
+#pragma unroll
+    for (int k = 0; k < W; ++k) v += red[k];
+  }
+  return v;
+}
+template <int W> __device__ __forceinline__ float leaf_max_f(float v, double *red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if constexpr (W > 1) {
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < W; ++k) v = fmaxf(v, (float)red[k]);
+  }
+  return v;
+}
+
+template <int NM, int W>
+__device__ __forceinline__ void leaf_moments(int ci, int start, int end, const float4 *Ps, const float4 *Qs,
+                                             CellSums *out, double *red) {
+  const int t = threadIdx.x % (32 * W);
   double s[7] = {0, 0, 0, 0, 0, 0, 0};
   float H = 0.f;
-  for (int i = start + lane; i < end; i += 32) {
+  for (int i = start + t; i < end; i += 32 * W) {
     const float4 p = Ps[i], q = Qs[i];
     s[0] += p.x; s[1] += p.y; s[2] += p.z; s[3] += q.x; s[4] += q.y; s[5] += q.z; s[6] += p.w;
     H = fmaxf(H, p.w);
   }
 #pragma unroll
-  for (int k = 0; k < 7; ++k) s[k] = warp_sum_d(s[k]);
+  for (int k = 0; k < 7; ++k) s[k] = leaf_sum_d<W>(s[k], red);
   const double cnt = (double)(end - start);
   const double cx = s[0] / cnt, cy = s[1] / cnt, cz = s[2] / cnt;
   double m[NM];
 #pragma unroll
   for (int k = 0; k < NM; ++k) m[k] = 0.0;
   float R = 0.f;
-  for (int i = start + lane; i < end; i += 32) {
+  for (int i = start + t; i < end; i += 32 * W) {
     const float4 p = Ps[i], q = Qs[i];
     const double y[3] = {p.x - cx, p.y - cy, p.z - cz};
     const double a[3] = {q.x, q.y, q.z};
@@ -263,12 +293,10 @@ __global__ void __launch_bounds__(128) leaf_moments_kernel(const TreeCell *cells
     }
   }
 #pragma unroll
-  for (int k = 0; k < NM; ++k) m[k] = warp_sum_d(m[k]);
-  for (int o = 16; o > 0; o >>= 1) {
-    R = fmaxf(R, __shfl_xor_sync(0xffffffffu, R, o));
-    H = fmaxf(H, __shfl_xor_sync(0xffffffffu, H, o));
-  }
-  if (lane == 0) {
+  for (int k = 0; k < NM; ++k) m[k] = leaf_sum_d<W>(m[k], red);
+  R = leaf_max_f<W>(R, red);
+  H = leaf_max_f<W>(H, red);
+  if (t == 0) {
     CellSums &c = out[ci];
 #pragma unroll
     for (int k = 0; k < 3; ++k) { c.x[k] = s[k]; c.a[k] = s[3 + k]; }
@@ -277,6 +305,26 @@ __global__ void __launch_bounds__(128) leaf_moments_kernel(const TreeCell *cells
     for (int k = 0; k < NM; ++k) c.m[k] = m[k];
     c.spread = __float_as_uint(R);
     c.hmax = H;
+  }
+}
+
+template <int NM>
+__global__ void __launch_bounds__(128) leaf_moments_kernel(const TreeCell *cells, const int *leaves, int nleaves,
+                                                           const float4 *Ps, const float4 *Qs, CellSums *out) {
+  const int li = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (li >= nleaves) return;
+  const int ci = leaves[li], start = cells[ci].start, end = cells[ci].end;
+  if (end - start <= kWarpLeaf) leaf_moments<NM, 1>(ci, start, end, Ps, Qs, out, nullptr);
+}
+// The leaves above kWarpLeaf among the cells [c0, c1) of the last level.
+template <int NM>
+__global__ void __launch_bounds__(32 * kLeafWarps) big_leaf_moments_kernel(const TreeCell *cells, int c0, int c1,
+                                                                           const float4 *Ps, const float4 *Qs,
+                                                                           CellSums *out) {
+  __shared__ double red[kLeafWarps];
+  for (int ci = c0 + blockIdx.x; ci < c1; ci += gridDim.x) {
+    const int start = cells[ci].start, end = cells[ci].end;
+    if (end - start > kWarpLeaf) leaf_moments<NM, kLeafWarps>(ci, start, end, Ps, Qs, out, red);
   }
 }
 
@@ -357,26 +405,42 @@ __global__ void __launch_bounds__(128) parent_moments_kernel(const TreeCell *cel
   }
 }
 
-// Spread radii of the split cells: one warp per leaf takes its particles'
-// largest distance from every ancestor's centroid.
+// Spread radii of the split cells: every leaf takes its particles' largest
+// distance from each ancestor's centroid; the large ones with a CTA per ancestor
+// (blockIdx.y).
+template <int W>
+__device__ __forceinline__ void leaf_spread(const TreeCell *cells, const TreeCell &l, int ci, const float4 *Ps,
+                                            CellSums *sums, double *red) {
+  const int t = threadIdx.x % (32 * W);
+  const double cnt = (double)(cells[ci].end - cells[ci].start);
+  const double cx = sums[ci].x[0] / cnt, cy = sums[ci].x[1] / cnt, cz = sums[ci].x[2] / cnt;
+  float R = 0.f;
+  for (int i = l.start + t; i < l.end; i += 32 * W) {
+    const float4 p = Ps[i];
+    const double y[3] = {p.x - cx, p.y - cy, p.z - cz};
+    R = fmaxf(R, (float)sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]));
+  }
+  R = leaf_max_f<W>(R, red);
+  // non-negative floats order as their bits
+  if (t == 0) atomicMax(&sums[ci].spread, __float_as_uint(R));
+}
 __global__ void __launch_bounds__(128) spread_kernel(const TreeCell *cells, const int *leaves, int nleaves,
                                                      const float4 *Ps, CellSums *sums) {
-  const int lane = threadIdx.x & 31;
   const int li = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (li >= nleaves) return;
   const TreeCell l = cells[leaves[li]];
-  for (int ci = l.parent; ci >= 0; ci = cells[ci].parent) {
-    const double cnt = (double)(cells[ci].end - cells[ci].start);
-    const double cx = sums[ci].x[0] / cnt, cy = sums[ci].x[1] / cnt, cz = sums[ci].x[2] / cnt;
-    float R = 0.f;
-    for (int i = l.start + lane; i < l.end; i += 32) {
-      const float4 p = Ps[i];
-      const double y[3] = {p.x - cx, p.y - cy, p.z - cz};
-      R = fmaxf(R, (float)sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]));
-    }
-    for (int o = 16; o > 0; o >>= 1) R = fmaxf(R, __shfl_xor_sync(0xffffffffu, R, o));
-    // non-negative floats order as their bits
-    if (lane == 0) atomicMax(&sums[ci].spread, __float_as_uint(R));
+  if (l.end - l.start > kWarpLeaf) return;
+  for (int ci = l.parent; ci >= 0; ci = cells[ci].parent) leaf_spread<1>(cells, l, ci, Ps, sums, nullptr);
+}
+__global__ void __launch_bounds__(32 * kLeafWarps) big_spread_kernel(const TreeCell *cells, int c0, int c1,
+                                                                     const float4 *Ps, CellSums *sums) {
+  __shared__ double red[kLeafWarps];
+  for (int k = c0 + blockIdx.x; k < c1; k += gridDim.x) {
+    const TreeCell l = cells[k];
+    if (l.end - l.start <= kWarpLeaf) continue;
+    int ci = l.parent;
+    for (int up = 0; up < (int)blockIdx.y; ++up) ci = cells[ci].parent;
+    leaf_spread<kLeafWarps>(cells, l, ci, Ps, sums, red);
   }
 }
 
