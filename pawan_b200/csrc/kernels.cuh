@@ -1370,6 +1370,58 @@ __global__ void __launch_bounds__(kProbeBlock) probe_kernel(const double *x0, co
   }
 }
 
+// The same with the lanes over the points, for calls whose points fill the
+// device by themselves (probe_by_points): a thread sums all particles for its
+// point, so there are no partial sums to store and reduce.
+template <int KER = kGaussian>
+__global__ void __launch_bounds__(kProbeBlock) probe_points_kernel(const double *x0, const double *sig, int64_t cap,
+                                                                   int64_t lo, int64_t hi, const double *pts,
+                                                                   int64_t npts, double *vel) {
+  __shared__ double sx[kProbeBlock][8];  // position, sigma^2, strength, 1/sigma
+  const int64_t pi = blockIdx.x * (int64_t)kProbeBlock + threadIdx.x;
+  const bool valid = pi < npts;
+  const int64_t pl = valid ? pi : npts - 1;
+  const double x = pts[3 * pl], y = pts[3 * pl + 1], z = pts[3 * pl + 2];
+  double u[3] = {0.0, 0.0, 0.0};
+  for (int64_t sb = lo; sb < hi; sb += kProbeBlock) {
+    __syncthreads();
+    const int64_t j = sb + threadIdx.x;
+    if (j < hi) {
+      double *s = sx[threadIdx.x];
+      for (int m = 0; m < 3; ++m) {
+        s[m] = x0[m * cap + j];
+        s[4 + m] = x0[(3 + m) * cap + j];
+      }
+      s[3] = sig[j] * sig[j];
+      s[7] = fast_rsqrt(s[3]);
+    }
+    __syncthreads();
+    const int cnt = (int)min((int64_t)kProbeBlock, hi - sb);
+#pragma unroll 2
+    for (int k = 0; k < cnt; ++k) {
+      const double *s = sx[k];
+      const double dx = x - s[0], dy = y - s[1], dz = z - s[2], s2 = s[3];
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      double q;
+      if constexpr (KER == kHighOrder) {
+        q = pair_terms_ho(r2, s2).q;
+      } else {
+        const bool near = !(r2 >= kFarU64 * s2);
+        const double ir = fast_rsqrt(r2);
+        q = ir * ir * ir;
+        if (__any_sync(0xffffffffu, near)) {
+          if (near) q = pair_terms(r2, s2, ir, s[7]).q;
+        }
+      }
+      u[0] += q * (s[5] * dz - s[6] * dy);
+      u[1] += q * (s[6] * dx - s[4] * dz);
+      u[2] += q * (s[4] * dy - s[5] * dx);
+    }
+  }
+  if (valid)
+    for (int m = 0; m < 3; ++m) vel[3 * pi + m] = u[m] * kInv4Pi;
+}
+
 static __global__ void probe_reduce_kernel(const double *part, int chunks, int64_t n3, double *vel) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n3; i += (int64_t)gridDim.x * blockDim.x) {
     double v = 0.0;

@@ -1375,6 +1375,22 @@ int pgpu_diagnose(pgpu_ctx *c, int32_t system, double *out, double *vbi) {
   return PGPU_OK;
 }
 
+// Whether the lanes of a probe call hold points instead of particles: from the
+// point counts on at which the points fill the device.  Gaussian pairs take the
+// far limit by warps, and 32 particles in a row are together where 32 points
+// need not be, so only wakes of a few hundred particles gain there.  Whole
+// calls, lanes over particles / points, in us:
+//   Gaussian, 30,000 points  100 particles: 747 / 733;  200: 761 / 802
+//     100,000 points  25: 1272 / 1075;  400: 1422 / 1387;  1000: 1563 / 1902
+//     1M points  25: 8376 / 7068;  400: 9573 / 8427;  5000: 27,427 / 37,490
+//   high-order, 30,000 points  1000: 816 / 853;  5000: 1182 / 1457
+//     60,000 points  100: 918 / 846;  5000: 1868 / 1805;  20,000: 4826 / 4468
+//     1M points  100: 8006 / 7431;  20,000: 72,202 / 47,387
+static bool probe_by_points(const pgpu_ctx *c, int64_t n, int64_t npts) {
+  if (c->cfg.kernel == PGPU_KERNEL_HIGHORDER) return npts >= 60000;
+  return npts >= 30000 && n <= (npts >= 100000 ? 400 : 128);
+}
+
 int pgpu_probe(pgpu_ctx *c, int32_t system, int64_t npts, const double *pts, double *vel) {
   if (!c) return PGPU_EINVAL;
   DeviceScope device_scope(c->cfg.device);
@@ -1393,7 +1409,8 @@ int pgpu_probe(pgpu_ctx *c, int32_t system, int64_t npts, const double *pts, dou
   // points, velocities and per-chunk sums: in the context's transfer staging
   // (free between calls, ordered on its stream) where they fit, as for a few
   // hundred points of any wake, else in an allocation of this call
-  const int64_t need = (6 + 3 * chunks) * npts;
+  const bool by_points = probe_by_points(c, hi - lo, npts);
+  const int64_t need = (6 + (by_points ? 0 : 3 * chunks)) * npts;
   const bool own = need > 8 * c->cap;
   double *d = c->stage;
   if (own) CK(cudaMallocAsync((void **)&d, need * sizeof(double), c->st));
@@ -1402,8 +1419,14 @@ int pgpu_probe(pgpu_ctx *c, int32_t system, int64_t npts, const double *pts, dou
   // the velocities come back through the ring where they fit
   double *h_vel = reinterpret_cast<double *>(io_take(c, 3 * npts * sizeof(double)));
   if (h_vel) d_vel = h_vel;
-  if (hi > lo) {
-    auto fn = c->cfg.kernel == PGPU_KERNEL_HIGHORDER ? probe_kernel<kHighOrder> : probe_kernel<kGaussian>;
+  const bool ho = c->cfg.kernel == PGPU_KERNEL_HIGHORDER;
+  if (hi > lo && by_points) {
+    auto fn = ho ? probe_points_kernel<kHighOrder> : probe_points_kernel<kGaussian>;
+    fn<<<(unsigned)ceil_div(npts, kProbeBlock), kProbeBlock, 0, c->st>>>(c->x0, c->sig, c->cap, lo, hi, d, npts, d_vel);
+    CK(cudaGetLastError());
+    c->launches++;
+  } else if (hi > lo) {
+    auto fn = ho ? probe_kernel<kHighOrder> : probe_kernel<kGaussian>;
     fn<<<dim3((unsigned)tiles, (unsigned)chunks), kProbeBlock, 0, c->st>>>(c->x0, c->sig, c->cap, lo, hi, per, d, npts,
                                                                            d_part);
     CK(cudaGetLastError());

@@ -60,3 +60,34 @@ def test_upload_launches(gpu, n, most):
     assert c.launch_count() - before <= most
     for got, ref in zip(c.particles(k), (w.pos, w.alpha, w.sigma, w.vol)):
         assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("kernel,n,npts,by_points", [
+    ("gaussian", 1, 30000, True), ("gaussian", 1, 29999, False), ("gaussian", 128, 30001, True),
+    ("gaussian", 129, 30000, False), ("gaussian", 257, 100000, True), ("gaussian", 400, 100031, True),
+    ("gaussian", 401, 100000, False), ("highorder", 25, 59999, False), ("highorder", 25, 60000, True),
+    ("highorder", 3000, 60001, True)])
+def test_probe_many_points(gpu, kernel, n, npts, by_points):
+    """Calls whose points fill the device sum each point in one thread, one launch instead of two; 1e-11 of the largest
+    velocity, as the probe tests of few points."""
+    w = cases.ring_stations(stations=max(16, -(-n // 25)), seed=3).subset(n)
+    pts = np.random.default_rng(n + npts).normal(0.0, 0.8, (npts, 3))
+    c = capi.Context(precision=capi.FP32C, nu=NU, kernel=kernel)
+    c.set_particles(c.add_wake(n), w)
+    c.probe(pts)
+    before = c.launch_count()
+    v = c.probe(pts)
+    assert c.launch_count() - before == (1 if by_points else 2)
+    rows = np.concatenate(([0, 31, 32, 255, 256, npts - 1], np.random.default_rng(1).integers(0, npts, 20)))
+    ref = np.array([O.restate_getvi(w, pts[k], kernel) for k in rows])
+    assert np.abs(v[rows] - ref).max() <= 1e-11 * np.abs(v).max()
+
+
+def test_probe_many_points_of_a_nan_particle(gpu):
+    for what in ("pos", "sigma", "alpha"):
+        w = cases.ring_stations(stations=16, seed=3).subset(100)
+        getattr(w, what)[17] = np.nan
+        c = capi.Context(precision=capi.FP32C, nu=NU)
+        c.set_particles(c.add_wake(100), w)
+        v = c.probe(np.random.default_rng(0).normal(0.0, 5.0, (30000, 3)))
+        assert np.isnan(v).any(axis=1).all()
