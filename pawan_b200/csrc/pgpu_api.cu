@@ -602,8 +602,21 @@ int rows_pay(pgpu_ctx *c, double pairs, bool *pay) {
   return PGPU_OK;
 }
 
+// Slice length of the row list: 32 sources (0) or 64 (1).  Longer slices share
+// the box and the fold among more pairs, shorter ones find more far pairs and
+// keep all eight warps of a row busy in systems of a few hundred particles.
+// Times per evaluation, 32-source / 64-source, in us:
+//   one Gaussian ring  5000: 55 / 61;  8000: 110 / 106;  20,000: 575 / 541
+//   FP64  10,000: 562 / 583;  7 systems of 6000: 1310 / 1323;  781 of 512: 1435 / 1856
+//   high-order  781 of 512: 507 / 485, FP64 913 / 907;  1562 of 256: 302 / 315, 520 / 619
+// A wake of several systems has pairs / targets sources on average.
+int slice_variant(double pairs, double targets, int kernel) {
+  return pairs >= 4.5e7 && pairs >= (kernel == PGPU_KERNEL_HIGHORDER ? 512.0 : 4000.0) * targets ? 1 : 0;
+}
+
 // Variant of the slices kernel for the context's next evaluations, -1 for the
-// CTA-wide tiles of pair_kernel.  Times per evaluation, CTA-wide 128 x 2 tiles
+// CTA-wide tiles of pair_kernel.  A shape or chunk count that was asked for, and
+// a tuned shape, keep the tiles.  Times per evaluation, CTA-wide 128 x 2 tiles
 // / 32-source / 64-source slices, in us:
 //   Gaussian rings (sigma = 0.02)  5000: 127 / 55 / 61;  8000: 184 / 110 / 106;
 //     20,000: 658 / 575 / 541;  40,000: 2103 / 2228 / 2065;  60,000: 4388 / 4982 / 4593
@@ -613,18 +626,18 @@ int rows_pay(pgpu_ctx *c, double pairs, bool *pay) {
 //     200,000: 76,306 / 58,493 / 58,840
 // The CTA-wide tiles need about 24 items per CTA to fill the device and gain
 // two targets per staged source; the slices' finer boxes find more far pairs.
-// So all take slices while all systems together have fewer than 48,000 targets
-// (16 rings of 2000-32,000, 160,000 in all: 5.8 ms in tiles, 6.3 ms in slices):
-// 64-source ones above 45 million pairs, 32-source ones with split positions.
+// So FP32C Gaussian contexts take slices while all systems together have fewer
+// than 48,000 targets (16 rings of 2000-40,000, 169,125 in all: 4.4 ms in tiles).
 // Beyond, contexts with split positions, which are meant for dense filaments,
-// keep the slices where the finer boxes pay (rows_pay).  A shape or chunk count that was asked
-// for, and a tuned shape, keep the tiles.  The high-order kernel's full terms
-// for every pair take the slices at any size (1000 particles: 14 against 52 us
-// in 256 x 1 tiles; 60,000: 6.7 against 8.9 ms per call), and
-// so does FP64 (5000 particles: 158 against 301 us in 128 x 1 tiles; 60,001:
-// 10.7 against 12.0 ms; 200,000: 121 against 125 ms; high-order 60,001: 12.5
-// against 14.2 ms), there too with 32-source slices below 45 million pairs
-// (10,000 particles: 562 against 583 us), 64-source ones above.
+// keep 32-source slices where the finer boxes pay (rows_pay).
+// The high-order kernel's full terms for every pair take the slices at any size
+// (1000 particles: 14 against 52 us in 256 x 1 tiles; 60,000: 6.7 against 8.9 ms
+// per call; FP64 60,001: 12.5 against 14.2 ms, 400,000: 553 against 610 ms), and
+// so does the Gaussian kernel in FP64 (5000 particles: 158 against 301 us in 128
+// x 1 tiles; 60,001: 10.7 against 12.0 ms; 1M: 2914 against 3065 ms), except for
+// systems of 33 to 256 particles with more than 150,000 targets in all, which
+// leave warps of a row idle (2000 of 100: 627 us in rows, 400 in tiles; 1000 of
+// 200: 603 and 531; but 781 of 129: 327 and 358; 16,000 of 25: 1081 and 1351).
 int choose_slices(pgpu_ctx *c, int *variant) {
   *variant = -1;
   if (!c->auto_shape || c->cfg.chunks > 0 || c->sur) return PGPU_OK;
@@ -640,7 +653,10 @@ int choose_slices(pgpu_ctx *c, int *variant) {
       if (int r = rows_pay(c, pairs, &pay)) return r;
     if (!pay) return PGPU_OK;
   }
-  *variant = uses_split(c) || pairs < 4.5e7 ? 0 : 1;
+  if (fp64(c) && c->cfg.kernel == PGPU_KERNEL_GAUSSIAN && targets > 150000.0 && pairs > 32.0 * targets &&
+      pairs <= 256.0 * targets)
+    return PGPU_OK;
+  *variant = uses_split(c) ? 0 : slice_variant(pairs, targets, c->cfg.kernel);
   return PGPU_OK;
 }
 
@@ -1474,9 +1490,12 @@ int pgpu_influence(pgpu_ctx *c) {
     }
   }
   // every particle of every system is a target; slice length as choose_slices
-  double pairs = 0.0;
-  for (size_t k = 0; k < c->sys.size(); ++k) pairs += (double)sys_n(c, (int)k) * (double)sys_n(c, (int)k);
-  const int v = pairs < 4.5e7 ? 0 : 1;
+  double pairs = 0.0, targets = 0.0;
+  for (size_t k = 0; k < c->sys.size(); ++k) {
+    pairs += (double)sys_n(c, (int)k) * (double)sys_n(c, (int)k);
+    targets += (double)sys_n(c, (int)k);
+  }
+  const int v = slice_variant(pairs, targets, c->cfg.kernel);
   const bool ho = c->cfg.kernel == PGPU_KERNEL_HIGHORDER;
   auto fn = v == 0 ? (ho ? field_kernel<1, kHighOrder> : field_kernel<1, kGaussian>)
                    : (ho ? field_kernel<2, kHighOrder> : field_kernel<2, kGaussian>);

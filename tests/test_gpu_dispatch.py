@@ -91,3 +91,26 @@ def test_probe_many_points_of_a_nan_particle(gpu):
         c.set_particles(c.add_wake(100), w)
         v = c.probe(np.random.default_rng(0).normal(0.0, 5.0, (30000, 3)))
         assert np.isnan(v).any(axis=1).all()
+
+
+@pytest.mark.parametrize("kernel", ["gaussian", "highorder"])
+def test_many_small_fp64_systems(gpu, kernel):
+    """Four times as many systems of 128 particles take about four times as long (their rows never took slices longer than
+    the systems; the first ones also pay for filling the device), and give the rates of the FP64 restatement."""
+    ms = []
+    for count in (781, 3125):
+        wakes = [cases.ring_stations(stations=16, seed=k).subset(128) for k in range(7)]
+        c = capi.Context(precision=capi.FP64, nu=NU, kernel=kernel)
+        ids = [c.add_wake(128, system=s) for s in range(count)]
+        for k in ids:
+            c.set_particles(k, wakes[k % 7])
+        c.solve()
+        c.pair_kernel_time()
+        for _ in range(3):
+            c.solve()
+        t, launches = c.pair_kernel_time()
+        ms.append(t / launches)
+        for k in (ids[0], ids[-1]):
+            for got, ref in zip(c.rates(k), O.restate_rates(wakes[k % 7], NU, kernel=kernel)):
+                assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
+    assert ms[1] <= 4.8 * ms[0]
