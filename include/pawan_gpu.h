@@ -315,12 +315,17 @@ int pgpu_kernel_shapes(int *block, int *tpt, int max);
  * systems alone (`reps` launches after one untimed).  If one shape is within
  * 2% of each class's fastest, every system uses it (one pair launch per
  * evaluation); otherwise each class uses its fastest shape, and an evaluation
- * is one pair launch per distinct shape, each over its classes' systems.
+ * is one pair launch per distinct shape, each over its classes' systems.  A
+ * context that was not asked for a shape and would take the row list for its
+ * systems times that too, and keeps it where it is faster over all classes than
+ * the shapes (*per_class is 0 then, and the classes give their fastest shape).
  * With cache_path set, a class already recorded there for this GPU name,
  * precision and kernel takes its recorded times instead of being timed, and
  * newly timed classes are appended, one JSON object per line:
  *   {"gpu": .., "precision": "fp32c"|"fp64", "kernel": "gaussian"|"highorder",
- *    "class": k, "nmin": .., "nmax": .., "block": .., "tpt": .., "ms": [one per shape]}
+ *    "class": k, "nmin": .., "nmax": .., "block": .., "tpt": .., "ms": [one per shape],
+ *    "row_sources": 32|64, "rows_ms": .. (the row list, where it was timed; a line
+ *    without them has it timed anew)}
  * classes[i] (up to max_classes) describes the i-th class present, by
  * increasing size; *per_class = 1 if the classes launch separately.  The
  * rates of the current state are recomputed with the chosen launches.  A

@@ -145,6 +145,7 @@ struct pgpu_ctx {
   // no shape was asked for or tuned: small FP32C Gaussian systems may take
   // the slices kernel (choose_slices); slices is its variant, -1 for none
   bool auto_shape = true;
+  bool shape_asked = false;  // the configuration names a shape
   int slices = -1;
   int grid_slices[kNumSlices] = {0};
   int nch = 1;
@@ -553,10 +554,11 @@ struct SlicesPlan {
   }
 };
 
-// Every system of the context, its owned targets or all of them.
-SlicesPlan build_slices_plan(const pgpu_ctx *c, int variant, int grid, bool own_targets) {
+// The systems' owned targets or all of them.
+SlicesPlan build_slices_plan(const pgpu_ctx *c, const std::vector<int> &systems, int variant, int grid,
+                             bool own_targets) {
   SlicesPlan p;
-  for (int s = 0; s < (int)c->sys.size(); ++s) {
+  for (int s : systems) {
     const int64_t n = sys_n(c, s);
     const auto t = own_targets ? owned(c, s) : std::make_pair<int64_t, int64_t>(0, sys_n(c, s));
     p.add(variant, c->sys[s].off, n, t.first, t.second);
@@ -679,7 +681,7 @@ int upload_plan(pgpu_ctx *c) {
   c->slices = -1;
   if (c->groups.empty() && (r = choose_slices(c, &c->slices))) return r;
   if (c->slices >= 0) {
-    SlicesPlan p = build_slices_plan(c, c->slices, c->grid_slices[c->slices], true);
+    SlicesPlan p = build_slices_plan(c, all_systems(c), c->slices, c->grid_slices[c->slices], true);
     plan = std::move(p.plan);
     c->nch = p.nch;
   } else if (c->groups.empty()) {
@@ -768,6 +770,18 @@ int join_side(pgpu_ctx *c) {
   return PGPU_OK;
 }
 
+// One launch of the row list `a` of slices variant v.
+template <typename T> int launch_rows(pgpu_ctx *c, int v, const PairArgs<T> &a) {
+  if constexpr (sizeof(T) == 4) {
+    slices_fn(v, c->cfg.kernel, uses_split(c))<<<c->grid_slices[v], 32 * kSliceWarps, 0, c->st>>>(a);
+  } else {
+    slices64_fn(v, c->cfg.kernel)<<<c->grid_slices[v], 32 * kSliceWarps, slices64_bytes(v), c->st>>>(a);
+  }
+  CK(cudaGetLastError());
+  c->launches++;
+  return PGPU_OK;
+}
+
 template <typename T> int launch_pair(pgpu_ctx *c, int slot) {
   PairArgs<T> a;
   a.P = static_cast<const v4_t<T> *>(c->P);
@@ -789,14 +803,7 @@ template <typename T> int launch_pair(pgpu_ctx *c, int slot) {
   a.L = c->d_L;
   if (int r = record_time(c, slot, 0)) return r;
   if (c->slices >= 0) {
-    if constexpr (sizeof(T) == 4) {
-      slices_fn(c->slices, c->cfg.kernel, uses_split(c))<<<c->grid_slices[c->slices], 32 * kSliceWarps, 0, c->st>>>(a);
-    } else {
-      slices64_fn(c->slices, c->cfg.kernel)
-          <<<c->grid_slices[c->slices], 32 * kSliceWarps, slices64_bytes(c->slices), c->st>>>(a);
-    }
-    CK(cudaGetLastError());
-    c->launches++;
+    if (int r = launch_rows(c, c->slices, a)) return r;
   } else if (c->groups.empty()) {
     pair_fn<T>(c->shape, c->cfg.kernel, uses_split(c))<<<c->grid[c->shape], kShapes[c->shape].block, 0, c->st>>>(a);
     CK(cudaGetLastError());
@@ -954,6 +961,7 @@ int pgpu_create(pgpu_ctx **out, const pgpu_config *cfg) {
                          c->cfg.block, c->cfg.tpt);
     c->shape = found;
     c->auto_shape = false;
+    c->shape_asked = true;
   } else if (c->cfg.kernel == PGPU_KERNEL_GAUSSIAN) {
     // untuned defaults: the fastest Gaussian shapes on the 1M ring, FP32C
     // 128 x 2 (1075 ms per evaluation against 1163 ms for 256 x 1) and FP64
@@ -1502,7 +1510,7 @@ int pgpu_influence(pgpu_ctx *c) {
   int nb = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 32 * kSliceWarps, 0));
   const int grid = std::max(1, nb) * c->sms;
-  const SlicesPlan p = build_slices_plan(c, v, grid, false);
+  const SlicesPlan p = build_slices_plan(c, all_systems(c), v, grid, false);
   const int nch = p.nch;
   CK(put_data(c, c->d_plan_field, p.plan.data(), p.plan.size() * sizeof(PlanEntry)));
   if (p.rows > 0) {
@@ -1750,14 +1758,24 @@ int size_class(int64_t n) {
 int64_t class_lo(int k) { return k == 0 ? 0 : (int64_t)1024 << (2 * k); }
 int64_t class_hi(int k) { return (int64_t)1024 << (2 * (k + 1)); }
 
-// Device time of one pair launch of `shape` over `systems` (their own plan and
-// chunk count), mean of `reps` launches after one untimed.
+// Device time of one pair launch of `shape` (kNumShapes + v: the row list of
+// slices variant v) over `systems` (their own plan and chunk count), mean of
+// `reps` launches after one untimed.
 template <typename T> int time_subset(pgpu_ctx *c, const std::vector<int> &systems, int shape, int reps, double *ms) {
   int r = upload_plan(c);  // system sizes on the device, for the source boxes
   if (r) return r;
-  const int nch = choose_nch_for(c, shape, systems);
-  std::vector<PlanEntry> plan = build_plan(c, systems, shape, nch);
-  plan.resize(c->sys.size() + 1, plan.back());
+  const int rows = shape - kNumShapes;
+  int nch;
+  std::vector<PlanEntry> plan;
+  if (rows >= 0) {
+    SlicesPlan p = build_slices_plan(c, systems, rows, c->grid_slices[rows], true);
+    plan = std::move(p.plan);
+    nch = p.nch;
+  } else {
+    nch = choose_nch_for(c, shape, systems);
+    plan = build_plan(c, systems, shape, nch);
+    plan.resize(c->sys.size() + 1, plan.back());
+  }
   // d_plan now holds this subset's plan: the next evaluation rebuilds the
   // context's own, also when the tuning stops early on an error
   c->plan_dirty = true;
@@ -1774,7 +1792,7 @@ template <typename T> int time_subset(pgpu_ctx *c, const std::vector<int> &syste
   a.nu2 = (T)(2.0 * c->cfg.nu);
   a.counters = c->d_counters;
   a.nfull = c->d_nfull;
-  if (uses_boxes(c)) {
+  if (uses_boxes(c) && rows < 0) {
     if ((r = launch_boxes(c))) return r;
     a.box = c->d_box;
   }
@@ -1782,9 +1800,13 @@ template <typename T> int time_subset(pgpu_ctx *c, const std::vector<int> &syste
   float total = 0.f;
   for (int k = 0; k <= reps; ++k) {
     CK(cudaEventRecord(c->ev[0][0], c->st));
-    pair_fn<T>(shape, c->cfg.kernel, uses_split(c))<<<c->grid[shape], kShapes[shape].block, 0, c->st>>>(a);
-    CK(cudaGetLastError());
-    c->launches++;
+    if (rows >= 0) {
+      if ((r = launch_rows(c, rows, a))) return r;
+    } else {
+      pair_fn<T>(shape, c->cfg.kernel, uses_split(c))<<<c->grid[shape], kShapes[shape].block, 0, c->st>>>(a);
+      CK(cudaGetLastError());
+      c->launches++;
+    }
     CK(cudaEventRecord(c->ev[0][1], c->st));
     CK(cudaEventSynchronize(c->ev[0][1]));
     float t = 0.f;
@@ -1851,7 +1873,17 @@ int pgpu_autotune_classes(pgpu_ctx *c, int reps, const char *cache_path, pgpu_tu
   const std::string gpu = prop.name;
   const std::string prec = fp64(c) ? "fp64" : "fp32c";
   const std::string ker = c->cfg.kernel == PGPU_KERNEL_HIGHORDER ? "highorder" : "gaussian";
-  // cached times: the last matching line of the file wins
+  // the context's own choice of the row list for these systems, if it makes one
+  int rows = -1;
+  if (!c->shape_asked) {
+    const bool auto_shape = c->auto_shape;
+    c->auto_shape = true;
+    r = choose_slices(c, &rows);
+    c->auto_shape = auto_shape;
+    if (r) return r;
+  }
+  // cached times: the last matching line of the file wins; the row list's time
+  // is an entry of its own after the shapes', negative where it is not known
   std::map<int, std::vector<double>> cached;
   if (cache_path && *cache_path) {
     if (FILE *f = fopen(cache_path, "r")) {
@@ -1859,10 +1891,14 @@ int pgpu_autotune_classes(pgpu_ctx *c, int reps, const char *cache_path, pgpu_tu
       while (fgets(buf, sizeof(buf), f)) {
         const std::string line(buf);
         double k = -1;
-        std::vector<double> ms(kNumShapes);
+        std::vector<double> ms(kNumShapes + 1, -1.0);
         if (json_str(line, "gpu") == gpu && json_str(line, "precision") == prec && json_str(line, "kernel") == ker &&
-            json_num(line, "class", &k) && json_ms(line, ms.data(), kNumShapes))
+            json_num(line, "class", &k) && json_ms(line, ms.data(), kNumShapes)) {
+          double v = -1;
+          if (rows >= 0 && json_num(line, "row_sources", &v) && (int)v == kSliceLen[rows])
+            json_num(line, "rows_ms", &ms[kNumShapes]);
           cached[(int)k] = ms;
+        }
       }
       fclose(f);
     }
@@ -1876,24 +1912,21 @@ int pgpu_autotune_classes(pgpu_ctx *c, int reps, const char *cache_path, pgpu_tu
   for (auto &kv : cls) {
     keys.push_back(kv.first);
     auto it = cached.find(kv.first);
-    if (it != cached.end()) {
-      tms.push_back(it->second);
-      from_cache.push_back(1);
-      continue;
-    }
-    std::vector<double> ms(kNumShapes);
-    for (int sh = 0; sh < kNumShapes; ++sh) {
-      r = fp64(c) ? time_subset<double>(c, kv.second, sh, reps, &ms[sh]) : time_subset<float>(c, kv.second, sh, reps, &ms[sh]);
+    from_cache.push_back(it != cached.end());
+    std::vector<double> ms = from_cache.back() ? it->second : std::vector<double>(kNumShapes + 1, -1.0);
+    for (int sh = from_cache.back() ? kNumShapes : 0; sh < kNumShapes + (rows >= 0); ++sh) {
+      if (sh == kNumShapes && ms[sh] >= 0.0) break;  // known from the cache
+      const int k = sh < kNumShapes ? sh : kNumShapes + rows;
+      r = fp64(c) ? time_subset<double>(c, kv.second, k, reps, &ms[sh]) : time_subset<float>(c, kv.second, k, reps, &ms[sh]);
       if (r) return r;
     }
     tms.push_back(ms);
-    from_cache.push_back(0);
   }
   // fastest shape per class, and the one shape with the least total time
   const size_t K = keys.size();
   std::vector<int> best(K);
   for (size_t i = 0; i < K; ++i)
-    best[i] = (int)(std::min_element(tms[i].begin(), tms[i].end()) - tms[i].begin());
+    best[i] = (int)(std::min_element(tms[i].begin(), tms[i].begin() + kNumShapes) - tms[i].begin());
   int single = 0;
   double single_t = 1e300;
   for (int sh = 0; sh < kNumShapes; ++sh) {
@@ -1903,10 +1936,17 @@ int pgpu_autotune_classes(pgpu_ctx *c, int reps, const char *cache_path, pgpu_tu
   }
   // one launch per class shape only if the single shape loses more than 2%
   // on some class
-  c->auto_shape = false;
   bool split = false;
   for (size_t i = 0; i < K; ++i)
     if (tms[i][single] > 1.02 * tms[i][best[i]]) split = true;
+  // the row list stays where it beats the chosen shapes over all classes
+  double rows_t = 0.0, shapes_t = 0.0;
+  for (size_t i = 0; i < K; ++i) {
+    rows_t += tms[i][kNumShapes];
+    shapes_t += tms[i][split ? best[i] : single];
+  }
+  c->auto_shape = rows >= 0 && rows_t <= shapes_t;
+  if (c->auto_shape) split = false;
   if (split) {
     c->sys_shape.assign(c->sys.size(), single);
     for (size_t i = 0; i < K; ++i)
@@ -1925,7 +1965,9 @@ int pgpu_autotune_classes(pgpu_ctx *c, int reps, const char *cache_path, pgpu_tu
                 gpu.c_str(), prec.c_str(), ker.c_str(), keys[i], (long long)class_lo(keys[i]),
                 (long long)class_hi(keys[i]), kShapes[best[i]].block, kShapes[best[i]].tpt);
         for (int sh = 0; sh < kNumShapes; ++sh) fprintf(f, "%s%.6g", sh ? ", " : "", tms[i][sh]);
-        fprintf(f, "]}\n");
+        fprintf(f, "]");
+        if (rows >= 0) fprintf(f, ", \"row_sources\": %d, \"rows_ms\": %.6g", kSliceLen[rows], tms[i][kNumShapes]);
+        fprintf(f, "}\n");
       }
       fclose(f);
     } else {

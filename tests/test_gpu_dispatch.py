@@ -114,3 +114,55 @@ def test_many_small_fp64_systems(gpu, kernel):
             for got, ref in zip(c.rates(k), O.restate_rates(wakes[k % 7], NU, kernel=kernel)):
                 assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
     assert ms[1] <= 4.8 * ms[0]
+
+
+@pytest.mark.parametrize("precision,kernel,split", [(capi.FP32C, "gaussian", False), (capi.FP32C, "gaussian", True),
+                                                    (capi.FP32C, "highorder", False)])
+def test_class_tuning_keeps_the_row_list(gpu, tmp_path, precision, kernel, split):
+    """Three small rings: the row list takes a third of the tiles' time, so tuning by class leaves it (no box kernel before
+    the pair launch, one pair launch), from measured and from cached times; results stay within FP32 rounding."""
+    wakes = [cases.ring_stations(stations=s, seed=s) for s in (40, 60, 200)]
+    cache = str(tmp_path / "tune.jsonl")
+    for run in range(2):
+        c = capi.Context(precision=precision, nu=NU, kernel=kernel, split_positions=split)
+        ids = [c.add_wake(w.n, system=s) for s, w in enumerate(wakes)]
+        for k, w in zip(ids, wakes):
+            c.set_particles(k, w)
+        c.solve()
+        before, c0 = [c.rates(k) for k in ids], c.pair_kernel_time()
+        for _ in range(3):
+            c.solve()
+        t0, n0 = c.pair_kernel_time()
+        tune = c.autotune_classes(reps=2, cache=cache)
+        assert not tune["per_class"] and all(x["from_cache"] == (run == 1) for x in tune["classes"])
+        assert launches(c) == 2
+        c.pair_kernel_time()
+        for _ in range(3):
+            c.solve()
+        t1, n1 = c.pair_kernel_time()
+        assert t1 / n1 <= 1.2 * t0 / n0
+        for k, rates in zip(ids, before):
+            for got, ref in zip(c.rates(k), rates):
+                assert np.array_equal(got, ref)
+
+
+def test_class_tuning_with_an_older_cache(gpu, tmp_path):
+    """Lines without the row list's time: it is timed, and loses to the shapes' recorded times here (1 us)."""
+    import json
+
+    import torch
+    shapes = capi.kernel_shapes()
+    b, t = shapes[1]
+    cache = tmp_path / "tune.jsonl"
+    cache.write_text("".join(json.dumps({
+        "gpu": torch.cuda.get_device_properties(0).name, "precision": "fp32c", "kernel": "gaussian", "class": k, "nmin": 0,
+        "nmax": 0, "block": b, "tpt": t, "ms": [0.001 if i == 1 else 9.0 for i in range(len(shapes))]}) + "\n"
+        for k in (0, 1)))
+    wakes = [cases.ring_stations(stations=s, seed=s) for s in (40, 200)]
+    c = capi.Context(precision=capi.FP32C, nu=NU)
+    ids = [c.add_wake(w.n, system=s) for s, w in enumerate(wakes)]
+    for k, w in zip(ids, wakes):
+        c.set_particles(k, w)
+    tune = c.autotune_classes(reps=1, cache=str(cache))
+    assert all(x["from_cache"] for x in tune["classes"]) and not tune["per_class"]
+    assert launches(c) == 3  # the tiles
