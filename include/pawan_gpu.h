@@ -303,7 +303,9 @@ int64_t pgpu_launch_count(pgpu_ctx *ctx);
  * context that was not asked for a shape keeps the library's own choice where
  * that is faster than every shape (block and tpt then give the fastest shape).
  * block/tpt receive the choice; ms_per_launch (may be NULL) receives the
- * time of each candidate in the order of pgpu_kernel_shapes. */
+ * time of each candidate in the order of pgpu_kernel_shapes.  With the surrogate
+ * enabled, whose evaluations have no shape, the choice stays as it is and the
+ * times are zero.  On an error the choice stays as it was. */
 int pgpu_autotune(pgpu_ctx *ctx, int reps, int *block, int *tpt, double *ms_per_launch);
 /* Number of compiled pair-kernel shapes and their (block, tpt). */
 int pgpu_kernel_shapes(int *block, int *tpt, int max);

@@ -1683,64 +1683,77 @@ int pgpu_kernel_shapes(int *block, int *tpt, int max) {
   return kNumShapes;
 }
 
+// Times every shape and, where the context was not asked for one, its own choice
+// of the row list, leaving the faster in place.
+static int autotune(pgpu_ctx *c, int reps, double *ms_per_launch) {
+  double best = 1e300;
+  int best_s = c->shape;
+  int64_t nl;
+  int r;
+  auto time = [&](double *ms) -> int {
+    for (int k = 0; k <= reps; ++k) {
+      int e = launch_eval(c, 0);
+      if (!e) e = collect_timing(c, 1);
+      if (e) return e;
+      if (k == 0) pgpu_pair_kernel_time(c, nullptr, nullptr);  // warm-up
+    }
+    pgpu_pair_kernel_time(c, ms, &nl);
+    *ms /= reps;
+    return PGPU_OK;
+  };
+  c->auto_shape = false;
+  for (int s = 0; s < kNumShapes; ++s) {
+    c->shape = s;
+    c->plan_dirty = true;
+    double ms;
+    if ((r = upload_plan(c))) return r;
+    if ((r = time(&ms))) return r;
+    if (ms_per_launch) ms_per_launch[s] = ms;
+    if (ms < best) { best = ms; best_s = s; }
+  }
+  c->shape = best_s;
+  if (!c->shape_asked) {
+    c->auto_shape = true;
+    c->plan_dirty = true;
+    if ((r = upload_plan(c))) return r;
+    double ms = 1e300;
+    if (c->slices >= 0 && (r = time(&ms))) return r;
+    c->auto_shape = ms <= best;
+  }
+  c->plan_dirty = true;
+  return upload_plan(c);
+}
+
 int pgpu_autotune(pgpu_ctx *c, int reps, int *block, int *tpt, double *ms_per_launch) {
   if (!c) return PGPU_EINVAL;
   DeviceScope device_scope(c->cfg.device);
   if (!c->frozen) return fail(c, PGPU_EINVAL, "no particles were uploaded");
   if (reps < 1) reps = 1;
-  c->sys_shape.clear();  // one shape for every system from here on
-  const bool auto_shape = c->auto_shape;
-  c->auto_shape = false;
-  const int saved = c->shape;
-  double best = 1e300;
-  int best_s = saved;
-  double ms_acc;
-  int64_t nl;
-  int r = pgpu_pair_kernel_time(c, &ms_acc, &nl);  // reset counters
-  for (int s = 0; s < kNumShapes; ++s) {
-    c->shape = s;
-    c->plan_dirty = true;
+  int r;
+  if (c->sur) {
+    // the surrogate's evaluations do not use the shape: nothing to choose
     if ((r = upload_plan(c))) return r;
-    if ((r = launch_eval(c, 0))) return r;  // warm-up
-    if ((r = collect_timing(c, 1))) return r;
+    for (int s = 0; s < kNumShapes && ms_per_launch; ++s) ms_per_launch[s] = 0.0;
+  } else {
+    const int shape = c->shape;
+    const bool auto_shape = c->auto_shape;
+    const std::vector<int> sys_shape = c->sys_shape;
+    c->sys_shape.clear();  // one shape for every system from here on
     pgpu_pair_kernel_time(c, nullptr, nullptr);
-    for (int k = 0; k < reps; ++k) {
-      if ((r = launch_eval(c, 0))) return r;
-      if ((r = collect_timing(c, 1))) return r;
+    if ((r = autotune(c, reps, ms_per_launch))) {
+      c->shape = shape;
+      c->auto_shape = auto_shape;
+      c->sys_shape = sys_shape;
+      c->plan_dirty = true;
+      return r;
     }
-    double ms;
-    pgpu_pair_kernel_time(c, &ms, &nl);
-    ms /= reps;
-    if (ms_per_launch) ms_per_launch[s] = ms;
-    if (ms < best) { best = ms; best_s = s; }
   }
-  c->shape = best_s;
-  c->plan_dirty = true;
-  if (auto_shape) {
-    // the row list stays where it beats every shape
-    c->auto_shape = true;
-    if ((r = upload_plan(c))) return r;
-    if (c->slices >= 0) {
-      for (int k = 0; k <= reps; ++k) {
-        if ((r = launch_eval(c, 0))) return r;
-        if ((r = collect_timing(c, 1))) return r;
-        if (k == 0) pgpu_pair_kernel_time(c, nullptr, nullptr);  // warm-up
-      }
-      double ms;
-      pgpu_pair_kernel_time(c, &ms, &nl);
-      c->auto_shape = ms / reps <= best;
-    } else {
-      c->auto_shape = false;
-    }
-    c->plan_dirty = true;
-  }
-  if ((r = upload_plan(c))) return r;
   // The partial buffer now holds the last candidate's chunks: recompute the
   // rates of the current state with the chosen shape.
   if ((r = pgpu_solve(c))) return r;
   pgpu_pair_kernel_time(c, nullptr, nullptr);
-  if (block) *block = kShapes[best_s].block;
-  if (tpt) *tpt = kShapes[best_s].tpt;
+  if (block) *block = kShapes[c->shape].block;
+  if (tpt) *tpt = kShapes[c->shape].tpt;
   return PGPU_OK;
 }
 

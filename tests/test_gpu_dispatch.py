@@ -166,3 +166,35 @@ def test_class_tuning_with_an_older_cache(gpu, tmp_path):
     tune = c.autotune_classes(reps=1, cache=str(cache))
     assert all(x["from_cache"] for x in tune["classes"]) and not tune["per_class"]
     assert launches(c) == 3  # the tiles
+
+
+def test_tuning_under_the_surrogate(gpu):
+    """The surrogate's evaluations have no shape: tuning leaves the choice alone, and the row list is back after it."""
+    w = cases.ring_stations(stations=40, seed=1)
+    c = capi.Context(precision=capi.FP32C, nu=NU)
+    k = c.add_wake(w.n)
+    c.set_particles(k, w)
+    c.solve()
+    before = c.rates(k)
+    c.surrogate_enable(0)
+    (block, tpt), ms = c.autotune(reps=1)
+    assert (block, tpt) == (128, 2) and set(ms.values()) == {0.0}
+    c.surrogate_disable()
+    assert launches(c) == 2  # the row list
+    for got, ref in zip(c.rates(k), before):
+        assert np.array_equal(got, ref)
+
+
+def test_tuning_again_at_another_size(gpu):
+    """A shape that won at a large size is weighed against the row list when the context is tuned at a small one."""
+    big = section_ring(60000)
+    small = cases.ring_stations(stations=40, seed=1)
+    c = capi.Context(precision=capi.FP32C, nu=NU)
+    k = c.add_wake(big.n)
+    c.set_particles(k, big)
+    c.autotune(reps=1)
+    assert launches(c) == 3  # tiles
+    c.set_particles(k, small)
+    assert launches(c) == 3  # tuned: stays
+    c.autotune(reps=2)
+    assert launches(c) == 2
