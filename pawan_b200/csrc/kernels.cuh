@@ -417,7 +417,7 @@ __device__ __forceinline__ void pair_body_generic(const PairArgs<T> &a) {
                   sdv[k][0] += pt.zd * (vt[k] * q.x - q.w * at[k][0]);
                   sdv[k][1] += pt.zd * (vt[k] * q.y - q.w * at[k][1]);
                   sdv[k][2] += pt.zd * (vt[k] * q.z - q.w * at[k][2]);
-                  ++nfull;
+                  nfull += t0 + tid + k * BLOCK < tend;
                 }
               }
             } else {
@@ -437,7 +437,7 @@ __device__ __forceinline__ void pair_body_generic(const PairArgs<T> &a) {
                   sdv[k][0] += pt.zd * (vt[k] * q.x - q.w * at[k][0]);
                   sdv[k][1] += pt.zd * (vt[k] * q.y - q.w * at[k][1]);
                   sdv[k][2] += pt.zd * (vt[k] * q.z - q.w * at[k][2]);
-                  if constexpr (KER == kGaussian) ++nfull;
+                  if constexpr (KER == kGaussian) nfull += t0 + tid + k * BLOCK < tend;
                 }
               }
             }

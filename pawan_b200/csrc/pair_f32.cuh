@@ -341,7 +341,9 @@ __device__ __forceinline__ void pair_body_f32(const PairArgs<float> &a) {
 #pragma unroll
     for (int k = 0; k < TPT; ++k) {
       int64_t ti = t0 + tid + k * BLOCK;
-      ti = ti < tend ? ti : tend - 1;
+      // threads past the end repeat the last target, and count none of its pairs
+      const bool live = ti < tend;
+      ti = live ? ti : tend - 1;
       const float4 p = a.P[ti];
       const float4 q = a.Q[ti];
       if constexpr (SPLIT) {
@@ -349,7 +351,7 @@ __device__ __forceinline__ void pair_body_f32(const PairArgs<float> &a) {
         xl[k][0] = l.x; xl[k][1] = l.y; xl[k][2] = l.z;
       }
       hst[k] = p.w;
-      h50[k] = kFarU * p.w;
+      h50[k] = TPT == 1 || live ? kFarU * p.w : -3.0e38f;  // with two targets or more, only counts
       at[k][0] = q.x; at[k][1] = q.y; at[k][2] = q.z; vt[k] = q.w;
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
@@ -599,7 +601,7 @@ __device__ __forceinline__ void pair_body_f32(const PairArgs<float> &a) {
       buf ^= 1;
     }
     cp_async_wait<0>();
-    const unsigned wsum = __reduce_add_sync(0xffffffffu, nfull);
+    const unsigned wsum = __reduce_add_sync(0xffffffffu, TPT > 1 || t0 + tid < tend ? nfull : 0u);
     if (lane == 0 && wsum) atomicAdd(a.nfull, (unsigned long long)wsum);
 
 #pragma unroll

@@ -346,7 +346,8 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices_kernel(PairAr
       }
       fold_group_f32(far, pt.x - rx, pt.y - ry, pt.z - rz, at, a.nu2, sv, sd, sp, sdv, vh, vl, dh, dl);
     }
-    const unsigned wsum = __reduce_add_sync(0xffffffffu, nfull);
+    // lanes past the end repeat the last target
+    const unsigned wsum = __reduce_add_sync(0xffffffffu, run.t0 + lane < run.tend ? nfull : 0u);
     if (lane == 0 && wsum) atomicAdd(a.nfull, (unsigned long long)wsum);
 
     __syncthreads();  // every warp is done with its slices

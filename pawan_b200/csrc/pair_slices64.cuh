@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps, 2) pair_slices64_kernel(Pair
       for (int m = 0; m < 6; ++m) two_sum_acc(hi[32 * m], lo[32 * m], add[m]);
     }
     if constexpr (KER == kGaussian) {
-      const unsigned wsum = __reduce_add_sync(0xffffffffu, nfull);
+      const unsigned wsum = __reduce_add_sync(0xffffffffu, run.t0 + lane < run.tend ? nfull : 0u);
       if (lane == 0 && wsum) atomicAdd(a.nfull, (unsigned long long)wsum);
     }
 #pragma unroll

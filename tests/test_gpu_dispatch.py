@@ -198,3 +198,21 @@ def test_tuning_again_at_another_size(gpu):
     assert launches(c) == 3  # tuned: stays
     c.autotune(reps=2)
     assert launches(c) == 2
+
+
+@pytest.mark.parametrize("shape", [{}, {"block": 128, "tpt": 1}, {"block": 128, "tpt": 2}, {"block": 64, "tpt": 2},
+                                   {"block": 128, "tpt": 4}])
+@pytest.mark.parametrize("precision,limit", [(capi.FP32C, 50.0), (capi.FP64, 100.0)])
+@pytest.mark.parametrize("n", [33, 1000, 1001, 1024])
+def test_pair_counts(gpu, n, precision, limit, shape):
+    """Pairs and full-formula pairs as counted on the CPU, in every kernel, also where lanes repeat the last target.  FP32C
+    decides u < 50 in FP32, so pairs within 1e-5 of it may go either way."""
+    w = cases.ring_stations(stations=-(-n // 25), sigma=0.02, seed=3).subset(n)
+    u = ((w.pos[:, None] - w.pos[None]) ** 2).sum(-1) / (0.5 * (w.sigma[:, None] ** 2 + w.sigma[None] ** 2))
+    c = capi.Context(precision=precision, nu=NU, **shape)
+    c.set_particles(c.add_wake(n), w)
+    c.solve()
+    pairs, full = c.pair_counts()
+    assert pairs == n * (n - 1)
+    slack = 1e-5 if precision == capi.FP32C else 1e-12
+    assert (u < limit * (1 - slack)).sum() - n <= full <= (u < limit * (1 + slack)).sum() - n
