@@ -274,7 +274,7 @@ int pgpu_snapshot_wait(pgpu_ctx *ctx, int32_t slot, double seconds, const double
 int pgpu_sync(pgpu_ctx *ctx);
 /* Pair-kernel timing (pgpu_pair_kernel_time) is on by default.  Reading the
  * CUDA-event times makes pgpu_solve / pgpu_step / pgpu_stage wait for their
- * pair kernels; with timing off (on = 0) those calls only queue work, and
+ * pair kernels (pgpu_step for a step's after queueing the next); with timing off (on = 0) those calls only queue work, and
  * pgpu_sync or pgpu_sync_timeout waits.  No PAWAN counterpart. */
 int pgpu_set_timing(pgpu_ctx *ctx, int on);
 /* pgpu_sync with a host watchdog: returns PGPU_ETIMEOUT if the queued work has
@@ -282,8 +282,13 @@ int pgpu_set_timing(pgpu_ctx *ctx, int on);
  * waits for it), else as pgpu_sync.  No PAWAN counterpart. */
 int pgpu_sync_timeout(pgpu_ctx *ctx, double seconds);
 
-/* Device time in milliseconds of the pair kernel launches since the last call
- * (CUDA events on the context stream), and the number of them. */
+/* Device time in milliseconds of the pair kernel launches since the last call,
+ * and the number of them.  Single evaluations (pgpu_solve, pgpu_stage, and
+ * pgpu_step without graphs) are bracketed by CUDA events on the context stream,
+ * which adds about 4 us of launch to each.  In the steps of a graph the events
+ * are on a branch beside the kernels, and the start event is not ordered before
+ * the kernel: a reading is about the kernel alone, to a few microseconds either
+ * way.  For kernels of some tens of microseconds use single evaluations. */
 int pgpu_pair_kernel_time(pgpu_ctx *ctx, double *ms, int64_t *launches);
 
 /* Ordered pair interactions (self pairs excluded) evaluated by the pair

@@ -216,3 +216,24 @@ def test_pair_counts(gpu, n, precision, limit, shape):
     assert pairs == n * (n - 1)
     slack = 1e-5 if precision == capi.FP32C else 1e-12
     assert (u < limit * (1 - slack)).sum() - n <= full <= (u < limit * (1 + slack)).sum() - n
+
+
+@pytest.mark.parametrize("precision", [capi.FP32C, capi.FP64])
+@pytest.mark.parametrize("n", [25, 1000, 5000])
+def test_pair_time_of_graph_steps(gpu, n, precision):
+    """Pair-kernel times of graph steps against those of the same steps without graphs, which bracket the launch: shorter by
+    the launch, about 4 us, and no longer; a few us more either way are allowed."""
+    w = cases.ring_stations(stations=-(-n // 25), seed=3).subset(n)
+    us = []
+    for graphs in (True, False):
+        c = capi.Context(precision=precision, nu=NU, use_graphs=graphs)
+        c.set_particles(c.add_wake(n), w)
+        best = 1e9
+        for _ in range(6):
+            c.step("rk4", 1e-4, 10)
+            t, launches = c.pair_kernel_time()
+            assert launches == 40
+            best = min(best, 1e3 * t / launches)
+        us.append(best)
+    assert us[1] - 9.0 <= us[0] <= us[1] + 3.0
+    assert us[0] > 0.5 * us[1]
