@@ -87,9 +87,9 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 // 1/sqrt(x) in FP64: the hardware approximation (rsqrt.approx.ftz.f64, good to
-// about 2^-20) refined by one third-order step of Halley's iteration for
+// about 2^-20) refined by one step of Chebyshev's third-order method for
 // f(y) = 1/y^2 - x: with e = 1 - x y^2, y + y e (1/2 + 3/8 e), whose error is
-// e^3 / 3 or so.  Five FP64 operations; arguments that are not positive normal
+// 5/16 e^3 (3e-18) and the roundings', 1.7e-16 in all.  Five FP64 operations; arguments that are not positive normal
 // numbers (zero, subnormal, infinite, NaN) take the library function.
 __device__ __forceinline__ double rsqrt_normal(double x) {  // x positive and normal
   double y;

@@ -223,3 +223,15 @@ def test_surrogate_tree_sizes(gpu, n, leaf, order):
     assert np.array_equal(cells[order_][1:, 0], cells[order_][:-1, 1])
     for got, want in zip(c.rates(ids[0]), ref):
         assert np.abs(got - want).max() <= 2.5e-3 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("kernel", ["gaussian", "highorder"])
+@pytest.mark.parametrize("npts", [1, 2, 3, 4, 5, 6, 7, 9])
+def test_probe_point_tiles(gpu, npts, kernel):
+    """Point tiles of four: last tiles of one to four points."""
+    w = ring(700)
+    pts = np.random.default_rng(npts).normal(0.0, 0.8, (npts, 3))
+    c, _ = context([w], capi.FP32C, kernel=kernel)
+    v = c.probe(pts)
+    ref = np.array([O.restate_getvi(w, p, kernel) for p in pts])
+    assert np.abs(v - ref).max() <= 1e-11 * np.abs(v).max()
