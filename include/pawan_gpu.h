@@ -59,9 +59,10 @@ typedef struct pgpu_config {
   double vinf[3];  /* uniform inflow added after each step, x += vinf dt
                       (__wake::updateVinfEffect, wake.cpp:564-577, called from integration.cpp:172) */
   int block;       /* pair-kernel threads per CTA; 0 = default (Gaussian: 128; high-order: 256) until pgpu_autotune.
-                      With block, tpt and chunks all 0, FP32C Gaussian systems of fewer than 48,000 targets in all or
-                      with split positions, the high-order kernel and the FP64 mode take the row-list kernel instead,
-                      which fills the device evenly at any size. */
+                      With block, tpt and chunks all 0, FP32C Gaussian systems of fewer than 48,000 targets in all (or
+                      with split positions, where their filaments are dense enough), the high-order kernel and the
+                      FP64 mode (but for very many systems of a few hundred particles) take the row-list kernel
+                      instead, which fills the device evenly at any size. */
   int tpt;         /* pair-kernel targets per thread; 0 = default (Gaussian FP32C: 2, FP64: 1; high-order: 1) */
   int chunks;      /* source chunks per system (1..16); 0 = automatic */
   int use_graphs;  /* capture each time step in a CUDA graph (default 1) */

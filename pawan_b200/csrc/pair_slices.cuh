@@ -1,6 +1,6 @@
 // FP32 (compensated) pair kernel for systems too small to fill the device with
-// the CTA-wide target tiles of pair_f32.cuh, and for dense filaments, where its
-// finer boxes find more far pairs.  Bound by the FP32 pipe from a few thousand
+// the CTA-wide target tiles of pair_f32.cuh, and for wakes of dense filaments,
+// where its finer boxes find more far pairs.  Bound by the FP32 pipe from a few thousand
 // particles on (64% busy on 20,000 particles, warps mostly waiting for it), by
 // latency below.  The 5000-particle station ring: 62 us per evaluation (4.1e11
 // pairs/s) against 167 us with 128 x 2 tiles (20 x 16 items, mostly idle SMs).
@@ -17,8 +17,9 @@
 //
 // High-order kernel (KER): every pair takes its full terms, two sources per
 // packed instruction, 42 FP32 operations in slices far from the targets and 58
-// in the others (two less where one sigma serves the slice), against 68 scalar instructions in the generic body; no pair
-// is cheap enough for wider tiles to pay, so it takes these slices at any size.
+// in the others (two less where one sigma serves the slice), against 68 scalar
+// instructions in the generic body; no pair is cheap enough for wider tiles to
+// pay, so it takes these slices at any size.
 #pragma once
 
 namespace pgpu {

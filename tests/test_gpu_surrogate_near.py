@@ -88,3 +88,27 @@ def test_collapsed_cluster_time(gpu):
         c.solve()
         best = min(best, c.surrogate_stats()["ms_tree"])
     assert best <= 5.0
+
+
+@pytest.mark.parametrize("radii", [1, 2])
+def test_expansion_orders(gpu, radii):
+    """Each moment of the far cells counts: with particles within 0.87 cube widths of a cell's centroid and the targets at
+    least five widths off, the next order drops the truncation to 0.87 / 5 = 0.17 of it; twice that bounds the ratio of the
+    largest errors, from order 1 to 2 and from 2 to 3 (against the direct sum, both FP32C)."""
+    w = cases.leapfrog_rings(60000)
+    if radii == 2:
+        w.sigma[::3] *= 0.8
+    c = capi.Context(precision=capi.FP32C, nu=NU)
+    k = c.add_wake(w.n)
+    c.set_particles(k, w)
+    c.solve()
+    ref = c.rates(k)
+    errors = []
+    for order in (1, 2, 3):
+        c.surrogate_enable(0, order=order, check_targets=0)
+        c.solve()
+        errors.append([np.linalg.norm(got - want, axis=1).max() / np.linalg.norm(want, axis=1).max()
+                       for got, want in zip(c.rates(k), ref)])
+    for low, high in zip(errors, errors[1:]):
+        for a, b in zip(low, high):
+            assert b <= 0.35 * a
